@@ -23,7 +23,7 @@ namespace dnufft {
 template <typename Tc, int NDIM>
 __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t cs1,
                             uint32_t npts, Geometry g, uint32_t *__restrict__ keys,
-                            uint32_t *__restrict__ idx, bool qbits) {
+                            uint32_t *__restrict__ idx, TileOrder order) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= npts) return;
   int t[NDIM];
@@ -40,7 +40,7 @@ __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t c
     key = uint32_t(t[0] >> g.log2tile);
   } else if constexpr (NDIM == 2) {
     key = uint32_t(t[0] >> g.log2tile) * uint32_t(g.ntiles[1]) + uint32_t(t[1] >> g.log2tile);
-    if (qbits) {
+    if (order.quadrant) {
       // quadrant, then the cell inside it in Morton order: consecutive points
       // (one K-block of the tensor-core spreader) lie close together, so each
       // accumulator cell receives contributions from fewer K-blocks
@@ -51,6 +51,12 @@ __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t c
         mort |= (((du >> b) & 1u) << (2 * b + 1)) | (((dv >> b) & 1u) << (2 * b));
       key = (key << 2) | (((t[0] & m) >= half) ? 2u : 0u) | (((t[1] & m) >= half) ? 1u : 0u);
       key = (key << (2 * lh)) | mort;
+    } else if (order.bin_bits) {
+      // bin of 8 x 8 cells inside the tile: consecutive points share the
+      // spreader's window
+      const uint32_t bm = (1u << (order.bin_bits >> 1)) - 1u;
+      key = (key << order.bin_bits) | ((uint32_t(t[0] >> 3) & bm) << (order.bin_bits >> 1)) |
+            (uint32_t(t[1] >> 3) & bm);
     }
   } else {
     uint32_t ss = uint32_t(g.ssmall), ms = (1u << ss) - 1u;
@@ -67,12 +73,12 @@ __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t c
 
 void launch_fold_keys(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
                       uint32_t npts, const Geometry &g, uint32_t *keys, uint32_t *idx,
-                      cudaStream_t st, bool quadrant_bits) {
+                      cudaStream_t st, TileOrder order) {
   if (npts == 0) return;
   dim3 block(256), grid((npts + 255) / 256);
 #define FK(TC, ND) \
   k_fold_keys<TC, ND><<<grid, block, 0, st>>>((const TC *)coord, cs0, cs1, npts, g, keys, idx, \
-                                               quadrant_bits)
+                                               order)
   if (coord_f64) {
     if (g.ndim == 1) FK(double, 1); else if (g.ndim == 2) FK(double, 2); else FK(double, 3);
   } else {
@@ -247,7 +253,7 @@ __global__ void k_radix_scatter(const uint32_t *__restrict__ kin, const uint32_t
 }
 
 size_t radix_workspace_bytes(uint32_t n, int keybits) {
-  int passes = (keybits + 10) / 11;
+  int passes = (keybits + RADIX_BITS - 1) / RADIX_BITS;
   if (passes < 1) passes = 1;
   int nbits = (keybits + passes - 1) / passes;
   uint64_t nblocks = (uint64_t(n) + RS_TILE - 1) / RS_TILE;
@@ -271,7 +277,7 @@ __global__ void k_copy_pairs(const uint32_t *__restrict__ ka, const uint32_t *__
 void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, void *ws,
                       cudaStream_t st) {
   if (n <= 1 || keybits <= 0) return;
-  int passes = (keybits + 10) / 11;
+  int passes = (keybits + RADIX_BITS - 1) / RADIX_BITS;
   int nbits = (keybits + passes - 1) / passes;
   uint32_t nblocks = uint32_t((uint64_t(n) + RS_TILE - 1) / RS_TILE);
   uint64_t hn = (uint64_t(1) << nbits) * nblocks;
@@ -291,7 +297,7 @@ void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, v
   static bool attr_set = false;
   if (!attr_set) {
     DN_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 RS_WARPS * (4 << 11)));
+                                 RS_WARPS * (4 << RADIX_BITS)));
     attr_set = true;
   }
   for (int pass = 0; pass < passes; ++pass) {
@@ -583,6 +589,72 @@ uint32_t build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, u
   uint32_t h = 0;
   read_words(src, 1, &h, st);
   return h;
+}
+
+// sorted positions of the points of groups [g0, g1), bin after bin: counts
+// per bin, then (after a scan into pos) the positions
+__global__ void k_gsel_count(const uint32_t *__restrict__ start, uint32_t nbins, int gbits,
+                             uint32_t g0, uint32_t g1, uint32_t *__restrict__ cnt) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nbins; t += gridDim.x * blockDim.x)
+    cnt[t] = start[(uint64_t(t) << gbits) + g1] - start[(uint64_t(t) << gbits) + g0];
+}
+
+__global__ void k_gsel_fill(const uint32_t *__restrict__ start, const uint32_t *__restrict__ cnt,
+                            const uint32_t *__restrict__ pos, uint32_t nbins, int gbits,
+                            uint32_t g0, uint32_t *__restrict__ sel) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nbins;
+       t += gridDim.x * blockDim.x) {
+    const uint32_t s = start[(uint64_t(t) << gbits) + g0], n = cnt[t];
+    uint32_t *d = sel + pos[t];
+    for (uint32_t k = 0; k < n; ++k) d[k] = s + k;
+  }
+}
+
+size_t group_select_workspace_bytes(uint32_t nbins) {
+  return size_t(2) * nbins * 4 + 256 + scan_workspace_bytes(nbins);
+}
+
+void build_group_select(const uint32_t *start, uint32_t nbins, int gbits, uint32_t g0, uint32_t g1,
+                        uint32_t *sel, void *ws, cudaStream_t st) {
+  uint32_t *cnt = static_cast<uint32_t *>(ws);
+  uint32_t *pos = cnt + nbins;
+  uint32_t *sws = reinterpret_cast<uint32_t *>(
+      (reinterpret_cast<uintptr_t>(pos + nbins) + 255) & ~uintptr_t(255));
+  k_gsel_count<<<grid_of(nbins), 256, 0, st>>>(start, nbins, gbits, g0, g1, cnt);
+  DN_LAUNCHED();
+  exclusive_scan(cnt, pos, nbins, sws, st);
+  k_gsel_fill<<<grid_of(nbins), 256, 0, st>>>(start, cnt, pos, nbins, gbits, g0, sel);
+  DN_LAUNCHED();
+}
+
+// histogram of the groups: in shared memory where it fits
+constexpr uint32_t GROUP_HIST_MAX = 8192;
+
+__global__ void k_group_counts(const uint32_t *__restrict__ group, uint32_t n, uint32_t ngroups,
+                               uint32_t *__restrict__ counts) {
+  extern __shared__ uint32_t gh[];
+  const bool sh = ngroups <= GROUP_HIST_MAX;
+  if (sh) {
+    for (uint32_t i = threadIdx.x; i < ngroups; i += blockDim.x) gh[i] = 0;
+    __syncthreads();
+  }
+  uint32_t *h = sh ? gh : counts;
+  for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += uint64_t(gridDim.x) * blockDim.x)
+    if (group[i] < ngroups) atomicAdd(&h[group[i]], 1u);
+  if (sh) {
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < ngroups; i += blockDim.x)
+      if (gh[i]) atomicAdd(&counts[i], gh[i]);
+  }
+}
+
+void launch_group_counts(const uint32_t *group, uint32_t n, uint32_t ngroups, uint32_t *counts,
+                         cudaStream_t st) {
+  DN_CUDA(cudaMemsetAsync(counts, 0, size_t(ngroups) * 4, st));
+  const size_t sm = ngroups <= GROUP_HIST_MAX ? size_t(ngroups) * 4 : 0;
+  k_group_counts<<<std::min(grid_of(n), 148u * 4u), 256, sm, st>>>(group, n, ngroups, counts);
+  DN_LAUNCHED();
 }
 
 }  // namespace dnufft

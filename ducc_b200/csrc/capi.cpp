@@ -39,7 +39,6 @@ namespace dnufft {
 
 constexpr uint32_t CHUNK = 1024;       // points per chunk (one CTA)
 constexpr uint32_t CHUNK_TC = 4096;    // tensor-core plans: fewer, longer chunks
-constexpr double TC_AUTO_DENSITY = 0.5;   // points per uniform mode from which 'auto' picks TC
 
 // ---------------------------------------------------------------- device buffers
 // Keep memory freed with cudaFreeAsync in the device's default pool instead of
@@ -340,6 +339,7 @@ struct Setup {
   std::vector<int> factors[3];
   int spreader = DNUFFT_SPREAD_AUTO;
   bool qbits = false;   // sort key carries the 2D tile quadrant and cell (tensor-core order)
+  TileOrder order;      // the key bits below the tile (2D)
   int keybits = 1;
   int tile_shift = 0;
   uint64_t max_tiles = 0;
@@ -372,7 +372,8 @@ static int bitlen64(uint64_t v) {
 }
 
 static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double epsilon,
-                        bool gridding, bool calc_f64, bool coord_f64, const dnufft_opts &o) {
+                        bool gridding, bool calc_f64, bool coord_f64, const dnufft_opts &o,
+                        bool run_order = false) {
   DN_REQUIRE(ndim >= 1 && ndim <= 3, ST_BADARG, "transform must be 1D/2D/3D");
   DN_REQUIRE(npoints <= 0xffffffffull, ST_BADARG, "too many nonuniform points");
   DN_REQUIRE(epsilon > 0, ST_BADARG, "epsilon must be positive");
@@ -458,24 +459,28 @@ static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double 
     s.tile_shift = 3 * g.ssmall;
     s.max_tiles = prod;
   }
-  // automatic choice for type 1: the tensor-core spreader where it is the
-  // faster one (measured on B200 from 256^2 to 4096^2 grids, uniform and
-  // clustered points: from about half a point per uniform mode up; below that
-  // its per-tile set-up and flush cost more than the plain atomics)
-  if (s.spreader == DNUFFT_SPREAD_AUTO && gridding && ndim == 2 && !calc_f64 &&
-      spread_tc_supported(g, calc_f64) &&
-      double(npoints) >= TC_AUTO_DENSITY * double(nuni[0]) * double(nuni[1]))
-    s.spreader = DNUFFT_SPREAD_TC;
+  // automatic choice: the plain spreader, faster than the tensor-core one at
+  // every density measured (W = 8, spreading alone: 5e7 clustered points on
+  // 4096^2 modes 2.02 against 3.49 ms, 8e6 points on 1024^2 0.31 / 0.51 ms,
+  // 2e4 points 0.04 / 0.08 ms) and the more accurate one
   if (s.spreader == DNUFFT_SPREAD_TC && spread_tc_supported(g, calc_f64)) {
     s.qbits = true;
+    s.order.quadrant = true;
     maxkey <<= 2 + tc_cell_bits(g);
     s.tile_shift = 2 + tc_cell_bits(g);
     // per-chunk set-up and flush of the tensor-core spreader cost more than
     // the plain one's: amortise them over longer chunks
     s.chunk = CHUNK_TC;
+  } else if (run_order && ndim == 2) {
+    // bins of 8 x 8 cells where the key has room for them
+    const int bb = 2 * (g.log2tile - 3);
+    if (bitlen64(maxkey) + bb <= 32) {
+      s.order.bin_bits = bb;
+      s.tile_shift = bb;
+    }
   }
   DN_REQUIRE(maxkey < (uint64_t(1) << 32), ST_UNSUPPORTED, "tile key space too large");
-  s.keybits = std::max(1, bitlen64(maxkey));
+  s.keybits = std::max(1, bitlen64(maxkey)) + s.order.bin_bits;
   if (s.spreader == DNUFFT_SPREAD_TC)
     DN_REQUIRE(spread_tc_supported(g, calc_f64), ST_UNSUPPORTED,
                "tensor-core spreader: 2D single precision (complex64) with support <= 8 only");
@@ -592,16 +597,20 @@ static uint32_t sm_count() {
   return uint32_t(n > 0 ? n : 1);
 }
 
-static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream_t st) {
+// need_chunks: the chunk list too (the 2D plain spreader needs none; the
+// number of chunks is read back to the host, which waits for the sort)
+static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream_t st,
+                        bool need_chunks = true) {
   uint32_t M = s.npoints;
   ix.perm = DevBuf(size_t(M) * 4, st);
   ix.keys = DevBuf(size_t(M) * 4, st);
   launch_fold_keys(s.coord_f64, coord.data, coord.stride[0], coord.stride[1], M, s.g,
-                   ix.keys.as<uint32_t>(), ix.perm.as<uint32_t>(), st, s.qbits);
+                   ix.keys.as<uint32_t>(), ix.perm.as<uint32_t>(), st, s.order);
   {
     DevBuf ws(radix_workspace_bytes(M, s.keybits), st);
     radix_sort_pairs(ix.keys.as<uint32_t>(), ix.perm.as<uint32_t>(), M, s.keybits, ws.p, st);
   }
+  if (!need_chunks) return;
   uint64_t maxchunks = std::min<uint64_t>(M, s.max_tiles) + M / s.chunk + 2;
   ix.chunks = DevBuf(size_t(maxchunks) * sizeof(Chunk), st);
   ix.count = DevBuf(16, st);
@@ -619,6 +628,9 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
                                 tc_cell_bits(s.g), st);
   }
 }
+
+// does type 1 of this setup work from a chunk list?
+static bool spread_needs_chunks(const Setup &s) { return s.g.ndim != 2 || s.qbits; }
 
 static size_t grid_cells(const Geometry &g) {
   size_t c = 1;
@@ -646,7 +658,7 @@ static void report_sizes(const Setup &s, bool gridding) {
 template <typename T>
 static void spread_points(const Setup &s, const PointsDesc &pts, const ChunkList &cl,
                           const TcBlocks *tb, const void *values, int64_t vs, void *grid, int *err,
-                          cudaStream_t st) {
+                          cudaStream_t st, const uint32_t *sel = nullptr, uint32_t nsel = 0) {
   const KernelPoly<T> &kp = *reinterpret_cast<const KernelPoly<T> *>(
       sizeof(T) == 4 ? static_cast<const void *>(&s.kpf) : static_cast<const void *>(&s.kpd));
   bool use_tc = false;
@@ -662,6 +674,8 @@ static void spread_points(const Setup &s, const PointsDesc &pts, const ChunkList
   if (use_tc) {
     launch_spread_tc(pts, *tb, s.g, s.kpf, values, vs, grid, reinterpret_cast<unsigned *>(err + 1),
                      err, st);
+  } else if (sel) {
+    launch_spread_run<T>(pts, sel, nsel, s.g, kp, values, vs, 0, grid, 0, 1, st);
   } else {
     launch_spread<T>(pts, cl, s.g, kp, values, vs, 0, grid, 0, 1, st);
   }
@@ -671,7 +685,8 @@ template <typename T>
 static void do_spread_fft(const Setup &s, const DevConst &dc, const PointsDesc &pts,
                           const ChunkList &cl, const TcBlocks *tb, const View &points,
                           const View &out, bool forward, bool fft_order, StageTimer &tm,
-                          cudaStream_t st, DevBuf *ws = nullptr, DevBuf *wk = nullptr) {
+                          cudaStream_t st, DevBuf *ws = nullptr, DevBuf *wk = nullptr,
+                          const uint32_t *sel = nullptr, uint32_t nsel = 0) {
   size_t cells = grid_cells(s.g);
   tm.mark("zeroing grid");
   DevBuf local;
@@ -680,7 +695,7 @@ static void do_spread_fft(const Setup &s, const DevConst &dc, const PointsDesc &
   DN_CUDA(cudaMemsetAsync(grid.p, 0, cells * sizeof(T) * 2, st));
   tm.mark("spreading");
   int *err = device_error_word();
-  spread_points<T>(s, pts, cl, tb, points.data, points.stride[0], grid.p, err, st);
+  spread_points<T>(s, pts, cl, tb, points.data, points.stride[0], grid.p, err, st, sel, nsel);
   tm.mark("FFT + correction");
   DevBuf localw;
   DevBuf &work = wk ? *wk : localw;
@@ -868,7 +883,7 @@ static void nu2u_pipelined(const Setup &s, const View &points, const View &coord
     sg.npoints = uint32_t(b - a);
     const View cv = coord_range(coord, dcoord.p, a, b, cb);
     Index ix;
-    build_index(sg, cv, ix, st);
+    build_index(sg, cv, ix, st, spread_needs_chunks(sg));
     PointsDesc pts{cv.data, cv.stride[0], cv.stride[1], false, s.coord_f64,
                    ix.perm.as<uint32_t>(), sg.npoints};
     ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
@@ -976,7 +991,7 @@ static void nu2u_impl(const dnufft_array *points_, const dnufft_array *coord_, i
   DN_REQUIRE(out.dtype == points.dtype, ST_BADARG, "out must have the dtype of points");
   bool f64 = points.dtype == DNUFFT_C128;
   Setup s = make_setup(ndim, out.shape, uint64_t(points.shape[0]), eps, true, f64,
-                       coord.dtype == DNUFFT_F64, o);
+                       coord.dtype == DNUFFT_F64, o, true);
   StageTimer tm(o.verbosity > 0, st);
   if (o.verbosity > 0) report_sizes(s, true);
   if (points.host && coord.host && pipe_groups(s.npoints) > 1) {
@@ -1007,7 +1022,7 @@ static void nu2u_impl(const dnufft_array *points_, const dnufft_array *coord_, i
   }
   tm.mark("building index");
   Index ix;
-  build_index(s, sc.dev, ix, st);
+  build_index(s, sc.dev, ix, st, spread_needs_chunks(s));
   tm.mark("wait for values copy");
   side.merge();
   PointsDesc pts{sc.dev.data, sc.dev.stride[0], sc.dev.stride[1], false, s.coord_f64,
@@ -1163,7 +1178,7 @@ static void plan_create_impl(int nu2u, const dnufft_array *coord_, const int64_t
   bool f64 = coord.dtype == DNUFFT_F64;
   auto p = std::make_unique<dnufft_plan>();
   p->o = o;
-  p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o);
+  p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o, true);
   DN_CUDA(cudaGetDevice(&p->device));
   upload_consts(p->s, p->dc, st);
   if (p->s.npoints > 0) {
@@ -1783,12 +1798,17 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
     for (int i = 0; i < ax[d].nfac; ++i) ax[d].fac[i] = s.factors[d][i];
     ax[d].tw = tw[d];
   }
-  // index: fold + stable sort + chunks (the chunk count read-back synchronises
-  // the stream, after which the host constant buffers may be released)
+  // index: fold + stable sort by tile + chunks (1D, 3D); the stream is
+  // synchronised here (chunk count read-back), after which the host constant
+  // buffers may be released
   launch_fold_keys(s.coord_f64, coord.data, coord.stride[0], coord.stride[1], M, g, keys, perm, st);
   radix_sort_pairs(keys, perm, M, s.keybits, rws, st);
-  uint32_t nch = build_chunks(keys, M, s.tile_shift, s.chunk, chunks, count, cws, st,
-                              /*zero_copy=*/false);
+  uint32_t nch = 0;
+  if (spread_needs_chunks(s))
+    nch = build_chunks(keys, M, s.tile_shift, s.chunk, chunks, count, cws, st,
+                       /*zero_copy=*/false);
+  else
+    DN_CUDA(cudaStreamSynchronize(st));
   PointsDesc pts{coord.data, coord.stride[0], coord.stride[1], false, s.coord_f64, perm, M};
   ChunkList cl{chunks, nch};
   // the scratch keeps the previous call's contents: the grid must start at zero
@@ -1855,11 +1875,13 @@ int nu2u_in_scratch(const dnufft_array *points, const dnufft_array *coord, int f
 
 // ---------------------------------------------------------------- grouped index
 // A 2D index over points that belong to groups (the w-gridder's first w
-// plane): sorted once by (tile, group), so that within every tile the points
-// of any run of groups are one contiguous range, and a type 1 or type 2
-// transform over such a run needs only a chunk list (one chunk per tile and
-// at most CHUNK points, so a tile is still flushed once), not a sort of its
-// own.  Plain spreader; kernel and grid as forced in the options.
+// plane), for type 1 or for type 2.  Type 2: sorted once by (tile, group), so
+// that within every tile the points of any run of groups are one contiguous
+// range, and a transform over such a run needs only a chunk list (one chunk per
+// tile and at most CHUNK points), not a sort of its own.  Type 1: sorted by
+// (tile, bin of 8 x 8 cells, group), and a transform takes the list of the
+// run's positions bin after bin (the plain spreader's order).  Kernel and grid
+// as forced in the options.
 struct GroupedPlan {
   Setup s;
   DevConst dcl;
@@ -1867,6 +1889,14 @@ struct GroupedPlan {
   DevBuf sorted_coord, perm, start, chunks, cws, grid, work;
   uint32_t ntiles = 0, ngroups = 0, nchunks = 0, g0 = 0, g1 = 0;
   int gbits = 0;
+  bool type1 = false;
+  std::vector<uint32_t> gcount;   // points per group
+  DevBuf sel;                     // type 1: sorted positions of the current run's points
+  uint64_t run_points(uint32_t a, uint32_t b) const {
+    uint64_t n = 0;
+    for (uint32_t k = a; k < b && k < ngroups; ++k) n += gcount[k];
+    return n;
+  }
 };
 
 static int bits_for(uint64_t v) {   // bits to hold 0..v
@@ -1878,14 +1908,15 @@ static int bits_for(uint64_t v) {   // bits to hold 0..v
 GroupedPlan *grouped_plan_create(const double *coord, uint32_t M, const uint32_t *group,
                                  uint32_t ngroups, const int64_t *shape, double eps,
                                  bool calc_f64, const dnufft_opts &opts, cudaStream_t st,
-                                 uint32_t *perm_out) {
+                                 bool type1, uint32_t *perm_out) {
   dnufft_opts o = opts;
   o.spreader = DNUFFT_SPREAD_PLAIN;
   auto gp = std::make_unique<GroupedPlan>();
   gp->s = make_setup(2, shape, M, eps, true, calc_f64, true, o);
+  gp->type1 = type1;
   Setup &s = gp->s;
   DN_REQUIRE(!s.qbits, ST_INTERNAL, "grouped index with a tensor-core key");
-  const int tilebits = s.keybits;
+  int tilebits = s.keybits;
   gp->gbits = bits_for(ngroups);
   // keys (tile << gbits | group) in 32 bits, and a start table of
   // ntiles * 2^gbits + 1 entries of at most 512 MB
@@ -1895,11 +1926,21 @@ GroupedPlan *grouped_plan_create(const double *coord, uint32_t M, const uint32_t
     return nullptr;
   gp->ngroups = ngroups;
   gp->ntiles = uint32_t(ntiles);
+  if (type1) {
+    // bins instead of tiles where key and table have room for them
+    const int bb = 2 * (s.g.log2tile - 3);
+    if (tilebits + bb + gp->gbits <= 32 &&
+        (ntiles << (bb + gp->gbits)) <= (uint64_t(1) << 27)) {
+      s.order.bin_bits = bb;
+      tilebits += bb;
+      gp->ntiles <<= bb;
+    }
+  }
   gp->dc = &consts_for(s, gp->dcl, st);
   DevBuf keys(size_t(M) * 4, st);
   gp->perm = DevBuf(size_t(M) * 4, st);
   launch_fold_keys(true, coord, 2, 1, M, s.g, keys.as<uint32_t>(), gp->perm.as<uint32_t>(), st,
-                   false);
+                   s.order);
   launch_group_keys(keys.as<uint32_t>(), group, M, gp->gbits, st);
   const int total = tilebits + gp->gbits;
   {
@@ -1911,8 +1952,18 @@ GroupedPlan *grouped_plan_create(const double *coord, uint32_t M, const uint32_t
   launch_key_starts(keys.as<uint32_t>(), M, nkeys, gp->start.as<uint32_t>(), st);
   gp->sorted_coord = DevBuf(size_t(M) * 16, st);
   launch_gather_coords(true, coord, 2, 1, 2, gp->perm.as<uint32_t>(), M, gp->sorted_coord.p, st);
-  gp->chunks = DevBuf((size_t(gp->ntiles) + M / s.chunk + 2) * sizeof(Chunk), st);
-  gp->cws = DevBuf(group_chunk_workspace_bytes(gp->ntiles), st);
+  if (type1) {
+    gp->sel = DevBuf(size_t(M) * 4, st);
+    gp->cws = DevBuf(group_select_workspace_bytes(gp->ntiles), st);
+  } else {
+    gp->chunks = DevBuf((size_t(gp->ntiles) + M / s.chunk + 2) * sizeof(Chunk), st);
+    gp->cws = DevBuf(group_chunk_workspace_bytes(gp->ntiles), st);
+  }
+  gp->gcount.assign(ngroups, 0u);
+  DevBuf counts(size_t(ngroups) * 4, st);
+  launch_group_counts(group, M, ngroups, counts.as<uint32_t>(), st);
+  DN_CUDA(cudaMemcpyAsync(gp->gcount.data(), counts.p, size_t(ngroups) * 4,
+                          cudaMemcpyDeviceToHost, st));
   if (perm_out)
     DN_CUDA(cudaMemcpyAsync(perm_out, gp->perm.p, size_t(M) * 4, cudaMemcpyDeviceToDevice, st));
   const size_t vb = calc_f64 ? 16 : 8;
@@ -1927,7 +1978,7 @@ void grouped_plan_destroy(GroupedPlan *gp, cudaStream_t st) {
   if (!gp) return;
   // buffers go back to the pool in the order of the stream that last used them
   for (DevBuf *b : {&gp->sorted_coord, &gp->perm, &gp->start, &gp->chunks, &gp->cws, &gp->grid,
-                    &gp->work})
+                    &gp->work, &gp->sel})
     b->st = st;
   delete gp;
 }
@@ -1966,8 +2017,16 @@ static View plain_view(void *data, int dtype, int ndim, int64_t s0, int64_t s1 =
 bool grouped_nu2u(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *values, void *out,
                   bool forward, cudaStream_t st) {
   const Setup &s = gp->s;
-  if (!grouped_chunks(gp, g0, g1, st)) return false;
-  const ChunkList cl{gp->chunks.as<Chunk>(), gp->nchunks};
+  DN_REQUIRE(gp->type1, ST_INTERNAL, "grouped index made for type 2");
+  const uint32_t n = uint32_t(gp->run_points(g0, g1));
+  if (n == 0) return false;
+  if (gp->g1 == 0 || gp->g0 != g0 || gp->g1 != g1) {
+    build_group_select(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1,
+                       gp->sel.as<uint32_t>(), gp->cws.p, st);
+    gp->g0 = g0;
+    gp->g1 = g1;
+  }
+  const ChunkList cl{nullptr, 0};
   const PointsDesc pts{gp->sorted_coord.p, 2, 1, true, true, gp->perm.as<uint32_t>(),
                        s.npoints};
   const int dt = s.calc_f64 ? DNUFFT_C128 : DNUFFT_C64;
@@ -1976,10 +2035,10 @@ bool grouped_nu2u(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *values,
   StageTimer tm(false, st);
   if (s.calc_f64)
     do_spread_fft<double>(s, *gp->dc, pts, cl, nullptr, vv, ov, forward, false, tm, st,
-                          &gp->grid, &gp->work);
+                          &gp->grid, &gp->work, gp->sel.as<uint32_t>(), n);
   else
     do_spread_fft<float>(s, *gp->dc, pts, cl, nullptr, vv, ov, forward, false, tm, st,
-                         &gp->grid, &gp->work);
+                         &gp->grid, &gp->work, gp->sel.as<uint32_t>(), n);
   return true;
 }
 
@@ -1988,7 +2047,8 @@ bool grouped_nu2u(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *values,
 bool grouped_u2nu(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *uni, void *out,
                   bool forward, cudaStream_t st) {
   const Setup &s = gp->s;
-  if (!grouped_chunks(gp, g0, g1, st)) return false;
+  DN_REQUIRE(!gp->type1, ST_INTERNAL, "grouped index made for type 1");
+  if (gp->run_points(g0, g1) == 0 || !grouped_chunks(gp, g0, g1, st)) return false;
   const ChunkList cl{gp->chunks.as<Chunk>(), gp->nchunks};
   const PointsDesc pts{gp->sorted_coord.p, 2, 1, true, true, gp->perm.as<uint32_t>(),
                        s.npoints};
@@ -2221,15 +2281,16 @@ int dnufft_plan_get_permutation(const dnufft_plan *p, uint32_t *out, void *strea
     DN_REQUIRE(p && out, dnufft::ST_BADARG, "null argument");
     if (p->s.npoints == 0) return DNUFFT_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!p->s.qbits) {
+    if (p->s.tile_shift == 0 || p->s.g.ndim != 2) {
       DN_CUDA(cudaMemcpyAsync(out, p->ix.perm.p, size_t(p->s.npoints) * 4, cudaMemcpyDefault, st));
     } else {
-      // the plan processes points in (tile, quadrant, cell) order; DUCC's
-      // permutation is the stable order by tile alone: re-sort the original
-      // coordinates
+      // the plan processes points in an order of its own inside every tile;
+      // DUCC's permutation is the stable order by tile alone: re-sort the
+      // original coordinates
       dnufft::Setup s2 = p->s;
       s2.qbits = false;
-      s2.keybits -= 2 + dnufft::tc_cell_bits(s2.g);
+      s2.order = dnufft::TileOrder();
+      s2.keybits = std::max(1, dnufft::bitlen64(s2.max_tiles));
       s2.tile_shift = 0;
       s2.chunk = dnufft::CHUNK;
       const uint32_t M = s2.npoints;
@@ -2242,7 +2303,7 @@ int dnufft_plan_get_permutation(const dnufft_plan *p, uint32_t *out, void *strea
       dnufft::launch_scatter_coords(s2.coord_f64, p->sorted_coord.p, nd, p->ix.perm.as<uint32_t>(),
                                     M, orig.p, st);
       dnufft::launch_fold_keys(s2.coord_f64, orig.p, nd, 1, M, s2.g, ix2.keys.as<uint32_t>(),
-                               ix2.perm.as<uint32_t>(), st, false);
+                               ix2.perm.as<uint32_t>(), st);
       dnufft::DevBuf ws(dnufft::radix_workspace_bytes(M, s2.keybits), st);
       dnufft::radix_sort_pairs(ix2.keys.as<uint32_t>(), ix2.perm.as<uint32_t>(), M, s2.keybits,
                                ws.p, st);
@@ -2300,6 +2361,7 @@ struct dnufft_batch {
   int max_ntrans = 1;
   uint32_t nchunks = 0;
   size_t sm_spread = 0, sm_interp = 0;
+  uint32_t nruns = 0, ppw = 32;   // spreading launch: CTAs, points per warp
   dnufft::DevBuf grids, insts, tab;
   void *fftb = nullptr;
   dnufft::BatchArray *htab = nullptr;    // pinned: [points | uniform] x nplans
@@ -2337,7 +2399,11 @@ static void batch_build(dnufft_batch *b, cudaStream_t st) {
     total += grid_cells(p->s.g) * size_t(b->ntrans[size_t(i)]) * sizeof(T) * 2;
   }
   b->grids = DevBuf(total, st);
-  uint32_t c0 = 0;
+  uint32_t c0 = 0, r0 = 0;
+  uint64_t points = 0;
+  for (int i = 0; i < n; ++i)
+    points += uint64_t(b->plans[size_t(i)]->s.npoints) * uint64_t(b->ntrans[size_t(i)]);
+  b->ppw = spread_multi_ppw(points);
   for (int i = 0; i < n; ++i) {
     const dnufft_plan *p = b->plans[size_t(i)];
     SpreadInst<T> &s = si[size_t(i)];
@@ -2352,6 +2418,8 @@ static void batch_build(dnufft_batch *b, cudaStream_t st) {
     s.ntrans = b->ntrans[size_t(i)];
     s.chunk0 = c0;
     c0 += p->ix.nchunks;
+    s.run0 = r0;
+    r0 += spread_multi_ctas<T>(p->s.npoints, b->ppw);
     b->sm_spread = std::max(b->sm_spread, spread_multi_smem<T>(p->s.g));
     b->sm_interp = std::max(b->sm_interp, interp_multi_smem<T>(p->s.g));
     FFTBatchInst &f = fi[size_t(i)];
@@ -2363,6 +2431,7 @@ static void batch_build(dnufft_batch *b, cudaStream_t st) {
     f.fft_order = p->o.fft_order != 0;
   }
   b->nchunks = c0;
+  b->nruns = r0;
   b->insts = DevBuf(si.size() * sizeof(SpreadInst<T>), st);
   DN_CUDA(cudaMemcpyAsync(b->insts.p, si.data(), si.size() * sizeof(SpreadInst<T>),
                           cudaMemcpyHostToDevice, st));
@@ -2451,7 +2520,7 @@ static void batch_record(dnufft_batch *b, int type, bool fwd, cudaStream_t cs) {
     for (int i = 0; i < n; ++i)
       bytes += grid_cells(b->plans[size_t(i)]->s.g) * size_t(b->ntrans[size_t(i)]) * sizeof(T) * 2;
     DN_CUDA(cudaMemsetAsync(b->grids.p, 0, bytes, cs));
-    launch_spread_multi<T>(insts, n, b->nchunks, b->max_ntrans, b->sm_spread, tab, cs);
+    launch_spread_multi<T>(insts, n, b->nruns, b->ppw, b->max_ntrans, b->sm_spread, tab, cs);
     fft_batch_run<T>(b->fftb, 0, tab + n, fwd, cs);
   } else {
     fft_batch_run<T>(b->fftb, 1, tab + n, fwd, cs);

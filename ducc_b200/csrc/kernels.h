@@ -6,17 +6,23 @@
 namespace dnufft {
 
 // ---- binning / sorting (binsort.cu)
-// quadrant_bits: append the point's quadrant within its 2D tile as two extra
-// key bits and, below them, the Morton code of its cell within the quadrant
-// (2 * (log2tile - 1) bits): the tensor-core spreader's processing order
+// Order of the points inside a 2D tile, as key bits below the tile:
+// tensor core (quadrant): the point's quadrant within its tile and below it
+// the Morton code of its cell within the quadrant (2 * (log2tile - 1) bits);
+// runs: its bin of 8 x 8 cells within the tile (bin_bits, k_spread_run's order)
+struct TileOrder {
+  bool quadrant = false;
+  int bin_bits = 0;
+};
 void launch_fold_keys(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
                       uint32_t npts, const Geometry &g, uint32_t *keys, uint32_t *idx,
-                      cudaStream_t st, bool quadrant_bits = false);
+                      cudaStream_t st, TileOrder order = TileOrder());
 // bits of the within-quadrant cell order in a tensor-core sort key
 inline int tc_cell_bits(const Geometry &g) { return 2 * (g.log2tile - 1); }
 size_t scan_workspace_bytes(uint64_t n);
 void exclusive_scan(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *ws,
                     cudaStream_t st);
+constexpr int RADIX_BITS = 11;   // most key bits a radix pass sorts
 size_t radix_workspace_bytes(uint32_t n, int keybits);
 void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, void *ws,
                       cudaStream_t st);
@@ -46,6 +52,15 @@ uint32_t build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, u
 void launch_scatter_coords(bool coord_f64, const void *sorted, int ndim, const uint32_t *perm,
                            uint32_t n, void *out, cudaStream_t st);
 
+// the points of groups [g0, g1) of a grouped index, in key order: their sorted
+// positions into sel (one entry per point)
+size_t group_select_workspace_bytes(uint32_t nbins);
+void build_group_select(const uint32_t *start, uint32_t nbins, int gbits, uint32_t g0, uint32_t g1,
+                        uint32_t *sel, void *ws, cudaStream_t st);
+// counts[k] = number of points with group k < ngroups (counts zeroed first)
+void launch_group_counts(const uint32_t *group, uint32_t n, uint32_t ngroups, uint32_t *counts,
+                         cudaStream_t st);
+
 // ---- spreading / interpolation (spread_*.cu)
 struct PointsDesc {
   const void *coord;      // sorted==true: contiguous (npts, ndim) in tile order
@@ -69,6 +84,13 @@ void launch_spread(const PointsDesc &pts, const ChunkList &cl, const Geometry &g
                    const KernelPoly<T> &kp, const void *values, int64_t vs,
                    int64_t vtrans, void *grid, int64_t gtrans, int ntrans,
                    cudaStream_t st);
+
+// 2D (launch_spread goes here; no chunk list): the points sel[0 .. npts) of
+// the sorted order, or all npts of it (sel null)
+template <typename T>
+void launch_spread_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts,
+                       const Geometry &g, const KernelPoly<T> &kp, const void *values, int64_t vs,
+                       int64_t vtrans, void *grid, int64_t gtrans, int ntrans, cudaStream_t st);
 
 // err: device error word; with it, 2D single-transform tiles inside the grid
 // are staged by TMA (a copy that never completes sets the word)
@@ -205,13 +227,17 @@ template <typename T> struct SpreadInst {
   KernelPoly<T> kp;
   void *grid;        // ntrans grids back to back
   int ntrans;
-  uint32_t chunk0;   // first chunk of this instance in the launch
+  uint32_t chunk0;   // first chunk of this instance in the interpolation launch
+  uint32_t run0;     // first CTA of this instance in the spreading launch
 };
-// one launch over the chunks of all instances (x) and their transforms (y);
-// vals: per-call table of the point arrays (type 1 input, type 2 output)
+// one launch over the chunks (interpolation) or runs of points (spreading:
+// ppw points per warp) of all instances (x) and their transforms (y); vals:
+// per-call table of the point arrays (type 1 input, type 2 output)
+uint32_t spread_multi_ppw(uint64_t total_points);
+template <typename T> uint32_t spread_multi_ctas(uint32_t npts, uint32_t ppw);
 template <typename T>
-void launch_spread_multi(const SpreadInst<T> *insts, int ninst, uint32_t nchunks, int max_ntrans,
-                         size_t smem, const BatchArray *vals, cudaStream_t st);
+void launch_spread_multi(const SpreadInst<T> *insts, int ninst, uint32_t nctas, uint32_t ppw,
+                         int max_ntrans, size_t smem, const BatchArray *vals, cudaStream_t st);
 template <typename T>
 void launch_interp_multi(const SpreadInst<T> *insts, int ninst, uint32_t nchunks, int max_ntrans,
                          size_t smem, const BatchArray *vals, cudaStream_t st);

@@ -1,4 +1,5 @@
-// Plain spreading (type 1) and interpolation (type 2) kernels.
+// Plain spreading (type 1; 1D and 3D, 2D: spread_run.cuh) and interpolation
+// (type 2) kernels.
 //
 // One CTA per chunk of tile-sorted points (at most CHUNK points of one tile).
 // Spreading: every warp takes 32 points at a time, each lane folds its point
@@ -116,8 +117,7 @@ __device__ __forceinline__ int64_t cell_index(int c, int S, uint32_t mS, bool fa
   return gidx;
 }
 
-// One chunk of one transform (the body of k_spread; also used by the
-// multi-instance kernel of batched transforms).
+// One chunk of one transform (the body of k_spread).
 template <typename T, typename Tc, int NDIM, int W>
 __device__ __forceinline__ void spread_chunk(const PointsDesc &pts, const Chunk ch, const Geometry &g,
                                              const KernelPoly<T> &kp,
@@ -193,10 +193,6 @@ __device__ __forceinline__ void spread_chunk(const PointsDesc &pts, const Chunk 
           if constexpr (NDIM == 1) {
             wt = wp[c];
             cell = o[0] + c;
-          } else if constexpr (NDIM == 2) {
-            int a = c / W, b = c - (c / W) * W;
-            wt = wp[a] * wp[W + b];
-            cell = (o[0] + a) * S + (o[1] + b);
           } else {
             int a = c / (W * W), r = c - a * (W * W), b = r / W, e = r - b * W;
             wt = wp[a] * wp[W + b] * wp[2 * W + e];
@@ -226,8 +222,7 @@ __device__ __forceinline__ void spread_chunk(const PointsDesc &pts, const Chunk 
 }
 
 // four CTAs per SM for single-precision values at float64 coordinates (whose
-// exact fold takes many registers): sparse tiles, where the CTAs are short,
-// need the warps
+// exact fold takes many registers)
 template <typename T, typename Tc> constexpr int spread_min_ctas() {
   return (sizeof(T) == 4 && sizeof(Tc) == 8) ? 4 : 1;
 }
@@ -719,12 +714,17 @@ void launch_spread_impl(const PointsDesc &pts, const ChunkList &cl, const Geomet
                         const KernelPoly<T> &kp, const void *values, int64_t vs,
                         int64_t vtrans, void *grid, int64_t gtrans, int ntrans,
                         cudaStream_t st) {
+  if (g.ndim == 2) {
+    launch_spread_run<T>(pts, nullptr, pts.npts, g, kp, values, vs, vtrans, grid, gtrans, ntrans,
+                         st);
+    return;
+  }
   if (cl.nchunks == 0 || ntrans == 0) return;
 #define DN_SD(TC, ND) spread_dispatch<T, TC, ND>(pts, cl, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st)
   if (pts.coord_f64) {
-    if (g.ndim == 1) DN_SD(double, 1); else if (g.ndim == 2) DN_SD(double, 2); else DN_SD(double, 3);
+    if (g.ndim == 1) DN_SD(double, 1); else DN_SD(double, 3);
   } else {
-    if (g.ndim == 1) DN_SD(float, 1); else if (g.ndim == 2) DN_SD(float, 2); else DN_SD(float, 3);
+    if (g.ndim == 1) DN_SD(float, 1); else DN_SD(float, 3);
   }
 #undef DN_SD
 }

@@ -918,11 +918,11 @@ struct Grouped {
   GroupedPlan *gp = nullptr;
   cudaStream_t st = nullptr;
   Grouped(const double *coord, uint32_t n, const uint32_t *key, const Params &P, int64_t nx,
-          int64_t ny, double eps, bool f64, const dnufft_opts &no, cudaStream_t s)
+          int64_t ny, double eps, bool f64, const dnufft_opts &no, bool type1, cudaStream_t s)
       : st(s) {
     const int64_t shape[2] = {nx, ny};
     gp = grouped_plan_create(coord, n, key, uint32_t(P.nplanes), shape, eps, f64, no, s,
-                             nullptr);
+                             type1, nullptr);
   }
   Grouped(const Grouped &) = delete;
   Grouped &operator=(const Grouped &) = delete;
@@ -981,7 +981,7 @@ static void vis2dirty_t(const Inputs &in, double psx, double psy, double eps,
   Buf key;
   plane_keys(ptr<double>(cv.wv), cv.nvis, P, key, st);
   Grouped gr(ptr<double>(cv.coord), cv.nvis, ptr<uint32_t>(key), P, nx, ny, eps, sizeof(C) == 8,
-             no, st);
+             no, true, st);
   const CorrNodes cn = make_nodes(P.W, P.beta, P.e0);
   if (gr.gp) {
     for (int64_t p = pl0; p < pl1; ++p) {
@@ -1084,7 +1084,7 @@ static void dirty2vis_t(const Inputs &in, const Arr &dirty, double psx, double p
   Buf key;
   plane_keys(ptr<double>(cv.wv), cv.nvis, P, key, st);
   Grouped gr(ptr<double>(cv.coord), cv.nvis, ptr<uint32_t>(key), P, nx, ny, eps, sizeof(C) == 8,
-             no, st);
+             no, false, st);
   if (gr.gp) {
     for (int64_t p = pl0; p < pl1; ++p) {
       const uint32_t g0 = uint32_t(std::max<int64_t>(0, p - P.W + 1)), g1 = uint32_t(p + 1);

@@ -43,10 +43,9 @@ extern "C" {
 #define DNUFFT_U8 5    /* masks of the w-gridder                                 */
 
 /* spreader selection (type 1) */
-/* AUTO: the tensor-core form for 2D complex64 type 1 with at least 0.5 points
-   per uniform mode (where it is measured faster), else plain */
+/* AUTO: plain (measured faster than the tensor-core form everywhere) */
 #define DNUFFT_SPREAD_AUTO 0
-#define DNUFFT_SPREAD_PLAIN 1  /* per-point FP32/FP64 atomics in shared memory   */
+#define DNUFFT_SPREAD_PLAIN 1  /* FP32/FP64 sums, in registers (2D) or shared memory */
 #define DNUFFT_SPREAD_TC 2     /* split-precision FP16 tcgen05 tile contraction  */
 
 typedef struct dnufft_array {

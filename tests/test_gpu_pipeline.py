@@ -2,8 +2,7 @@
 groups whose host->device copies (and, for type 2, device->host copies of the
 results) overlap the sorting and spreading / interpolation of the other
 groups.  Checked against the same calls on device arrays (one group, no
-overlap), in complex64 (tensor-core spreader chosen by 'auto' at this density)
-and complex128, both signs, and against the direct NUDFT on a sample of
+overlap), in complex64 and complex128, both signs, and against the direct NUDFT on a sample of
 modes / points.
 """
 import numpy as np

@@ -22,7 +22,7 @@ def _problem(ndim, M, single, seed):
     return coord, vals
 
 
-CASES = [((256, 240), 400_000, True, 1e-6),     # tensor-core spreader ('auto')
+CASES = [((256, 240), 400_000, True, 1e-6),     # dense
          ((96, 80), 30_000, True, 1e-5),        # plain
          ((96, 80), 30_000, False, 1e-11),
          ((400,), 20_000, False, 1e-10),

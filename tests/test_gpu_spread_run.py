@@ -1,0 +1,97 @@
+"""The spreading and interpolation kernels on their own (plan.spread,
+plan.interp) against the FP64 oracle, for every kernel support and at the sizes
+where they can go wrong: oversampled grids down to 16 cells (windows that wrap
+around the grid), numbers of points around a warp's batch, points on bin and
+grid edges, a clustered set (one bin), and values that are not finite.
+
+Tolerances: single precision, the Horner evaluation of degree D = W + 3 <= 11
+and the product of the weights round at most 2 (2 D + 2) 2^-24 = 3e-6 relative
+to the largest weights; double, the polynomial coefficients of planner and
+oracle agree to about 1e-11.
+"""
+import numpy as np
+import pytest
+
+from ducc_b200 import nufft
+from oracle import nufft_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _force(W, single, nover, ndim):
+    """(kernel row, oversampled shape) with support W."""
+    for k, row in enumerate(O.kernel_db()):
+        if row[0] == W and row[6] == single and row[5] == ndim:
+            return k, nover
+    pytest.skip("no kernel of this support")
+
+
+def _coords(kind, M, nover, rng):
+    ndim = len(nover)
+    if kind == "uniform":
+        return rng.uniform(-np.pi, np.pi, (M, ndim))
+    if kind == "bin":      # all in a few cells
+        return rng.uniform(0.3, 0.3 + 3 * 2 * np.pi / max(nover), (M, ndim))
+    # cell edges, the first and the last cells of the period included
+    n = np.array(nover)
+    return rng.integers(-n, n, (M, ndim)) * (2 * np.pi / n)
+
+
+def _case(W, single, shape, nover, M, kind, seed=1):
+    rng = np.random.default_rng(seed)
+    ct = np.float32 if single else np.float64
+    coord = _coords(kind, M, nover, rng).astype(ct)
+    vals = (rng.standard_normal(M) + 1j * rng.standard_normal(M)).astype(
+        np.complex64 if single else np.complex128)
+    k, nov = _force(W, single, nover, len(shape))
+    p = O.Params(shape, 1e-3, single, M, True, force=(k, nov))
+    return p, k, nov, coord, vals
+
+
+GRIDS2 = [((5, 6), (16, 16)), ((9, 40), (18, 88)), ((30, 13), (64, 28)), ((50, 60), (110, 126))]
+
+
+def _run(W, single, shape, nover, M, kind):
+    import torch
+    p, k, nov, coord, vals = _case(W, single, shape, nover, M, kind)
+    plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=shape,
+                      epsilon=1e-3, force_kernel=k, force_nover=nov, spreader="plain")
+    got = plan.spread(points=torch.from_numpy(vals).cuda())
+    tol = 3e-6 if single else 1e-10
+    assert O.l2error(got.cpu().numpy(), O.spread(p, coord, vals)) < tol
+    rng = np.random.default_rng(5)
+    grid = (rng.standard_normal(nov) + 1j * rng.standard_normal(nov)).astype(vals.dtype)
+    out = plan.interp(grid=torch.from_numpy(grid).cuda())
+    assert O.l2error(out.cpu().numpy(), O.interpolate(p, grid, coord)) < tol
+
+
+@pytest.mark.parametrize("W", range(4, 9))
+@pytest.mark.parametrize("shape,nover", GRIDS2)
+@pytest.mark.parametrize("M,kind", [(1, "uniform"), (33, "edges"), (300, "bin"), (2500, "uniform")])
+def test_2d_single(W, shape, nover, M, kind):
+    _run(W, True, shape, nover, M, kind)
+
+
+@pytest.mark.parametrize("W", range(4, 17))
+@pytest.mark.parametrize("shape,nover", GRIDS2)
+@pytest.mark.parametrize("M,kind", [(1, "uniform"), (17, "edges"), (300, "bin"), (2500, "uniform")])
+def test_2d_double(W, shape, nover, M, kind):
+    _run(W, False, shape, nover, M, kind)
+
+
+@pytest.mark.parametrize("single", [True, False])
+def test_nonfinite_value_stays_in_its_footprint(single):
+    import torch
+    W = 6
+    p, k, nov, coord, vals = _case(W, single, (50, 60), (110, 126), 200, "uniform")
+    vals[77] = np.inf
+    plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=(50, 60),
+                      epsilon=1e-3, force_kernel=k, force_nover=nov, spreader="plain")
+    got = plan.spread(points=torch.from_numpy(vals).cuda()).cpu().numpy()
+    i0, _ = O.getpix(p, coord[77:78])
+    bad = np.zeros(nov, bool)
+    bad[np.ix_((i0[0, 0] + np.arange(W)) % nov[0], (i0[0, 1] + np.arange(W)) % nov[1])] = True
+    assert np.array_equal(~np.isfinite(got), bad)
+    vals[77] = 0
+    ref = O.spread(p, coord, vals)
+    assert O.l2error(got[~bad], ref[~bad]) < (3e-6 if single else 1e-10)
