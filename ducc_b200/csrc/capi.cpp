@@ -342,6 +342,7 @@ struct Setup {
   TileOrder order;      // the key bits below the tile (2D)
   int keybits = 1;
   int tile_shift = 0;
+  int ducc_keybits = 1;   // of DUCC's tile key (the stable order permutation() returns)
   uint64_t max_tiles = 0;
   uint32_t chunk = CHUNK;   // largest chunk (consecutive sorted points of one tile)
 };
@@ -463,6 +464,7 @@ static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double 
   // every density measured (W = 8, spreading alone: 5e7 clustered points on
   // 4096^2 modes 2.02 against 3.49 ms, 8e6 points on 1024^2 0.31 / 0.51 ms,
   // 2e4 points 0.04 / 0.08 ms) and the more accurate one
+  s.ducc_keybits = std::max(1, bitlen64(maxkey));
   if (s.spreader == DNUFFT_SPREAD_TC && spread_tc_supported(g, calc_f64)) {
     s.qbits = true;
     s.order.quadrant = true;
@@ -477,6 +479,15 @@ static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double 
     if (bitlen64(maxkey) + bb <= 32) {
       s.order.bin_bits = bb;
       s.tile_shift = bb;
+    }
+  } else if (run_order && ndim == 3) {
+    // bins and, inside them, the first axis, where the key has room for them
+    const int lb = spread_run3_bin_log2(g.W), bb = 3 * (g.log2tile - lb);
+    if (bitlen64(s.max_tiles) + bb + lb <= 32) {
+      s.order.bin_bits = bb;
+      s.order.bin_log2 = lb;
+      s.tile_shift = bb + lb;
+      maxkey = s.max_tiles << lb;   // (bin_bits are added below)
     }
   }
   DN_REQUIRE(maxkey < (uint64_t(1) << 32), ST_UNSUPPORTED, "tile key space too large");
@@ -597,7 +608,7 @@ static uint32_t sm_count() {
   return uint32_t(n > 0 ? n : 1);
 }
 
-// need_chunks: the chunk list too (the 2D plain spreader needs none; the
+// need_chunks: the chunk list too (the 2D and 3D plain spreaders need none; the
 // number of chunks is read back to the host, which waits for the sort)
 static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream_t st,
                         bool need_chunks = true) {
@@ -630,7 +641,7 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
 }
 
 // does type 1 of this setup work from a chunk list?
-static bool spread_needs_chunks(const Setup &s) { return s.g.ndim != 2 || s.qbits; }
+static bool spread_needs_chunks(const Setup &s) { return s.g.ndim == 1 || s.qbits; }
 
 static size_t grid_cells(const Geometry &g) {
   size_t c = 1;
@@ -2281,7 +2292,7 @@ int dnufft_plan_get_permutation(const dnufft_plan *p, uint32_t *out, void *strea
     DN_REQUIRE(p && out, dnufft::ST_BADARG, "null argument");
     if (p->s.npoints == 0) return DNUFFT_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (p->s.tile_shift == 0 || p->s.g.ndim != 2) {
+    if (!p->s.qbits && p->s.order.bin_bits == 0) {
       DN_CUDA(cudaMemcpyAsync(out, p->ix.perm.p, size_t(p->s.npoints) * 4, cudaMemcpyDefault, st));
     } else {
       // the plan processes points in an order of its own inside every tile;
@@ -2290,8 +2301,7 @@ int dnufft_plan_get_permutation(const dnufft_plan *p, uint32_t *out, void *strea
       dnufft::Setup s2 = p->s;
       s2.qbits = false;
       s2.order = dnufft::TileOrder();
-      s2.keybits = std::max(1, dnufft::bitlen64(s2.max_tiles));
-      s2.tile_shift = 0;
+      s2.keybits = s2.ducc_keybits;
       s2.chunk = dnufft::CHUNK;
       const uint32_t M = s2.npoints;
       const int nd = s2.g.ndim;

@@ -6,14 +6,16 @@
 namespace dnufft {
 
 // ---- binning / sorting (binsort.cu)
-// Order of the points inside a 2D tile, as key bits below the tile:
-// tensor core (quadrant): the point's quadrant within its tile and below it
+// Order of the points inside a 2D or 3D tile, as key bits below the tile:
+// tensor core (2D, quadrant): the point's quadrant within its tile and below it
 // the Morton code of its cell within the quadrant (2 * (log2tile - 1) bits);
-// runs: its bin of 8 x 8 cells within the tile (bin_bits, k_spread_run's order)
+// runs: its bin of (2^bin_log2)^d cells within the tile (bin_bits), and in 3D
+// its first-axis position in the bin (the order of k_spread_run, k_spread_run3)
 struct TileOrder {
   bool quadrant = false;
-  int bin_bits = 0;
+  int bin_bits = 0, bin_log2 = 3;
 };
+int spread_run3_bin_log2(int W);
 void launch_fold_keys(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
                       uint32_t npts, const Geometry &g, uint32_t *keys, uint32_t *idx,
                       cudaStream_t st, TileOrder order = TileOrder());
@@ -91,6 +93,12 @@ template <typename T>
 void launch_spread_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts,
                        const Geometry &g, const KernelPoly<T> &kp, const void *values, int64_t vs,
                        int64_t vtrans, void *grid, int64_t gtrans, int ntrans, cudaStream_t st);
+
+// 3D (launch_spread goes here; no chunk list)
+template <typename T>
+void launch_spread_run3(const PointsDesc &pts, const Geometry &g, const KernelPoly<T> &kp,
+                        const void *values, int64_t vs, int64_t vtrans, void *grid,
+                        int64_t gtrans, int ntrans, cudaStream_t st);
 
 // err: device error word; with it, 2D single-transform tiles inside the grid
 // are staged by TMA (a copy that never completes sets the word)

@@ -719,12 +719,16 @@ void launch_spread_impl(const PointsDesc &pts, const ChunkList &cl, const Geomet
                          st);
     return;
   }
+  if (g.ndim == 3) {
+    launch_spread_run3<T>(pts, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st);
+    return;
+  }
   if (cl.nchunks == 0 || ntrans == 0) return;
 #define DN_SD(TC, ND) spread_dispatch<T, TC, ND>(pts, cl, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st)
   if (pts.coord_f64) {
-    if (g.ndim == 1) DN_SD(double, 1); else DN_SD(double, 3);
+    DN_SD(double, 1);
   } else {
-    if (g.ndim == 1) DN_SD(float, 1); else DN_SD(float, 3);
+    DN_SD(float, 1);
   }
 #undef DN_SD
 }

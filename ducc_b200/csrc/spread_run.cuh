@@ -38,6 +38,8 @@
 // Mirrors HelperNu2u / spreading_helper (src/ducc0/nufft/nufft.h:917-1204).
 #pragma once
 
+#include <algorithm>
+
 #include "spread_impl.cuh"
 
 namespace dnufft {
@@ -311,11 +313,13 @@ __device__ __forceinline__ void spread_run(const PointsDesc &pts, const uint32_t
   if (cu >= 0) flush();
 }
 
-// points per warp: a multiple of 32; about 24 warps per SM get work before
-// longer runs save flushes
+// points per warp: about 24 warps per SM get work before longer runs save
+// flushes; a multiple of 32 from 32 up, at least 8 (few points: a warp adds its
+// points one after the other, so more warps finish sooner)
 inline uint32_t run_points_per_warp(uint64_t npts) {
-  uint64_t p = npts / (148 * 24) / 32 * 32;
-  return uint32_t(p < 32 ? 32 : (p > 256 ? 256 : p));
+  const uint64_t p = npts / (148 * 24);
+  return uint32_t(p < 32 ? std::max<uint64_t>(8, p & ~uint64_t(7))
+                         : std::min<uint64_t>(256, p & ~uint64_t(31)));
 }
 
 template <typename T, typename Tc, int W>

@@ -79,18 +79,36 @@ def test_2d_double(W, shape, nover, M, kind):
     _run(W, False, shape, nover, M, kind)
 
 
+GRIDS3 = [((3, 4, 5), (16, 16, 16)), ((10, 5, 20), (22, 18, 44)), ((15, 20, 9), (36, 48, 20))]
+
+
+@pytest.mark.parametrize("W", range(4, 9))
+@pytest.mark.parametrize("shape,nover", GRIDS3)
+@pytest.mark.parametrize("M,kind", [(1, "uniform"), (129, "edges"), (300, "bin"), (1500, "uniform")])
+def test_3d_single(W, shape, nover, M, kind):
+    _run(W, True, shape, nover, M, kind)
+
+
+@pytest.mark.parametrize("W", range(4, 17))
+@pytest.mark.parametrize("shape,nover", GRIDS3)
+@pytest.mark.parametrize("M,kind", [(1, "uniform"), (65, "edges"), (300, "bin"), (900, "uniform")])
+def test_3d_double(W, shape, nover, M, kind):
+    _run(W, False, shape, nover, M, kind)
+
+
 @pytest.mark.parametrize("single", [True, False])
-def test_nonfinite_value_stays_in_its_footprint(single):
+@pytest.mark.parametrize("shape,nover", [((50, 60), (110, 126)), ((15, 20, 9), (36, 48, 20))])
+def test_nonfinite_value_stays_in_its_footprint(single, shape, nover):
     import torch
     W = 6
-    p, k, nov, coord, vals = _case(W, single, (50, 60), (110, 126), 200, "uniform")
+    p, k, nov, coord, vals = _case(W, single, shape, nover, 200, "uniform")
     vals[77] = np.inf
-    plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=(50, 60),
+    plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=shape,
                       epsilon=1e-3, force_kernel=k, force_nover=nov, spreader="plain")
     got = plan.spread(points=torch.from_numpy(vals).cuda()).cpu().numpy()
     i0, _ = O.getpix(p, coord[77:78])
     bad = np.zeros(nov, bool)
-    bad[np.ix_((i0[0, 0] + np.arange(W)) % nov[0], (i0[0, 1] + np.arange(W)) % nov[1])] = True
+    bad[np.ix_(*[(i0[0, d] + np.arange(W)) % nov[d] for d in range(len(nov))])] = True
     assert np.array_equal(~np.isfinite(got), bad)
     vals[77] = 0
     ref = O.spread(p, coord, vals)
