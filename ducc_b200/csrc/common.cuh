@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <cstring>
 
 #include "dnufft_internal.h"
 
@@ -58,17 +59,60 @@ __device__ __forceinline__ void fold_f32(double x, double coordfct, int n, doubl
 
 typedef unsigned __int128 u128;
 
-__device__ __forceinline__ int bitlen128(u128 v) {
+__host__ __device__ __forceinline__ int clz64(uint64_t v) {
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)v);
+#else
+  return __builtin_clzll(v);
+#endif
+}
+// binary64 operations that are never contracted
+__host__ __device__ __forceinline__ double mul_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  volatile double r = a * b;
+  return r;
+#endif
+}
+__host__ __device__ __forceinline__ double add_rn(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dadd_rn(a, b);
+#else
+  volatile double r = a + b;
+  return r;
+#endif
+}
+__host__ __device__ __forceinline__ uint64_t bits_of(double a) {
+#ifdef __CUDA_ARCH__
+  return uint64_t(__double_as_longlong(a));
+#else
+  uint64_t r;
+  memcpy(&r, &a, 8);
+  return r;
+#endif
+}
+__host__ __device__ __forceinline__ double of_bits(uint64_t a) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)a);
+#else
+  double r;
+  memcpy(&r, &a, 8);
+  return r;
+#endif
+}
+
+__host__ __device__ __forceinline__ int bitlen128(u128 v) {
   uint64_t hi = uint64_t(v >> 64), lo = uint64_t(v);
-  if (hi) return 128 - __clzll((long long)hi);
-  if (lo) return 64 - __clzll((long long)lo);
+  if (hi) return 128 - clz64(hi);
+  if (lo) return 64 - clz64(lo);
   return 0;
 }
 
 // Round v (whose true value may exceed v by less than one unit in the last
 // place when 'sticky' is set) to 'keep' significant bits, round-to-nearest-even.
 // Returns the rounded integer and the number of dropped bits in *drop.
-__device__ __forceinline__ u128 round_sig(u128 v, bool sticky, int keep, int *drop) {
+__host__ __device__ __forceinline__ u128 round_sig(u128 v, bool sticky, int keep, int *drop) {
   int bl = bitlen128(v);
   if (bl <= keep) {
     *drop = 0;
@@ -88,12 +132,12 @@ __device__ __forceinline__ u128 round_sig(u128 v, bool sticky, int keep, int *dr
   return r;
 }
 
-__device__ __forceinline__ void fold_f64(double x, double coordfct, int n, double shift,
-                                         int maxi0, int &i0, double &frac) {
-  double tmp = __dmul_rn(x, coordfct);
-  double f = tmp - floor(tmp);
+// the fold of a fractional position f in 128-bit integers (any f)
+__host__ __device__ __noinline__ inline void fold_f64_int(double f, int n, double shift, int maxi0,
+                                                          int *i0_, double *frac_) {
+  int i0;
   // exact f = mant * 2^e
-  uint64_t bits = uint64_t(__double_as_longlong(f));
+  uint64_t bits = bits_of(f);
   int ex = int((bits >> 52) & 0x7ff);
   uint64_t mant = bits & ((uint64_t(1) << 52) - 1);
   int e;
@@ -134,7 +178,52 @@ __device__ __forceinline__ void fold_f64(double x, double coordfct, int n, doubl
   u128 D64 = round_sig(Dv, sticky, 64, &drop);
   int drop2;
   u128 D53 = round_sig(D64, false, 53, &drop2);
-  frac = ldexp(double(uint64_t(D53)), drop + drop2 - 64);
+  *i0_ = i0;
+  *frac_ = ldexp(double(uint64_t(D53)), drop + drop2 - 64);
+}
+
+// 1.5 * 2^(ex(a) - 11) for a normal a > 2^-1000: adding and subtracting it
+// rounds a small number to the last place of a 64-bit significand of a's
+// exponent (nearest even: the upper 53 bits are an even number of those places)
+__host__ __device__ __forceinline__ double round64_magic(double a) {
+  return of_bits((bits_of(a) & 0x7ff0000000000000ull) - (uint64_t(11) << 52) +
+                 0x0008000000000000ull);
+}
+
+// The same fold in pairs of doubles (about 40 instructions for 400): the
+// product f * n is hi + lo exactly, its rounding to 64 bits touches lo alone,
+// and every following sum stays exact in two doubles as long as the operands'
+// exponents are within 38 of one another.  Where that, or the exponent of a sum
+// (its upper part a power of two), or the integer part (within 2^-29 of an
+// integer) is in doubt, the integer version decides.
+__host__ __device__ __forceinline__ void fold_f64(double x, double coordfct, int n, double shift,
+                                                  int maxi0, int &i0, double &frac) {
+  const double tmp = mul_rn(x, coordfct);
+  const double f = add_rn(tmp, -floor(tmp));
+  const double dn = double(n);
+  const double hi = mul_rn(f, dn), lo = fma(f, dn, -hi);
+  const double m1 = round64_magic(hi);
+  const double lo64 = add_rn(add_rn(lo, m1), -m1);
+  // integer part of hi + lo64 + shift (shift: a multiple of 1/2)
+  const double ih = floor(hi), is = floor(shift);
+  const double r = add_rn(add_rn(add_rn(hi, -ih), add_rn(shift, -is)), lo64);
+  const double fr = floor(r);
+  const int k = int(ih) + (int(is) - n) + int(fr);
+  const double off = add_rn(r, -fr);
+  bool ok = hi >= 0x1p-38 && (bits_of(hi) & 0x000fffffffffffffull) != 0 && off > 0x1p-29 &&
+            off < 1. - 0x1p-29;
+  i0 = k < maxi0 ? k : maxi0;
+  // hi + lo64 - i0 = s + l exactly
+  const double di = -double(i0);
+  const double s = add_rn(hi, di);
+  const double bb = add_rn(s, -hi);
+  const double e1 = add_rn(add_rn(hi, -add_rn(s, -bb)), add_rn(di, -bb));
+  const double l = add_rn(e1, lo64);
+  const double m2 = round64_magic(s);
+  const double l64 = add_rn(add_rn(l, m2), -m2);
+  ok = ok && s > 0x1p-38 && (bits_of(s) & 0x000fffffffffffffull) != 0;
+  frac = add_rn(s, l64);
+  if (!ok) fold_f64_int(f, n, shift, maxi0, &i0, &frac);
 }
 
 template <typename Tc>
