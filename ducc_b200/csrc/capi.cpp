@@ -640,8 +640,9 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
   }
 }
 
-// does type 1 of this setup work from a chunk list?
+// do type 1 / type 2 of this setup work from a chunk list?
 static bool spread_needs_chunks(const Setup &s) { return s.g.ndim == 1 || s.qbits; }
+static bool interp_needs_chunks(const Setup &s) { return s.g.ndim != 2 || !s.calc_f64; }
 
 static size_t grid_cells(const Geometry &g) {
   size_t c = 1;
@@ -726,7 +727,8 @@ template <typename T>
 static void do_fft_interp(const Setup &s, const DevConst &dc, const PointsDesc &pts,
                           const ChunkList &cl, const View &uni, const View &out, bool forward,
                           bool fft_order, StageTimer &tm, cudaStream_t st, DevBuf *ws = nullptr,
-                          DevBuf *wk = nullptr, SideStream *side = nullptr) {
+                          DevBuf *wk = nullptr, SideStream *side = nullptr,
+                          const uint32_t *sel = nullptr, uint32_t nsel = 0) {
   size_t cells = grid_cells(s.g);
   DevBuf local;
   DevBuf &grid = ws ? *ws : local;
@@ -749,7 +751,15 @@ static void do_fft_interp(const Setup &s, const DevConst &dc, const PointsDesc &
   tm.mark("interpolation");
   const KernelPoly<T> &kp = *reinterpret_cast<const KernelPoly<T> *>(
       sizeof(T) == 4 ? static_cast<const void *>(&s.kpf) : static_cast<const void *>(&s.kpd));
-  launch_interp<T>(pts, cl, s.g, kp, grid.p, 0, out.data, out.stride[0], 0, 1, st, err);
+  bool done = false;
+  if constexpr (sizeof(T) == 8) {
+    if (sel) {
+      launch_interp_run(pts, sel, nsel, s.g, kp, grid.p, 0, out.data, out.stride[0], 0, 1, st);
+      done = true;
+    }
+  }
+  if (!done)
+    launch_interp<T>(pts, cl, s.g, kp, grid.p, 0, out.data, out.stride[0], 0, 1, st, err);
   tm.mark("output copy");
   check_device_error(err, st);
 }
@@ -965,7 +975,7 @@ static void u2nu_pipelined(const Setup &s, const View &uni, const View &coord, c
     sg.npoints = uint32_t(b - a);
     const View cv = coord_range(coord, dcoord.p, a, b, cb);
     Index ix;
-    build_index(sg, cv, ix, st);
+    build_index(sg, cv, ix, st, interp_needs_chunks(sg));
     PointsDesc pts{cv.data, cv.stride[0], cv.stride[1], false, s.coord_f64,
                    ix.perm.as<uint32_t>(), sg.npoints};
     ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
@@ -1065,7 +1075,7 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   DN_REQUIRE(out.dtype == uni.dtype, ST_BADARG, "out must have the dtype of grid");
   bool f64 = uni.dtype == DNUFFT_C128;
   Setup s = make_setup(ndim, uni.shape, uint64_t(coord.shape[0]), eps, false, f64,
-                       coord.dtype == DNUFFT_F64, o);
+                       coord.dtype == DNUFFT_F64, o, f64 && ndim == 2);
   StageTimer tm(o.verbosity > 0, st);
   if (o.verbosity > 0) report_sizes(s, false);
   if (s.npoints == 0) return;
@@ -1094,7 +1104,7 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   side.start();   // the FFT pass may use the buffers from here on
   tm.mark("building index");
   Index ix;
-  build_index(s, sc.dev, ix, st);
+  build_index(s, sc.dev, ix, st, interp_needs_chunks(s));
   PointsDesc pts{sc.dev.data, sc.dev.stride[0], sc.dev.stride[1], false, s.coord_f64,
                  ix.perm.as<uint32_t>(), s.npoints};
   ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
@@ -1886,13 +1896,14 @@ int nu2u_in_scratch(const dnufft_array *points, const dnufft_array *coord, int f
 
 // ---------------------------------------------------------------- grouped index
 // A 2D index over points that belong to groups (the w-gridder's first w
-// plane), for type 1 or for type 2.  Type 2: sorted once by (tile, group), so
-// that within every tile the points of any run of groups are one contiguous
-// range, and a transform over such a run needs only a chunk list (one chunk per
-// tile and at most CHUNK points), not a sort of its own.  Type 1: sorted by
-// (tile, bin of 8 x 8 cells, group), and a transform takes the list of the
-// run's positions bin after bin (the plain spreader's order).  Kernel and grid
-// as forced in the options.
+// plane), for type 1 or for type 2.  Type 2 in single precision: sorted once by
+// (tile, group), so that within every tile the points of any run of groups are
+// one contiguous range, and a transform over such a run needs only a chunk list
+// (one chunk per tile and at most CHUNK points), not a sort of its own.  Type 1
+// and double precision ("runs"): sorted by (tile, bin of 8 x 8 cells, group),
+// and a transform takes the list of the run's positions bin after bin (the
+// order of k_spread_run and k_interp_run).  Kernel and grid as forced in the
+// options.
 struct GroupedPlan {
   Setup s;
   DevConst dcl;
@@ -1900,9 +1911,9 @@ struct GroupedPlan {
   DevBuf sorted_coord, perm, start, chunks, cws, grid, work;
   uint32_t ntiles = 0, ngroups = 0, nchunks = 0, g0 = 0, g1 = 0;
   int gbits = 0;
-  bool type1 = false;
+  bool type1 = false, runs = false;
   std::vector<uint32_t> gcount;   // points per group
-  DevBuf sel;                     // type 1: sorted positions of the current run's points
+  DevBuf sel;                     // runs: sorted positions of the current run's points
   uint64_t run_points(uint32_t a, uint32_t b) const {
     uint64_t n = 0;
     for (uint32_t k = a; k < b && k < ngroups; ++k) n += gcount[k];
@@ -1925,6 +1936,7 @@ GroupedPlan *grouped_plan_create(const double *coord, uint32_t M, const uint32_t
   auto gp = std::make_unique<GroupedPlan>();
   gp->s = make_setup(2, shape, M, eps, true, calc_f64, true, o);
   gp->type1 = type1;
+  gp->runs = type1 || calc_f64;
   Setup &s = gp->s;
   DN_REQUIRE(!s.qbits, ST_INTERNAL, "grouped index with a tensor-core key");
   int tilebits = s.keybits;
@@ -1937,7 +1949,7 @@ GroupedPlan *grouped_plan_create(const double *coord, uint32_t M, const uint32_t
     return nullptr;
   gp->ngroups = ngroups;
   gp->ntiles = uint32_t(ntiles);
-  if (type1) {
+  if (gp->runs) {
     // bins instead of tiles where key and table have room for them
     const int bb = 2 * (s.g.log2tile - 3);
     if (tilebits + bb + gp->gbits <= 32 &&
@@ -1963,7 +1975,7 @@ GroupedPlan *grouped_plan_create(const double *coord, uint32_t M, const uint32_t
   launch_key_starts(keys.as<uint32_t>(), M, nkeys, gp->start.as<uint32_t>(), st);
   gp->sorted_coord = DevBuf(size_t(M) * 16, st);
   launch_gather_coords(true, coord, 2, 1, 2, gp->perm.as<uint32_t>(), M, gp->sorted_coord.p, st);
-  if (type1) {
+  if (gp->runs) {
     gp->sel = DevBuf(size_t(M) * 4, st);
     gp->cws = DevBuf(group_select_workspace_bytes(gp->ntiles), st);
   } else {
@@ -2008,6 +2020,19 @@ static bool grouped_chunks(GroupedPlan *gp, uint32_t g0, uint32_t g1, cudaStream
   return gp->nchunks > 0;
 }
 
+// position list of groups [g0, g1), kept for the next call with the same run;
+// the number of points
+static uint32_t grouped_select(GroupedPlan *gp, uint32_t g0, uint32_t g1, cudaStream_t st) {
+  const uint32_t n = uint32_t(gp->run_points(g0, g1));
+  if (n > 0 && (gp->g1 == 0 || gp->g0 != g0 || gp->g1 != g1)) {
+    build_group_select(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1,
+                       gp->sel.as<uint32_t>(), gp->cws.p, st);
+    gp->g0 = g0;
+    gp->g1 = g1;
+  }
+  return n;
+}
+
 static View plain_view(void *data, int dtype, int ndim, int64_t s0, int64_t s1 = 0) {
   View v;
   std::memset(&v, 0, sizeof(v));
@@ -2029,14 +2054,8 @@ bool grouped_nu2u(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *values,
                   bool forward, cudaStream_t st) {
   const Setup &s = gp->s;
   DN_REQUIRE(gp->type1, ST_INTERNAL, "grouped index made for type 2");
-  const uint32_t n = uint32_t(gp->run_points(g0, g1));
+  const uint32_t n = grouped_select(gp, g0, g1, st);
   if (n == 0) return false;
-  if (gp->g1 == 0 || gp->g0 != g0 || gp->g1 != g1) {
-    build_group_select(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1,
-                       gp->sel.as<uint32_t>(), gp->cws.p, st);
-    gp->g0 = g0;
-    gp->g1 = g1;
-  }
   const ChunkList cl{nullptr, 0};
   const PointsDesc pts{gp->sorted_coord.p, 2, 1, true, true, gp->perm.as<uint32_t>(),
                        s.npoints};
@@ -2059,7 +2078,9 @@ bool grouped_u2nu(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *uni, vo
                   bool forward, cudaStream_t st) {
   const Setup &s = gp->s;
   DN_REQUIRE(!gp->type1, ST_INTERNAL, "grouped index made for type 1");
-  if (gp->run_points(g0, g1) == 0 || !grouped_chunks(gp, g0, g1, st)) return false;
+  if (gp->run_points(g0, g1) == 0) return false;
+  const uint32_t n = gp->runs ? grouped_select(gp, g0, g1, st) : 0u;
+  if (!gp->runs && !grouped_chunks(gp, g0, g1, st)) return false;
   const ChunkList cl{gp->chunks.as<Chunk>(), gp->nchunks};
   const PointsDesc pts{gp->sorted_coord.p, 2, 1, true, true, gp->perm.as<uint32_t>(),
                        s.npoints};
@@ -2069,7 +2090,7 @@ bool grouped_u2nu(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *uni, vo
   StageTimer tm(false, st);
   if (s.calc_f64)
     do_fft_interp<double>(s, *gp->dc, pts, cl, uv, ov, forward, false, tm, st, &gp->grid,
-                          &gp->work);
+                          &gp->work, nullptr, gp->sel.as<uint32_t>(), n);
   else
     do_fft_interp<float>(s, *gp->dc, pts, cl, uv, ov, forward, false, tm, st, &gp->grid,
                          &gp->work);

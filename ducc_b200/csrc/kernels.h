@@ -108,6 +108,13 @@ void launch_interp(const PointsDesc &pts, const ChunkList &cl, const Geometry &g
                    void *out, int64_t os, int64_t otrans, int ntrans, cudaStream_t st,
                    int *err = nullptr);
 
+// 2D double precision (launch_interp goes here; no chunk list): the points
+// sel[0 .. npts) of the sorted order, or all npts of it (sel null)
+void launch_interp_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts,
+                       const Geometry &g, const KernelPoly<double> &kp, const void *grid,
+                       int64_t gtrans, void *out, int64_t os, int64_t otrans, int ntrans,
+                       cudaStream_t st);
+
 // grad[j*gs0 + d*gs1] = Re(conj(wts[j*ws]) * d/dx_{j,d} interp(grid)(x_j)), in
 // the coordinates' dtype (interp_grad.cu)
 template <typename T>

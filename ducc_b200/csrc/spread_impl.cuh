@@ -737,12 +737,20 @@ template <typename T>
 void launch_interp_impl(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
                         const KernelPoly<T> &kp, const void *grid, int64_t gtrans, void *out,
                         int64_t os, int64_t otrans, int ntrans, cudaStream_t st, int *err) {
+  if constexpr (sizeof(T) == 8) {
+    if (g.ndim == 2) {
+      launch_interp_run(pts, nullptr, pts.npts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
+      return;
+    }
+  }
   if (cl.nchunks == 0 || ntrans == 0) return;
 #define DN_ID(TC, ND) interp_dispatch<T, TC, ND>(pts, cl, g, kp, grid, gtrans, out, os, otrans, ntrans, st, err)
-  if (pts.coord_f64) {
-    if (g.ndim == 1) DN_ID(double, 1); else if (g.ndim == 2) DN_ID(double, 2); else DN_ID(double, 3);
-  } else {
-    if (g.ndim == 1) DN_ID(float, 1); else if (g.ndim == 2) DN_ID(float, 2); else DN_ID(float, 3);
+  if (g.ndim == 1) {
+    if (pts.coord_f64) DN_ID(double, 1); else DN_ID(float, 1);
+  } else if (g.ndim == 3) {
+    if (pts.coord_f64) DN_ID(double, 3); else DN_ID(float, 3);
+  } else if constexpr (sizeof(T) == 4) {
+    if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
   }
 #undef DN_ID
 }
