@@ -419,13 +419,10 @@ void read_words(const uint32_t *const *src, int n, uint32_t *out, cudaStream_t s
   for (int i = 0; i < n; ++i) out[i] = h[i];
 }
 
-// Builds the chunk list from sorted keys; returns the number of chunks (the
-// count is read back to the host, which synchronises the stream once: through
-// mapped host memory, or with zero_copy false, which allocates nothing, by a
-// device->host copy).
+// Builds the chunk list from sorted keys.
 uint32_t build_chunks(const uint32_t *skeys, uint32_t n, int tile_shift, uint32_t chunk,
                       Chunk *chunks, uint32_t *d_count, void *ws, cudaStream_t st,
-                      bool zero_copy) {
+                      bool zero_copy, bool read_back) {
   if (n == 0) return 0;
   uint32_t *flags = static_cast<uint32_t *>(ws);
   uint32_t *pos = flags + n;
@@ -442,6 +439,7 @@ uint32_t build_chunks(const uint32_t *skeys, uint32_t n, int tile_shift, uint32_
   k_chunk_counts<<<g, 256, 0, st>>>(chunks, d_count, n);
   DN_LAUNCHED();
   uint32_t h = 0;
+  if (!read_back) return 0;
   if (zero_copy) {
     const uint32_t *src[1] = {d_count};
     read_words(src, 1, &h, st);
@@ -580,9 +578,9 @@ size_t group_chunk_workspace_bytes(uint32_t ntiles) {
   return size_t(2) * (ntiles + 1) * 4 + 256 + scan_workspace_bytes(uint64_t(ntiles) + 1);
 }
 
-uint32_t build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, uint32_t g0,
-                            uint32_t g1, uint32_t chunk, Chunk *chunks, void *ws,
-                            cudaStream_t st) {
+const uint32_t *build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, uint32_t g0,
+                                   uint32_t g1, uint32_t chunk, Chunk *chunks, void *ws,
+                                   cudaStream_t st) {
   uint32_t *cnt = static_cast<uint32_t *>(ws);
   uint32_t *pos = cnt + (ntiles + 1);
   uint32_t *sws = reinterpret_cast<uint32_t *>(
@@ -594,10 +592,7 @@ uint32_t build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, u
   k_gchunk_fill<<<grid_of(ntiles), 256, 0, st>>>(start, cnt, pos, ntiles, gbits, g0, g1, chunk,
                                                  chunks);
   DN_LAUNCHED();
-  const uint32_t *src[1] = {pos + ntiles};
-  uint32_t h = 0;
-  read_words(src, 1, &h, st);
-  return h;
+  return pos + ntiles;
 }
 
 // sorted positions of the points of groups [g0, g1), bin after bin: counts

@@ -83,6 +83,11 @@ struct DevBuf {
 };
 
 // ---------------------------------------------------------------- device error word
+bool &bounded_wait_launched() {
+  static thread_local bool launched = false;
+  return launched;
+}
+
 // Kernels with bounded waits set this word instead of hanging; it is read back
 // after such a kernel (outside stream capture) and turned into ST_TIMEOUT.
 static int *device_error_word() {
@@ -100,10 +105,19 @@ static int *device_error_word() {
   return words[dev];
 }
 
+// Every call ends here, waiting for its stream (plans share their grid between
+// calls on any streams; arrays may be reused once a call returns).  Only kernels
+// with bounded waits (marked by their launchers in bounded_wait_launched) can set
+// the word: without one there is nothing to read.
 static void check_device_error(int *word, cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   DN_CUDA(cudaStreamIsCapturing(st, &cs));
   if (cs != cudaStreamCaptureStatusNone) return;
+  if (!bounded_wait_launched()) {
+    DN_CUDA(cudaStreamSynchronize(st));
+    return;
+  }
+  bounded_wait_launched() = false;
   uint32_t h = 0;
   const uint32_t *src[1] = {reinterpret_cast<const uint32_t *>(word)};
   read_words(src, 1, &h, st);
@@ -247,11 +261,17 @@ static int64_t nelem(const View &v) {
   return s;
 }
 
+static size_t host_bytes(const View &v) { return size_t(nelem(v)) * dtype_size(v.dtype); }
+
 // A second stream of an unplanned call on host arrays: host->device copies
 // (and work that needs only them) run there while the caller's stream builds
 // the index, forked from and joined back into the caller's stream by events.
 // Created only for calls with host arrays (device-array calls, e.g. recorded
 // into a stream capture, keep to the caller's stream); inactive otherwise.
+// Small arrays are copied on the caller's stream: making and destroying a
+// stream and two events costs about 50 us, the copy of 1 MB 20 us.
+constexpr size_t SIDE_MIN_BYTES = size_t(1) << 20;
+
 struct SideStream {
   cudaStream_t main, s = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -335,7 +355,6 @@ struct Setup {
   double ofactor = 0, beta = 0, e0 = 0, epsilon = 0;
   KernelPoly<float> kpf;
   KernelPoly<double> kpd;
-  std::vector<double> corfac[3];
   std::vector<int> factors[3];
   int spreader = DNUFFT_SPREAD_AUTO;
   bool qbits = false;   // sort key carries the 2D tile quadrant and cell (tensor-core order)
@@ -495,12 +514,16 @@ static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double 
   if (s.spreader == DNUFFT_SPREAD_TC)
     DN_REQUIRE(spread_tc_supported(g, calc_f64), ST_UNSUPPORTED,
                "tensor-core spreader: 2D single precision (complex64) with support <= 8 only");
-  auto coeff = kernel_coeffs(g.W, s.beta, s.e0);
-  fill_poly(s, coeff);
-  for (int d = 0; d < ndim; ++d)
-    s.corfac[d] = correction_factors(size_t(g.nuni[d] / 2 + 1), 1. / double(g.nover[d]), g.W,
-                                     s.beta, s.e0);
+  fill_poly(s, kernel_coeffs_of(s.kidx));
   return s;
+}
+
+// correction factors of an axis: computed where they are uploaded, not in
+// make_setup (0.2 ms of cosines for 1430 modes, which a call whose constants
+// are already on the device does not need)
+static std::vector<double> corfac_of(const Setup &s, int d) {
+  return correction_factors(size_t(s.g.nuni[d] / 2 + 1), 1. / double(s.g.nover[d]), s.g.W, s.beta,
+                            s.e0);
 }
 
 // device-resident per-transform constants: correction factors and twiddles
@@ -513,9 +536,10 @@ struct DevConst {
 
 static void upload_consts(const Setup &s, DevConst &dc, cudaStream_t st) {
   for (int d = 0; d < s.g.ndim; ++d) {
-    size_t nb = s.corfac[d].size() * sizeof(double);
+    const std::vector<double> cf = corfac_of(s, d);
+    size_t nb = cf.size() * sizeof(double);
     dc.corfac[d] = DevBuf(nb, st);
-    DN_CUDA(cudaMemcpyAsync(dc.corfac[d].p, s.corfac[d].data(), nb, cudaMemcpyHostToDevice, st));
+    DN_CUDA(cudaMemcpyAsync(dc.corfac[d].p, cf.data(), nb, cudaMemcpyHostToDevice, st));
     dc.cf[d] = dc.corfac[d].as<double>();
     int n = int(s.g.nover[d]);
     size_t esz = s.calc_f64 ? 16 : 8;
@@ -547,12 +571,12 @@ static void upload_consts(const Setup &s, DevConst &dc, cudaStream_t st) {
   DN_CUDA(cudaStreamSynchronize(st));
 }
 
-// Constants of an unplanned call, shared by later unplanned calls with the same
-// geometry on the same device: the upload (host twiddles, pageable copies and
-// a stream synchronisation) then happens once instead of on every call.  Up to
-// MAX_SHARED geometries per process are kept (about the size of their
-// twiddle tables each) for the life of the process; beyond that a call uploads
-// into the caller's `local` as before.  An entry is complete (its stream was
+// Constants of an unplanned call or a plan, shared by later calls and plans with
+// the same geometry on the same device: the upload (host cosines, pageable
+// copies and a stream synchronisation) then happens once.  Up to MAX_SHARED
+// geometries per process are kept (about the size of their twiddle tables
+// each) for the life of the process; beyond that a call uploads into the
+// caller's `local`.  An entry is complete (its stream was
 // synchronised) before it is published, so any stream may read it.
 static const DevConst &consts_for(const Setup &s, DevConst &local, cudaStream_t st) {
   constexpr size_t MAX_SHARED = 32;
@@ -594,7 +618,18 @@ static const DevConst &consts_for(const Setup &s, DevConst &local, cudaStream_t 
 // index: tile permutation, sorted keys and chunk list
 struct Index {
   DevBuf perm, keys, chunks, count;
-  uint32_t nchunks = 0;
+  uint32_t nchunks = 0;      // number of chunks, or an upper bound of it
+  bool counted = false;      // nchunks is the number
+  ChunkList chunk_list() const {
+    return ChunkList{chunks.as<Chunk>(), nchunks, counted ? nullptr : count.as<uint32_t>()};
+  }
+  // replaces the bound by the number (synchronises st)
+  void read_count(cudaStream_t st) {
+    if (counted || nchunks == 0) return;
+    const uint32_t *src[1] = {count.as<uint32_t>()};
+    read_words(src, 1, &nchunks, st);
+    counted = true;
+  }
   // tensor-core order only: K-block list and per-CTA ranges
   DevBuf kblk, kbrange;
   uint32_t nkblk = 0, groups = 0;
@@ -608,8 +643,9 @@ static uint32_t sm_count() {
   return uint32_t(n > 0 ? n : 1);
 }
 
-// need_chunks: the chunk list too (the 2D and 3D plain spreaders need none; the
-// number of chunks is read back to the host, which waits for the sort)
+// need_chunks: the chunk list too (the 2D and 3D plain spreaders need none).
+// Only the tensor-core order reads counts back to the host, which waits for the
+// sort; launches over chunks cover an upper bound of their number.
 static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream_t st,
                         bool need_chunks = true) {
   uint32_t M = s.npoints;
@@ -626,14 +662,17 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
   ix.chunks = DevBuf(size_t(maxchunks) * sizeof(Chunk), st);
   ix.count = DevBuf(16, st);
   DevBuf ws(chunk_workspace_bytes(M), st);
-  ix.nchunks = build_chunks(ix.keys.as<uint32_t>(), M, s.tile_shift, s.chunk, ix.chunks.as<Chunk>(),
-                            ix.count.as<uint32_t>(), ws.p, st);
+  const uint32_t n = build_chunks(ix.keys.as<uint32_t>(), M, s.tile_shift, s.chunk,
+                                  ix.chunks.as<Chunk>(), ix.count.as<uint32_t>(), ws.p, st, true,
+                                  s.qbits);
+  ix.counted = s.qbits || M == 0;
+  ix.nchunks = ix.counted ? n : uint32_t(std::min<uint64_t>(maxchunks, M));
   if (s.qbits && ix.nchunks > 0) {
     ix.groups = sm_count();
     ix.kblk = DevBuf(size_t(tc_kblock_upper_bound(M, ix.nchunks)) * sizeof(uint2), st);
     ix.kbrange = DevBuf(size_t(ix.groups + 1) * sizeof(uint32_t), st);
     DevBuf kws(tc_kblock_workspace_bytes(ix.nchunks), st);
-    ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
+    const ChunkList cl = ix.chunk_list();
     ix.nkblk = build_tc_kblocks(ix.keys.as<uint32_t>(), cl, ix.groups, kws.p, ix.kblk.as<uint2>(),
                                 ix.kbrange.as<uint32_t>(), ix.count.as<uint32_t>(),
                                 tc_cell_bits(s.g), st);
@@ -698,7 +737,7 @@ static void do_spread_fft(const Setup &s, const DevConst &dc, const PointsDesc &
                           const ChunkList &cl, const TcBlocks *tb, const View &points,
                           const View &out, bool forward, bool fft_order, StageTimer &tm,
                           cudaStream_t st, DevBuf *ws = nullptr, DevBuf *wk = nullptr,
-                          const uint32_t *sel = nullptr, uint32_t nsel = 0) {
+                          const uint32_t *sel = nullptr, uint32_t nsel = 0, bool check = true) {
   size_t cells = grid_cells(s.g);
   tm.mark("zeroing grid");
   DevBuf local;
@@ -716,7 +755,7 @@ static void do_spread_fft(const Setup &s, const DevConst &dc, const PointsDesc &
   fft_nu2u_tail<T>(grid.p, s.g, dc.ax, forward, dc.cf, fft_order, out.data, out.stride, st,
                    work.p, err);
   tm.mark("output copy");   // last mark of a planned call; an unplanned call copies out next
-  check_device_error(err, st);
+  if (check) check_device_error(err, st);
 }
 
 // With a side stream, the FFT pass runs there and st waits for it before the
@@ -728,7 +767,7 @@ static void do_fft_interp(const Setup &s, const DevConst &dc, const PointsDesc &
                           const ChunkList &cl, const View &uni, const View &out, bool forward,
                           bool fft_order, StageTimer &tm, cudaStream_t st, DevBuf *ws = nullptr,
                           DevBuf *wk = nullptr, SideStream *side = nullptr,
-                          const uint32_t *sel = nullptr, uint32_t nsel = 0) {
+                          const uint32_t *sel = nullptr, uint32_t nsel = 0, bool check = true) {
   size_t cells = grid_cells(s.g);
   DevBuf local;
   DevBuf &grid = ws ? *ws : local;
@@ -758,10 +797,13 @@ static void do_fft_interp(const Setup &s, const DevConst &dc, const PointsDesc &
       done = true;
     }
   }
+  // tiles staged by TMA only after a row FFT whose bounded waits are read back
+  // anyway (the same time per launch, and no tensor map for small grids)
   if (!done)
-    launch_interp<T>(pts, cl, s.g, kp, grid.p, 0, out.data, out.stride[0], 0, 1, st, err);
+    launch_interp<T>(pts, cl, s.g, kp, grid.p, 0, out.data, out.stride[0], 0, 1, st,
+                     bounded_wait_launched() ? err : nullptr);
   tm.mark("output copy");
-  check_device_error(err, st);
+  if (check) check_device_error(err, st);
 }
 
 template <typename T>
@@ -907,7 +949,7 @@ static void nu2u_pipelined(const Setup &s, const View &points, const View &coord
     build_index(sg, cv, ix, st, spread_needs_chunks(sg));
     PointsDesc pts{cv.data, cv.stride[0], cv.stride[1], false, s.coord_f64,
                    ix.perm.as<uint32_t>(), sg.npoints};
-    ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
+    ChunkList cl = ix.chunk_list();
     const TcBlocks tb = ix.tc();
     spread_points<T>(sg, pts, cl, &tb, static_cast<char *>(dvals.p) + a * vb, 1, grid.p, err, st);
   }
@@ -978,7 +1020,7 @@ static void u2nu_pipelined(const Setup &s, const View &uni, const View &coord, c
     build_index(sg, cv, ix, st, interp_needs_chunks(sg));
     PointsDesc pts{cv.data, cv.stride[0], cv.stride[1], false, s.coord_f64,
                    ix.perm.as<uint32_t>(), sg.npoints};
-    ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
+    const ChunkList cl = ix.chunk_list();
     launch_interp<T>(pts, cl, s.g, kp, grid.p, 0,
                      static_cast<char *>(ov.data) + a * size_t(ov.stride[0]) * vb, ov.stride[0], 0,
                      1, st, err);
@@ -1032,7 +1074,7 @@ static void nu2u_impl(const dnufft_array *points_, const dnufft_array *coord_, i
   tm.mark("coordinates host->device");
   // host arrays: the coordinates next; the point values follow on a side
   // stream while this stream builds the index
-  SideStream side(st, points.host);
+  SideStream side(st, points.host && host_bytes(points) >= SIDE_MIN_BYTES);
   Staged sc(coord, true, false, st);
   Staged sp(points, true, false, st, &side), so(out, false, true, st);
   if (s.npoints == 0) {
@@ -1048,7 +1090,7 @@ static void nu2u_impl(const dnufft_array *points_, const dnufft_array *coord_, i
   side.merge();
   PointsDesc pts{sc.dev.data, sc.dev.stride[0], sc.dev.stride[1], false, s.coord_f64,
                  ix.perm.as<uint32_t>(), s.npoints};
-  ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
+  const ChunkList cl = ix.chunk_list();
   const TcBlocks tb = ix.tc();
   if (f64)
     do_spread_fft<double>(s, dc, pts, cl, &tb, sp.dev, so.dev, forward != 0,
@@ -1094,7 +1136,7 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   tm.mark("coordinates host->device");
   // host arrays: the coordinates first; the uniform grid follows on a side
   // stream, which also runs the FFT pass, while this stream builds the index
-  SideStream side(st, uni.host);
+  SideStream side(st, uni.host && host_bytes(uni) >= SIDE_MIN_BYTES);
   Staged sc(coord, true, false, st), so(out, false, true, st);
   Staged su(uni, true, false, st, &side);
   const size_t esz = f64 ? 16 : 8;
@@ -1107,7 +1149,7 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   build_index(s, sc.dev, ix, st, interp_needs_chunks(s));
   PointsDesc pts{sc.dev.data, sc.dev.stride[0], sc.dev.stride[1], false, s.coord_f64,
                  ix.perm.as<uint32_t>(), s.npoints};
-  ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
+  const ChunkList cl = ix.chunk_list();
   if (f64)
     do_fft_interp<double>(s, dc, pts, cl, su.dev, so.dev, forward != 0, o.fft_order != 0, tm, st,
                           &grid, &work, side.active() ? &side : nullptr);
@@ -1146,7 +1188,7 @@ static void u2nu_dcoord_impl(const dnufft_array *grid_, const dnufft_array *coor
   build_index(s, sc.dev, ix, st);
   PointsDesc pts{sc.dev.data, sc.dev.stride[0], sc.dev.stride[1], false, s.coord_f64,
                  ix.perm.as<uint32_t>(), s.npoints};
-  ChunkList cl{ix.chunks.as<Chunk>(), ix.nchunks};
+  const ChunkList cl = ix.chunk_list();
   if (f64)
     do_fft_dcoord<double>(s, dc, pts, cl, su.dev, sw.dev, sg.dev, forward != 0, o.fft_order != 0,
                           tm, st);
@@ -1175,7 +1217,8 @@ struct PlanGroup {
 
 struct dnufft_plan {
   dnufft::Setup s;
-  dnufft::DevConst dc;
+  dnufft::DevConst own;                      // constants where the shared ones are full
+  const dnufft::DevConst *dc = nullptr;
   dnufft::Index ix;
   dnufft::DevBuf sorted_coord;
   dnufft::DevBuf grid;   // oversampled grid, allocated on first execution
@@ -1201,7 +1244,7 @@ static void plan_create_impl(int nu2u, const dnufft_array *coord_, const int64_t
   p->o = o;
   p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o, true);
   DN_CUDA(cudaGetDevice(&p->device));
-  upload_consts(p->s, p->dc, st);
+  p->dc = &consts_for(p->s, p->own, st);
   if (p->s.npoints > 0) {
     Staged sc(coord, true, false, st);
     build_index(p->s, sc.dev, p->ix, st);
@@ -1231,6 +1274,8 @@ static void plan_create_impl(int nu2u, const dnufft_array *coord_, const int64_t
         pg.ix.keys.release();
       }
     }
+    p->ix.read_count(st);
+    for (auto &pg : p->groups) pg.ix.read_count(st);
   }
   DN_CUDA(cudaStreamSynchronize(st));
   *out = p.release();
@@ -1281,13 +1326,13 @@ static void plan_nu2u_groups(dnufft_plan *p, const View &points, const View &out
     DN_CUDA(cudaStreamWaitEvent(st, copied.ev[size_t(gi)], 0));
     Setup sg = s;
     sg.npoints = uint32_t(pg.b - pg.a);
-    const ChunkList cl{pg.ix.chunks.as<Chunk>(), pg.ix.nchunks};
+    const ChunkList cl = pg.ix.chunk_list();
     const TcBlocks tb = pg.ix.tc();
     spread_points<T>(sg, group_points(p, pg), cl, s.qbits ? &tb : nullptr,
                      static_cast<char *>(dvals.p) + pg.a * vb, 1, p->grid.p, err, st);
   }
   tm.mark("FFT + correction");
-  fft_nu2u_tail<T>(p->grid.p, s.g, p->dc.ax, forward, p->dc.cf, p->o.fft_order != 0,
+  fft_nu2u_tail<T>(p->grid.p, s.g, p->dc->ax, forward, p->dc->cf, p->o.fft_order != 0,
                    so.dev.data, so.dev.stride, st, p->work.p, err);
   tm.mark("output copy");
   check_device_error(err, st);
@@ -1311,14 +1356,14 @@ static void plan_u2nu_groups(dnufft_plan *p, const View &uni, const View &out, b
   down.start();
   int *err = device_error_word();
   tm.mark("correction + FFT");
-  fft_u2nu_head<T>(su.dev.data, su.dev.stride, s.g, p->dc.ax, forward, p->dc.cf,
+  fft_u2nu_head<T>(su.dev.data, su.dev.stride, s.g, p->dc->ax, forward, p->dc->cf,
                    p->o.fft_order != 0, p->grid.p, st, p->work.p, err);
   tm.mark("groups: interpolation");
   const KernelPoly<T> &kp = *reinterpret_cast<const KernelPoly<T> *>(
       sizeof(T) == 4 ? static_cast<const void *>(&s.kpf) : static_cast<const void *>(&s.kpd));
   for (int gi = 0; gi < G; ++gi) {
     const PlanGroup &pg = p->groups[size_t(gi)];
-    const ChunkList cl{pg.ix.chunks.as<Chunk>(), pg.ix.nchunks};
+    const ChunkList cl = pg.ix.chunk_list();
     launch_interp<T>(group_points(p, pg), cl, s.g, kp, p->grid.p, 0,
                      static_cast<char *>(dout.p) + pg.a * vb, 1, 0, 1, st, err);
     DN_CUDA(cudaEventRecord(done.ev[size_t(gi)], st));
@@ -1407,17 +1452,17 @@ static void plan_exec_one(dnufft_plan *p, bool type1, int forward, int verbosity
   plan_buffers(p, st);
   PointsDesc pts{p->sorted_coord.p, int64_t(s.g.ndim), 1, true, s.coord_f64,
                  p->ix.perm.as<uint32_t>(), s.npoints};
-  ChunkList cl{p->ix.chunks.as<Chunk>(), p->ix.nchunks};
+  ChunkList cl = p->ix.chunk_list();
   bool fo = p->o.fft_order != 0;
   if (type1) {
     const TcBlocks tb = p->ix.tc();
     const TcBlocks *sk = s.qbits ? &tb : nullptr;
-    if (f64) do_spread_fft<double>(s, p->dc, pts, cl, sk, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
-    else do_spread_fft<float>(s, p->dc, pts, cl, sk, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
+    if (f64) do_spread_fft<double>(s, *p->dc, pts, cl, sk, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
+    else do_spread_fft<float>(s, *p->dc, pts, cl, sk, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
     tm.report("nu2u (planned)");
   } else {
-    if (f64) do_fft_interp<double>(s, p->dc, pts, cl, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
-    else do_fft_interp<float>(s, p->dc, pts, cl, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
+    if (f64) do_fft_interp<double>(s, *p->dc, pts, cl, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
+    else do_fft_interp<float>(s, *p->dc, pts, cl, si.dev, so.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
     tm.report("u2nu (planned)");
   }
   so.finish();
@@ -1448,10 +1493,10 @@ static void plan_dcoord_impl(dnufft_plan *p, int forward, const dnufft_array *gr
   }
   PointsDesc pts{p->sorted_coord.p, int64_t(s.g.ndim), 1, true, s.coord_f64,
                  p->ix.perm.as<uint32_t>(), s.npoints};
-  ChunkList cl{p->ix.chunks.as<Chunk>(), p->ix.nchunks};
+  ChunkList cl = p->ix.chunk_list();
   bool fo = p->o.fft_order != 0;
-  if (f64) do_fft_dcoord<double>(s, p->dc, pts, cl, su.dev, sw.dev, sg.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
-  else do_fft_dcoord<float>(s, p->dc, pts, cl, su.dev, sw.dev, sg.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
+  if (f64) do_fft_dcoord<double>(s, *p->dc, pts, cl, su.dev, sw.dev, sg.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
+  else do_fft_dcoord<float>(s, *p->dc, pts, cl, su.dev, sw.dev, sg.dev, forward != 0, fo, tm, st, &p->grid, &p->work);
   tm.report("u2nu_dcoord (planned)");
   sg.finish();
 }
@@ -1498,7 +1543,7 @@ static void plan_spread_impl(dnufft_plan *p, const dnufft_array *points_, dnufft
     Staged sp(points, true, false, st);
     PointsDesc pts{p->sorted_coord.p, int64_t(s.g.ndim), 1, true, s.coord_f64,
                    p->ix.perm.as<uint32_t>(), s.npoints};
-    ChunkList cl{p->ix.chunks.as<Chunk>(), p->ix.nchunks};
+    ChunkList cl = p->ix.chunk_list();
     const TcBlocks tb = p->ix.tc();
     const TcBlocks *sk = s.qbits ? &tb : nullptr;
     int *err = device_error_word();
@@ -1528,10 +1573,10 @@ static void plan_grid_to_uniform_impl(dnufft_plan *p, int forward, dnufft_array 
   int *err = device_error_word();
   const bool fo = p->o.fft_order != 0;
   if (f64)
-    fft_nu2u_tail<double>(grid.data, s.g, p->dc.ax, forward != 0, p->dc.cf, fo, so.dev.data,
+    fft_nu2u_tail<double>(grid.data, s.g, p->dc->ax, forward != 0, p->dc->cf, fo, so.dev.data,
                           so.dev.stride, st, p->work.p, err);
   else
-    fft_nu2u_tail<float>(grid.data, s.g, p->dc.ax, forward != 0, p->dc.cf, fo, so.dev.data,
+    fft_nu2u_tail<float>(grid.data, s.g, p->dc->ax, forward != 0, p->dc->cf, fo, so.dev.data,
                          so.dev.stride, st, p->work.p, err);
   check_device_error(err, st);
   so.finish();
@@ -1562,9 +1607,9 @@ static void plan_rows_fft_impl(dnufft_plan *p, int forward, dnufft_array *rows_,
   if (r.shape[0] == 0) return;
   int *err = device_error_word();
   if (p->s.calc_f64)
-    fft_nu2u_rows<double>(r.data, int(r.shape[0]), p->s.g, p->dc.ax, forward != 0, st, err);
+    fft_nu2u_rows<double>(r.data, int(r.shape[0]), p->s.g, p->dc->ax, forward != 0, st, err);
   else
-    fft_nu2u_rows<float>(r.data, int(r.shape[0]), p->s.g, p->dc.ax, forward != 0, st, err);
+    fft_nu2u_rows<float>(r.data, int(r.shape[0]), p->s.g, p->dc->ax, forward != 0, st, err);
   check_device_error(err, st);
 }
 
@@ -1575,9 +1620,9 @@ static void plan_rows_fft_kept_in_impl(dnufft_plan *p, int forward, dnufft_array
   if (r.shape[0] == 0) return;
   int *err = device_error_word();
   if (p->s.calc_f64)
-    fft_u2nu_rows<double>(r.data, int(r.shape[0]), p->s.g, p->dc.ax, forward != 0, st, err);
+    fft_u2nu_rows<double>(r.data, int(r.shape[0]), p->s.g, p->dc->ax, forward != 0, st, err);
   else
-    fft_u2nu_rows<float>(r.data, int(r.shape[0]), p->s.g, p->dc.ax, forward != 0, st, err);
+    fft_u2nu_rows<float>(r.data, int(r.shape[0]), p->s.g, p->dc->ax, forward != 0, st, err);
   check_device_error(err, st);
 }
 
@@ -1608,11 +1653,11 @@ static void plan_uniform_to_cols_impl(dnufft_plan *p, int forward, const dnufft_
   }
   const bool fo = p->o.fft_order != 0;
   const bool ok =
-      f64 ? fft_u2nu_cols_range<double>(uni.data, uni.stride, s.g, p->dc.ax, forward != 0,
-                                        p->dc.cf, fo, cols.data, int(nc), int(col0), st,
+      f64 ? fft_u2nu_cols_range<double>(uni.data, uni.stride, s.g, p->dc->ax, forward != 0,
+                                        p->dc->cf, fo, cols.data, int(nc), int(col0), st,
                                         p->work.p)
-          : fft_u2nu_cols_range<float>(uni.data, uni.stride, s.g, p->dc.ax, forward != 0,
-                                       p->dc.cf, fo, cols.data, int(nc), int(col0), st,
+          : fft_u2nu_cols_range<float>(uni.data, uni.stride, s.g, p->dc->ax, forward != 0,
+                                       p->dc->cf, fo, cols.data, int(nc), int(col0), st,
                                        p->work.p);
   DN_REQUIRE(ok, ST_UNSUPPORTED,
              "column blocks need the four-step column passes (oversampled rows >= 1024)");
@@ -1631,7 +1676,7 @@ static void plan_interp_impl(dnufft_plan *p, const dnufft_array *grid_, dnufft_a
   if (s.npoints == 0) return;
   PointsDesc pts{p->sorted_coord.p, int64_t(s.g.ndim), 1, true, s.coord_f64,
                  p->ix.perm.as<uint32_t>(), s.npoints};
-  ChunkList cl{p->ix.chunks.as<Chunk>(), p->ix.nchunks};
+  ChunkList cl = p->ix.chunk_list();
   if (s.calc_f64)
     launch_interp<double>(pts, cl, s.g, s.kpd, grid.data, 0, out.data, out.stride[0], 0, 1, st);
   else
@@ -1672,10 +1717,10 @@ static void plan_cols_to_uniform_impl(dnufft_plan *p, int forward, dnufft_array 
   }
   const bool fo = p->o.fft_order != 0;
   if (f64)
-    fft_nu2u_cols<double>(grid.data, gc, p->dc.ax, forward != 0, p->dc.cf, fo, so.dev.data,
+    fft_nu2u_cols<double>(grid.data, gc, p->dc->ax, forward != 0, p->dc->cf, fo, so.dev.data,
                           so.dev.stride, st, p->work.p);
   else
-    fft_nu2u_cols<float>(grid.data, gc, p->dc.ax, forward != 0, p->dc.cf, fo, so.dev.data,
+    fft_nu2u_cols<float>(grid.data, gc, p->dc->ax, forward != 0, p->dc->cf, fo, so.dev.data,
                          so.dev.stride, st, p->work.p);
   so.finish();
 }
@@ -1707,11 +1752,11 @@ static void plan_cols_range_impl(dnufft_plan *p, int forward, dnufft_array *cols
   }
   const bool fo = p->o.fft_order != 0;
   const bool ok =
-      f64 ? fft_nu2u_cols_range<double>(cols.data, int(nc), int(col0), s.g, p->dc.ax,
-                                        forward != 0, p->dc.cf, fo, out.data, out.stride, st,
+      f64 ? fft_nu2u_cols_range<double>(cols.data, int(nc), int(col0), s.g, p->dc->ax,
+                                        forward != 0, p->dc->cf, fo, out.data, out.stride, st,
                                         p->work.p)
-          : fft_nu2u_cols_range<float>(cols.data, int(nc), int(col0), s.g, p->dc.ax,
-                                       forward != 0, p->dc.cf, fo, out.data, out.stride, st,
+          : fft_nu2u_cols_range<float>(cols.data, int(nc), int(col0), s.g, p->dc->ax,
+                                       forward != 0, p->dc->cf, fo, out.data, out.stride, st,
                                        p->work.p);
   DN_REQUIRE(ok, ST_UNSUPPORTED,
              "column blocks need the four-step column passes (oversampled rows >= 1024)");
@@ -1757,8 +1802,10 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
   Carver cv(scratch, cap);
   double *cf[3] = {nullptr, nullptr, nullptr};
   void *tw[3] = {nullptr, nullptr, nullptr};
+  std::vector<double> corfac[3];
   for (int d = 0; d < g.ndim; ++d) {
-    cf[d] = static_cast<double *>(cv.take(s.corfac[d].size() * sizeof(double)));
+    corfac[d] = corfac_of(s, d);
+    cf[d] = static_cast<double *>(cv.take(corfac[d].size() * sizeof(double)));
     tw[d] = cv.take(size_t(g.nover[d]) * csz);
   }
   uint32_t *keys = static_cast<uint32_t *>(cv.take(size_t(M) * 4));
@@ -1775,7 +1822,7 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
     // measure what would have been needed for the message
     Carver probe(nullptr, ~size_t(0));
     for (int d = 0; d < g.ndim; ++d) {
-      probe.take(s.corfac[d].size() * sizeof(double));
+      probe.take(corfac[d].size() * sizeof(double));
       probe.take(size_t(g.nover[d]) * csz);
     }
     probe.take(size_t(M) * 4);
@@ -1794,7 +1841,7 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
   std::vector<std::vector<double>> hd(g.ndim);
   std::vector<std::vector<float>> hf(g.ndim);
   for (int d = 0; d < g.ndim; ++d) {
-    DN_CUDA(cudaMemcpyAsync(cf[d], s.corfac[d].data(), s.corfac[d].size() * sizeof(double),
+    DN_CUDA(cudaMemcpyAsync(cf[d], corfac[d].data(), corfac[d].size() * sizeof(double),
                             cudaMemcpyHostToDevice, st));
     const int n = int(g.nover[d]);
     if (sizeof(T) == 8) {
@@ -1909,7 +1956,8 @@ struct GroupedPlan {
   DevConst dcl;
   const DevConst *dc = nullptr;
   DevBuf sorted_coord, perm, start, chunks, cws, grid, work;
-  uint32_t ntiles = 0, ngroups = 0, nchunks = 0, g0 = 0, g1 = 0;
+  uint32_t ntiles = 0, ngroups = 0, g0 = 0, g1 = 0;
+  const uint32_t *chunk_count = nullptr;   // (in cws)
   int gbits = 0;
   bool type1 = false, runs = false;
   std::vector<uint32_t> gcount;   // points per group
@@ -2008,16 +2056,19 @@ void grouped_plan_destroy(GroupedPlan *gp, cudaStream_t st) {
 
 const uint32_t *grouped_plan_perm(const GroupedPlan *gp) { return gp->perm.as<uint32_t>(); }
 
-// chunk list of groups [g0, g1), kept for the next call with the same run;
-// false: no point in the run
-static bool grouped_chunks(GroupedPlan *gp, uint32_t g0, uint32_t g1, cudaStream_t st) {
+// chunk list of the n points of groups [g0, g1), kept for the next call with the
+// same run
+static ChunkList grouped_chunks(GroupedPlan *gp, uint32_t g0, uint32_t g1, uint64_t n,
+                                cudaStream_t st) {
   if (gp->g1 == 0 || gp->g0 != g0 || gp->g1 != g1) {
-    gp->nchunks = build_group_chunks(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1,
-                                     gp->s.chunk, gp->chunks.as<Chunk>(), gp->cws.p, st);
+    gp->chunk_count = build_group_chunks(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1,
+                                         gp->s.chunk, gp->chunks.as<Chunk>(), gp->cws.p, st);
     gp->g0 = g0;
     gp->g1 = g1;
   }
-  return gp->nchunks > 0;
+  const uint64_t bound = std::min<uint64_t>(n, gp->ntiles) + n / gp->s.chunk;
+  return ChunkList{gp->chunks.as<Chunk>(), uint32_t(std::min<uint64_t>(bound, n)),
+                   gp->chunk_count};
 }
 
 // position list of groups [g0, g1), kept for the next call with the same run;
@@ -2065,10 +2116,10 @@ bool grouped_nu2u(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *values,
   StageTimer tm(false, st);
   if (s.calc_f64)
     do_spread_fft<double>(s, *gp->dc, pts, cl, nullptr, vv, ov, forward, false, tm, st,
-                          &gp->grid, &gp->work, gp->sel.as<uint32_t>(), n);
+                          &gp->grid, &gp->work, gp->sel.as<uint32_t>(), n, false);
   else
     do_spread_fft<float>(s, *gp->dc, pts, cl, nullptr, vv, ov, forward, false, tm, st,
-                         &gp->grid, &gp->work, gp->sel.as<uint32_t>(), n);
+                         &gp->grid, &gp->work, gp->sel.as<uint32_t>(), n, false);
   return true;
 }
 
@@ -2078,10 +2129,10 @@ bool grouped_u2nu(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *uni, vo
                   bool forward, cudaStream_t st) {
   const Setup &s = gp->s;
   DN_REQUIRE(!gp->type1, ST_INTERNAL, "grouped index made for type 1");
-  if (gp->run_points(g0, g1) == 0) return false;
+  const uint64_t pn = gp->run_points(g0, g1);
+  if (pn == 0) return false;
   const uint32_t n = gp->runs ? grouped_select(gp, g0, g1, st) : 0u;
-  if (!gp->runs && !grouped_chunks(gp, g0, g1, st)) return false;
-  const ChunkList cl{gp->chunks.as<Chunk>(), gp->nchunks};
+  const ChunkList cl = gp->runs ? ChunkList{nullptr, 0} : grouped_chunks(gp, g0, g1, pn, st);
   const PointsDesc pts{gp->sorted_coord.p, 2, 1, true, true, gp->perm.as<uint32_t>(),
                        s.npoints};
   const int dt = s.calc_f64 ? DNUFFT_C128 : DNUFFT_C64;
@@ -2090,12 +2141,15 @@ bool grouped_u2nu(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *uni, vo
   StageTimer tm(false, st);
   if (s.calc_f64)
     do_fft_interp<double>(s, *gp->dc, pts, cl, uv, ov, forward, false, tm, st, &gp->grid,
-                          &gp->work, nullptr, gp->sel.as<uint32_t>(), n);
+                          &gp->work, nullptr, gp->sel.as<uint32_t>(), n, false);
   else
     do_fft_interp<float>(s, *gp->dc, pts, cl, uv, ov, forward, false, tm, st, &gp->grid,
-                         &gp->work);
+                         &gp->work, nullptr, nullptr, 0, false);
   return true;
 }
+
+// the grouped transforms leave their bounded waits to one check after the last
+void grouped_check(cudaStream_t st) { check_device_error(device_error_word(), st); }
 
 void set_last_error(const char *msg) { g_last_error = msg; }
 
@@ -2273,7 +2327,7 @@ int dnufft_plan_destroy(dnufft_plan *plan) {
       plan->sorted_coord.st = st;
       plan->grid.st = st;
       plan->work.st = st;
-      for (int d = 0; d < 3; ++d) plan->dc.corfac[d].st = plan->dc.tw[d].st = st;
+      for (int d = 0; d < 3; ++d) plan->own.corfac[d].st = plan->own.tw[d].st = st;
       for (auto &pg : plan->groups) {
         pg.ix.perm.st = pg.ix.chunks.st = pg.ix.count.st = pg.ix.keys.st = st;
         pg.ix.kblk.st = pg.ix.kbrange.st = st;
@@ -2355,6 +2409,7 @@ int dnufft_selftest_wait_timeout(int64_t limit_ns, void *stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int *err = dnufft::device_error_word();
     dnufft::launch_wait_selftest(err, (unsigned long long)limit_ns, st);
+    dnufft::bounded_wait_launched() = true;
     dnufft::check_device_error(err, st);
   })
 }
@@ -2455,8 +2510,8 @@ static void batch_build(dnufft_batch *b, cudaStream_t st) {
     b->sm_interp = std::max(b->sm_interp, interp_multi_smem<T>(p->s.g));
     FFTBatchInst &f = fi[size_t(i)];
     f.g = p->s.g;
-    f.ax = p->dc.ax;
-    for (int d = 0; d < 3; ++d) f.corfac[d] = p->dc.cf[d];
+    f.ax = p->dc->ax;
+    for (int d = 0; d < 3; ++d) f.corfac[d] = p->dc->cf[d];
     f.grid = s.grid;
     f.ntrans = s.ntrans;
     f.fft_order = p->o.fft_order != 0;

@@ -72,6 +72,8 @@ size_t find_parameters(double epsilon, double sigma_min, double sigma_max,
                        std::vector<size_t> &nover);
 size_t effective_threads(size_t nthreads);
 std::vector<double> kernel_coeffs(int W, double beta_scaled, double e0);
+// the coefficients of a row of kernel_db(), computed once per row
+const std::vector<double> &kernel_coeffs_of(int row);
 std::vector<double> correction_factors(size_t n, double dx, int W, double beta_scaled,
                                        double e0);
 // the quadrature of the correction function 1 / sum_k wpsi[k] cos(pi W x[k] v)
@@ -130,5 +132,8 @@ bool grouped_nu2u(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *values,
                   bool forward, cudaStream_t st);
 bool grouped_u2nu(GroupedPlan *gp, uint32_t g0, uint32_t g1, const void *uni, void *out,
                   bool forward, cudaStream_t st);
+// reads the error word of the transforms' bounded waits back (throws); once,
+// after the last of a call's transforms
+void grouped_check(cudaStream_t st);
 
 }  // namespace dnufft

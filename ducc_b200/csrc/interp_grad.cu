@@ -20,12 +20,14 @@ namespace dnufft {
 
 template <typename T, typename Tc, int NDIM, int W>
 __global__ void __launch_bounds__(SP_THREADS)
-    k_interp_dcoord(PointsDesc pts, const Chunk *__restrict__ chunks, Geometry g,
+    k_interp_dcoord(PointsDesc pts, const Chunk *__restrict__ chunks,
+                    const uint32_t *nchunks, Geometry g,
                     KernelPoly<T> kp, const cplx<T> *__restrict__ grid,
                     const cplx<T> *__restrict__ wts, int64_t ws, Tc *__restrict__ grad,
                     int64_t gs0, int64_t gs1) {
   constexpr bool SMEM = BufferLayout<T>::smem(NDIM);
   extern __shared__ __align__(16) unsigned char smraw[];
+  if (nchunks && blockIdx.x >= *nchunks) return;
   const Chunk ch = chunks[blockIdx.x];
   const int S = (1 << g.log2tile) + W;
   int ncell = S;
@@ -141,7 +143,7 @@ static void dcoord_w(const PointsDesc &pts, const ChunkList &cl, const Geometry 
   size_t sm = interp_smem_bytes<T, NDIM, W>(g);
   auto kern = k_interp_dcoord<T, Tc, NDIM, W>;
   DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-  kern<<<cl.nchunks, SP_THREADS, sm, st>>>(pts, cl.chunks, g, kp,
+  kern<<<cl.nchunks, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
                                           static_cast<const cplx<T> *>(grid),
                                           static_cast<const cplx<T> *>(wts), ws,
                                           static_cast<Tc *>(grad), gs0, gs1);

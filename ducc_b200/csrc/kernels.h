@@ -5,6 +5,11 @@
 
 namespace dnufft {
 
+// set by the launchers of kernels that wait on mbarriers with a time limit and
+// report through the device error word; per host thread, cleared where the word
+// is read back
+bool &bounded_wait_launched();
+
 // ---- binning / sorting (binsort.cu)
 // Order of the points inside a 2D or 3D tile, as key bits below the tile:
 // tensor core (2D, quadrant): the point's quadrant within its tile and below it
@@ -29,9 +34,12 @@ size_t radix_workspace_bytes(uint32_t n, int keybits);
 void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, void *ws,
                       cudaStream_t st);
 size_t chunk_workspace_bytes(uint32_t n);
+// returns the number of chunks, read back (synchronises st): through mapped
+// host memory, or by a memcpy (zero_copy false: nothing is allocated); with
+// read_back false returns 0 and leaves the number in *d_count only
 uint32_t build_chunks(const uint32_t *skeys, uint32_t n, int tile_shift, uint32_t chunk,
                       Chunk *chunks, uint32_t *d_count, void *ws, cudaStream_t st,
-                      bool zero_copy = true);
+                      bool zero_copy = true, bool read_back = true);
 // reads n (1..8) device words into out through mapped host memory; synchronises st
 void read_words(const uint32_t *const *src, int n, uint32_t *out, cudaStream_t st);
 void launch_gather_coords(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
@@ -40,14 +48,14 @@ void launch_gather_coords(bool coord_f64, const void *coord, int64_t cs0, int64_
 
 // grouped index (points sorted by (tile, group)): keys = keys << gbits | group;
 // start[k] (k = 0..nkeys) = first sorted point whose key is >= k; the chunks
-// (at most `chunk` points) of groups [g0, g1) of every tile, their number
-// returned (read back: synchronises st)
+// (at most `chunk` points) of groups [g0, g1) of every tile; returns where their
+// number is on the device (in ws)
 void launch_group_keys(uint32_t *keys, const uint32_t *group, uint32_t n, int gbits,
                        cudaStream_t st);
 void launch_key_starts(const uint32_t *skeys, uint32_t n, uint32_t nkeys, uint32_t *start,
                        cudaStream_t st);
 size_t group_chunk_workspace_bytes(uint32_t ntiles);
-uint32_t build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, uint32_t g0,
+const uint32_t *build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, uint32_t g0,
                             uint32_t g1, uint32_t chunk, Chunk *chunks, void *ws,
                             cudaStream_t st);
 
@@ -73,9 +81,12 @@ struct PointsDesc {
   uint32_t npts;
 };
 
+// nchunks: the number of chunks, or with count an upper bound of it (the true
+// number is *count on the device)
 struct ChunkList {
   const Chunk *chunks;
   uint32_t nchunks;
+  const uint32_t *count = nullptr;
 };
 
 // grid: contiguous oversampled grid (nover[0] x ... ), complex<T>

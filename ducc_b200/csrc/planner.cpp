@@ -16,6 +16,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <cstdlib>
 #include <thread>
 #include <sched.h>
@@ -186,6 +188,18 @@ std::vector<double> kernel_coeffs(int W, double beta, double e0) {
     for (int j = 0; j <= D; ++j) coeff[size_t(j) * W + i] = mono[D - j];
   }
   return coeff;
+}
+
+const std::vector<double> &kernel_coeffs_of(int row) {
+  static std::mutex mu;
+  static std::map<int, std::vector<double>> *cache = new std::map<int, std::vector<double>>();
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = cache->find(row);
+  if (it == cache->end()) {
+    const KernelShape &k = kDB[size_t(row)];
+    it = cache->emplace(row, kernel_coeffs(k.W, k.beta * k.W, k.e0)).first;
+  }
+  return it->second;   // (entries are never removed)
 }
 
 // Gauss-Legendre nodes (x>=0) and weights on [-1,1] by Newton iteration on P_m.

@@ -229,10 +229,11 @@ template <typename T, typename Tc> constexpr int spread_min_ctas() {
 
 template <typename T, typename Tc, int NDIM, int W>
 __global__ void __launch_bounds__(SP_THREADS, spread_min_ctas<T, Tc>())
-    k_spread(PointsDesc pts, const Chunk *__restrict__ chunks, Geometry g, KernelPoly<T> kp,
-             const cplx<T> *__restrict__ values, int64_t vs, int64_t vtrans,
+    k_spread(PointsDesc pts, const Chunk *__restrict__ chunks, const uint32_t *nchunks, Geometry g,
+             KernelPoly<T> kp, const cplx<T> *__restrict__ values, int64_t vs, int64_t vtrans,
              cplx<T> *__restrict__ grid, int64_t gtrans) {
   extern __shared__ __align__(16) unsigned char smraw[];
+  if (nchunks && blockIdx.x >= *nchunks) return;
   spread_chunk<T, Tc, NDIM, W>(pts, chunks[blockIdx.x], g, kp,
                                values + int64_t(blockIdx.y) * vtrans, vs,
                                grid + int64_t(blockIdx.y) * gtrans, smraw);
@@ -597,12 +598,14 @@ template <typename T, int NDIM> constexpr int interp_min_ctas() {
 // transform); err: device error word for a tile copy that never completes
 template <typename T, typename Tc, int NDIM, int W>
 __global__ void __launch_bounds__(SP_THREADS, interp_min_ctas<T, NDIM>())
-    k_interp(PointsDesc pts, const Chunk *__restrict__ chunks, Geometry g, KernelPoly<T> kp,
+    k_interp(PointsDesc pts, const Chunk *__restrict__ chunks, const uint32_t *nchunks, Geometry g,
+             KernelPoly<T> kp,
              const cplx<T> *__restrict__ grid, int64_t gtrans, cplx<T> *__restrict__ out,
              int64_t os, int64_t otrans, const __grid_constant__ CUtensorMap tmap, int tpitch,
              int *err) {
   extern __shared__ __align__(128) unsigned char smraw_tile[];
   __shared__ uint64_t tbar;
+  if (nchunks && blockIdx.x >= *nchunks) return;
   interp_chunk<T, Tc, NDIM, W>(pts, chunks[blockIdx.x], g, kp, grid + int64_t(blockIdx.y) * gtrans,
                                out + int64_t(blockIdx.y) * otrans, os, smraw_tile,
                                tpitch > 0 ? &tmap : nullptr, tpitch, &tbar, err);
@@ -645,8 +648,8 @@ void spread_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
   auto kern = k_spread<T, Tc, NDIM, W>;
   DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   dim3 grd(cl.nchunks, ntrans);
-  kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, g, kp, static_cast<const cplx<T> *>(values), vs,
-                                    vtrans, static_cast<cplx<T> *>(grid), gtrans);
+  kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
+                                    static_cast<const cplx<T> *>(values), vs, vtrans, static_cast<cplx<T> *>(grid), gtrans);
   DN_LAUNCHED();
 }
 
@@ -668,10 +671,11 @@ void interp_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
   auto kern = k_interp<T, Tc, NDIM, W>;
   DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   dim3 grd(cl.nchunks, ntrans);
-  kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, g, kp, static_cast<const cplx<T> *>(grid),
-                                    gtrans, static_cast<cplx<T> *>(out), os, otrans, map, tpitch,
+  kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
+                                    static_cast<const cplx<T> *>(grid), gtrans, static_cast<cplx<T> *>(out), os, otrans, map, tpitch,
                                     err);
   DN_LAUNCHED();
+  if (tpitch > 0) bounded_wait_launched() = true;
 }
 
 // W dispatch: float supports W 4..8, double 4..16 (the kernel table's ranges)

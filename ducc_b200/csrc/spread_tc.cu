@@ -1003,6 +1003,7 @@ void launch_spread_tc(const PointsDesc &pts, const TcBlocks &tb, const Geometry 
                                                static_cast<const float2 *>(values), vs, absmax, \
                                                static_cast<float2 *>(grid), err);               \
     DN_LAUNCHED();                                                                              \
+    bounded_wait_launched() = true;                                                             \
     return;                                                                                     \
   }
   if (pts.coord_f64) {

@@ -1001,6 +1001,7 @@ static void vis2dirty_t(const Inputs &in, double psx, double psy, double eps,
     k_wg_correct<T><<<grid_for(nx * ny), 256, 0, st>>>(dp, dirty.stride[0], dirty.stride[1], g,
                                                        cn, P.dw, o.divide_by_n);
     DN_LAUNCHED();
+    grouped_check(st);
     return;
   }
   PlaneOrder<C> po;
@@ -1101,6 +1102,7 @@ static void dirty2vis_t(const Inputs &in, const Arr &dirty, double psx, double p
         ptr<cplx<C>>(acc), ptr<double>(cv.coord), ptr<double>(cv.wv), ptr<uint32_t>(cv.idx),
         cv.nvis, in.c, P.lshift, P.mshift, P.nshift, vp, vis.stride[0], vis.stride[1]);
     DN_LAUNCHED();
+    grouped_check(st);
     return;
   }
   PlaneOrder<C> po;
