@@ -4,8 +4,9 @@
 //                  tile key (src/ducc0/nufft/nufft.h:892-907, :1364-1381,
 //                  :1862-1892).
 //  radix sort    - stable LSD radix sort of (key, index) pairs, up to 11 bits per
-//                  pass: per-block digit histograms, one device-wide exclusive
-//                  scan, and a scatter whose in-block ranks come from warp-level
+//                  pass: per-block digit histograms, an exclusive scan of every
+//                  digit's row of them (one launch; each scatter block adds up the
+//                  digits' totals itself), and a scatter whose in-block ranks come from warp-level
 //                  __match_any_sync, so equal keys keep their input order.  A
 //                  stable sort by key reproduces DUCC's coord_idx exactly
 //                  (bucket_sort2, src/ducc0/infra/bucket_sort.h:170-354).
@@ -210,13 +211,45 @@ __global__ void k_radix_hist(const uint32_t *__restrict__ keys, uint32_t n, int 
     hist[uint64_t(i) * nblocks + blockIdx.x] = sh[i];
 }
 
+// exclusive scan of row d = blockIdx.x of the histograms in place, its sum to
+// totals[d]
+__global__ void k_radix_scan(uint32_t *__restrict__ hist, uint32_t nblocks,
+                             uint32_t *__restrict__ totals) {
+  __shared__ uint32_t ws[32];
+  uint32_t *row = hist + uint64_t(blockIdx.x) * nblocks;
+  uint32_t carry = 0;
+  for (uint32_t b = 0; b < nblocks; b += blockDim.x) {
+    const uint32_t i = b + threadIdx.x;
+    const uint32_t v = i < nblocks ? row[i] : 0u;
+    uint32_t tot;
+    const uint32_t ex = block_excl_scan(v, ws, &tot);
+    if (i < nblocks) row[i] = carry + ex;
+    carry += tot;
+    __syncthreads();   // (ws)
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
 __global__ void k_radix_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                                 uint32_t *__restrict__ kout, uint32_t *__restrict__ vout,
                                 uint32_t n, int shift, int nbits,
-                                const uint32_t *__restrict__ offs, uint32_t nblocks) {
+                                const uint32_t *__restrict__ offs,
+                                const uint32_t *__restrict__ totals, uint32_t nblocks) {
   extern __shared__ uint32_t sh[];
+  __shared__ uint32_t ws[32];
   const int nb = 1 << nbits;
   uint32_t *whist = sh;                        // [RS_WARPS][nb] counts, then offsets
+  uint32_t *dbase = sh + RS_WARPS * nb;        // [nb] first position of every digit
+  {
+    const int per = (nb + int(blockDim.x) - 1) / int(blockDim.x), d0 = int(threadIdx.x) * per;
+    uint32_t s = 0;
+    for (int d = d0; d < min(d0 + per, nb); ++d) s += totals[d];
+    uint32_t run = block_excl_scan(s, ws, nullptr);
+    for (int d = d0; d < min(d0 + per, nb); ++d) {
+      dbase[d] = run;
+      run += totals[d];
+    }
+  }
   const uint32_t mask = uint32_t(nb - 1);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < RS_WARPS * nb; i += blockDim.x) whist[i] = 0;
@@ -241,7 +274,7 @@ __global__ void k_radix_scatter(const uint32_t *__restrict__ kin, const uint32_t
   __syncthreads();
   // per digit: global offset of this block + counts of earlier warps
   for (int d = threadIdx.x; d < nb; d += blockDim.x) {
-    uint32_t run = offs[uint64_t(d) * nblocks + blockIdx.x];
+    uint32_t run = dbase[d] + offs[uint64_t(d) * nblocks + blockIdx.x];
 #pragma unroll
     for (int ww = 0; ww < RS_WARPS; ++ww) {
       uint32_t c = whist[ww * nb + d];
@@ -268,8 +301,8 @@ size_t radix_workspace_bytes(uint32_t n, int keybits) {
   uint64_t nblocks = (uint64_t(n) + RS_TILE - 1) / RS_TILE;
   uint64_t hn = (uint64_t(1) << nbits) * nblocks;
   return 2 * size_t(n) * sizeof(uint32_t)       // ping-pong keys/values
-         + 2 * hn * sizeof(uint32_t)            // histogram + offsets
-         + scan_workspace_bytes(hn) + 1024;
+         + hn * sizeof(uint32_t)                // histograms, scanned in place
+         + (sizeof(uint32_t) << nbits) + 256;   // totals of the digits
 }
 
 // element-wise copy of the sorted pairs back (the ping-pong halves of the
@@ -297,28 +330,27 @@ void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, v
   p += size_t(n) * 4;
   uint32_t *hist = reinterpret_cast<uint32_t *>(p);
   p += hn * 4;
-  uint32_t *offs = reinterpret_cast<uint32_t *>(p);
-  p += hn * 4;
-  uint32_t *sws = reinterpret_cast<uint32_t *>((reinterpret_cast<uintptr_t>(p) + 255) & ~uintptr_t(255));
+  uint32_t *totals = reinterpret_cast<uint32_t *>(p);
   uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
   size_t hsm = sizeof(uint32_t) << nbits;
-  size_t ssm = size_t(RS_WARPS) * hsm;
+  size_t ssm = size_t(RS_WARPS + 1) * hsm;
   static bool attr_set = false;
   if (!attr_set) {
     DN_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 RS_WARPS * (4 << RADIX_BITS)));
+                                 (RS_WARPS + 1) * (4 << RADIX_BITS)));
     attr_set = true;
   }
   for (int pass = 0; pass < passes; ++pass) {
     int shift = pass * nbits;
     int bits = (keybits - shift < nbits) ? keybits - shift : nbits;
     if (bits <= 0) break;
-    uint64_t hn_pass = (uint64_t(1) << bits) * nblocks;
     k_radix_hist<<<nblocks, 256, hsm, st>>>(ka, n, shift, bits, hist, nblocks);
     DN_LAUNCHED();
-    exclusive_scan(hist, offs, hn_pass, sws, st);
-    k_radix_scatter<<<nblocks, RS_WARPS * 32, ssm, st>>>(ka, va, kb, vb, n, shift, bits, offs,
-                                                         nblocks);
+    k_radix_scan<<<1u << bits, nblocks <= 128 ? 32 : (nblocks <= 2048 ? 256 : 1024), 0,
+                   st>>>(hist, nblocks, totals);
+    DN_LAUNCHED();
+    k_radix_scatter<<<nblocks, RS_WARPS * 32, ssm, st>>>(ka, va, kb, vb, n, shift, bits, hist,
+                                                         totals, nblocks);
     DN_LAUNCHED();
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -419,25 +451,77 @@ void read_words(const uint32_t *const *src, int n, uint32_t *out, cudaStream_t s
   for (int i = 0; i < n; ++i) out[i] = h[i];
 }
 
+// The chunk list of up to CHUNK_TILES tiles: where every tile starts (a binary
+// search each), then one block counts, scans and writes.  Two launches over the
+// tiles instead of seven over the points.
+constexpr uint32_t CHUNK_TILES = 16384;
+constexpr int CT_THREADS = 1024;
+
+__global__ void k_tile_starts(const uint32_t *__restrict__ skeys, uint32_t n, int tile_shift,
+                              uint32_t ntiles, uint32_t *__restrict__ start) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t > ntiles) return;
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo) / 2;
+    if ((skeys[mid] >> tile_shift) < t) lo = mid + 1;
+    else hi = mid;
+  }
+  start[t] = lo;
+}
+
+__global__ void __launch_bounds__(CT_THREADS)
+    k_tile_chunks(const uint32_t *__restrict__ start, uint32_t ntiles, uint32_t chunk,
+                  Chunk *__restrict__ chunks, uint32_t *__restrict__ count) {
+  __shared__ uint32_t ws[32];
+  const uint32_t per = (ntiles + CT_THREADS - 1) / CT_THREADS;
+  const uint32_t t0 = min(ntiles, threadIdx.x * per), t1 = min(ntiles, t0 + per);
+  uint32_t s = 0;
+  for (uint32_t t = t0; t < t1; ++t) s += (start[t + 1] - start[t] + chunk - 1) / chunk;
+  uint32_t tot;
+  uint32_t pos = block_excl_scan(s, ws, &tot);
+  for (uint32_t t = t0; t < t1; ++t) {
+    const uint32_t e = start[t + 1];
+    for (uint32_t b = start[t]; b < e; b += chunk) {
+      Chunk c;
+      c.start = b;
+      c.count = min(chunk, e - b);
+      c.tile = t;
+      c.pad = 0;
+      chunks[pos++] = c;
+    }
+  }
+  if (threadIdx.x == 0) *count = tot;
+}
+
 // Builds the chunk list from sorted keys.
 uint32_t build_chunks(const uint32_t *skeys, uint32_t n, int tile_shift, uint32_t chunk,
                       Chunk *chunks, uint32_t *d_count, void *ws, cudaStream_t st,
-                      bool zero_copy, bool read_back) {
+                      bool zero_copy, bool read_back, uint64_t ntiles) {
   if (n == 0) return 0;
-  uint32_t *flags = static_cast<uint32_t *>(ws);
-  uint32_t *pos = flags + n;
-  uint32_t *sws = reinterpret_cast<uint32_t *>(
-      (reinterpret_cast<uintptr_t>(pos + n) + 255) & ~uintptr_t(255));
-  unsigned g = (n + 255) / 256;
-  k_chunk_flags<<<g, 256, 0, st>>>(skeys, n, tile_shift, chunk, flags);
-  DN_LAUNCHED();
-  exclusive_scan(flags, pos, n, sws, st);
-  k_chunk_fill<<<g, 256, 0, st>>>(skeys, flags, pos, n, tile_shift, chunks);
-  DN_LAUNCHED();
-  k_count_total<<<1, 1, 0, st>>>(flags, pos, n, d_count);
-  DN_LAUNCHED();
-  k_chunk_counts<<<g, 256, 0, st>>>(chunks, d_count, n);
-  DN_LAUNCHED();
+  if (ntiles <= CHUNK_TILES && ntiles < 2 * uint64_t(n)) {   // (its table fits ws)
+    uint32_t *start = static_cast<uint32_t *>(ws);
+    k_tile_starts<<<unsigned(ntiles / 256 + 1), 256, 0, st>>>(skeys, n, tile_shift,
+                                                              uint32_t(ntiles), start);
+    DN_LAUNCHED();
+    k_tile_chunks<<<1, CT_THREADS, 0, st>>>(start, uint32_t(ntiles), chunk, chunks, d_count);
+    DN_LAUNCHED();
+  } else {
+    uint32_t *flags = static_cast<uint32_t *>(ws);
+    uint32_t *pos = flags + n;
+    uint32_t *sws = reinterpret_cast<uint32_t *>(
+        (reinterpret_cast<uintptr_t>(pos + n) + 255) & ~uintptr_t(255));
+    unsigned g = (n + 255) / 256;
+    k_chunk_flags<<<g, 256, 0, st>>>(skeys, n, tile_shift, chunk, flags);
+    DN_LAUNCHED();
+    exclusive_scan(flags, pos, n, sws, st);
+    k_chunk_fill<<<g, 256, 0, st>>>(skeys, flags, pos, n, tile_shift, chunks);
+    DN_LAUNCHED();
+    k_count_total<<<1, 1, 0, st>>>(flags, pos, n, d_count);
+    DN_LAUNCHED();
+    k_chunk_counts<<<g, 256, 0, st>>>(chunks, d_count, n);
+    DN_LAUNCHED();
+  }
   uint32_t h = 0;
   if (!read_back) return 0;
   if (zero_copy) {

@@ -664,7 +664,7 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
   DevBuf ws(chunk_workspace_bytes(M), st);
   const uint32_t n = build_chunks(ix.keys.as<uint32_t>(), M, s.tile_shift, s.chunk,
                                   ix.chunks.as<Chunk>(), ix.count.as<uint32_t>(), ws.p, st, true,
-                                  s.qbits);
+                                  s.qbits, s.max_tiles);
   ix.counted = s.qbits || M == 0;
   ix.nchunks = ix.counted ? n : uint32_t(std::min<uint64_t>(maxchunks, M));
   if (s.qbits && ix.nchunks > 0) {

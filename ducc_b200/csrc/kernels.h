@@ -36,10 +36,12 @@ void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, v
 size_t chunk_workspace_bytes(uint32_t n);
 // returns the number of chunks, read back (synchronises st): through mapped
 // host memory, or by a memcpy (zero_copy false: nothing is allocated); with
-// read_back false returns 0 and leaves the number in *d_count only
+// read_back false returns 0 and leaves the number in *d_count only.  ntiles: the
+// number of tiles (every tile < ntiles) where known
 uint32_t build_chunks(const uint32_t *skeys, uint32_t n, int tile_shift, uint32_t chunk,
                       Chunk *chunks, uint32_t *d_count, void *ws, cudaStream_t st,
-                      bool zero_copy = true, bool read_back = true);
+                      bool zero_copy = true, bool read_back = true,
+                      uint64_t ntiles = ~uint64_t(0));
 // reads n (1..8) device words into out through mapped host memory; synchronises st
 void read_words(const uint32_t *const *src, int n, uint32_t *out, cudaStream_t st);
 void launch_gather_coords(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
