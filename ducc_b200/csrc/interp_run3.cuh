@@ -1,0 +1,216 @@
+// Double-precision 3D interpolation (type 2) with the window of a bin in
+// registers: the transpose of spread_run3.cuh.
+//
+// A CTA takes consecutive sorted points and has one warp per plane of the window
+// of their bin (8^3 cells, 4^3 for W > 12).  A batch of points is staged in
+// shared memory (plane, row and column weights, zero-filled to the window); every
+// warp keeps its plane of the grid in the fragments of FP64 matrix instructions
+// (as k_interp_run), forms the points' sums over the plane eight at a time
+// (skipping those whose footprints do not touch it) and leaves them, times the
+// plane weight, in shared memory, where they are added over the planes.
+//
+// Reading W^3 cells of 16 bytes through L1 per point took 700 SM cycles per point
+// at W = 12; the matrix instructions take 165.
+//
+// Mirrors HelperU2nu / interpolation_helper (src/ducc0/nufft/nufft.h:1508-1729).
+#pragma once
+
+#include "interp_run.cuh"
+#include "spread_run3.cuh"
+
+namespace dnufft {
+
+template <int W> struct Interp3Shape {
+  static constexpr int LB = run3_bin_log2(W), BIN = 1 << LB;
+  static constexpr int SPAN = BIN - 1 + W;
+  static constexpr int RT = (SPAN + 3) / 4, KT = (SPAN + 3) / 4;
+  static constexpr int PLANES = (SPAN + 3) / 4 * 4, ROWS = 4 * RT, COLS = 4 * KT;
+  static constexpr int THREADS = 32 * SPAN;
+  static constexpr int BATCH = 64;
+  static constexpr int ST0 = PLANES + ROWS + COLS;
+  static constexpr int ST = ST0 % 8 == 4 ? ST0 : ST0 + 4;   // 4 or 12 modulo 16
+  static constexpr size_t SMEM = size_t(BATCH) * ST * 8 + size_t(SPAN) * BATCH * 16 +
+                                 size_t(BATCH) * sizeof(int4);
+};
+
+template <typename Tc, int W>
+__global__ void __launch_bounds__(Interp3Shape<W>::THREADS)
+    k_interp_run3(const __grid_constant__ PointsDesc pts, uint32_t ppb,
+                  const __grid_constant__ Geometry g, const __grid_constant__ KernelPoly<double> kp,
+                  const double2 *__restrict__ grid, int64_t gtrans, double2 *__restrict__ out,
+                  int64_t os, int64_t otrans) {
+  using R = Interp3Shape<W>;
+  constexpr int B = R::BATCH;
+  extern __shared__ __align__(16) unsigned char smraw_run[];
+  double *st = reinterpret_cast<double *>(smraw_run);
+  double2 *part = reinterpret_cast<double2 *>(st + B * R::ST);   // [plane][point]
+  // every staged point: bins of the three axes, output index
+  int4 *info = reinterpret_cast<int4 *>(part + R::SPAN * B);
+  grid += int64_t(blockIdx.y) * gtrans;
+  out += int64_t(blockIdx.y) * otrans;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n0 = int(g.nover[0]), n1 = int(g.nover[1]), n2 = int(g.nover[2]);
+  const uint32_t first = blockIdx.x * ppb;
+  const uint32_t last = uint32_t(min(uint64_t(pts.npts), uint64_t(first) + ppb));
+  double G[R::RT][R::KT];
+  int cu = -1, cv = -1, cw = -1;
+  bool finite = true;
+  auto load_window = [&]() {
+    const int u = wrap2(cu * R::BIN - g.nsafe + warp, n0), v0 = cv * R::BIN - g.nsafe,
+              w0 = cw * R::BIN - g.nsafe;
+    const double *pl = reinterpret_cast<const double *>(grid + int64_t(u) * n1 * n2) +
+                       ((lane >> 2) & 1);
+    bool ok = true;
+#pragma unroll
+    for (int r = 0; r < R::RT; ++r) {
+      const double *row = pl + 2 * int64_t(wrap2(v0 + 4 * r + (lane >> 3), n1)) * n2;
+#pragma unroll
+      for (int k = 0; k < R::KT; ++k) {
+        G[r][k] = __ldg(row + 2 * wrap2(w0 + 4 * k + (lane & 3), n2));
+        ok = ok && isfinite(G[r][k]);
+      }
+    }
+    finite = __all_sync(0xffffffffu, ok);
+  };
+  for (uint32_t base = first; base < last; base += B) {
+    const int np = int(min(uint32_t(B), last - base));
+    {
+      // (every thread is past the reads of the last batch: the barrier before
+      // its sums)
+      float4 *z4 = reinterpret_cast<float4 *>(st);
+      const int nz = np * (R::ST / 2);
+      for (int i = tid; i < nz; i += R::THREADS) z4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    for (int it = tid; it < 3 * np; it += R::THREADS) {
+      const int ax = it / np, q = it - ax * np;
+      const uint32_t i = base + uint32_t(q), j = pts.perm[i];
+      const Tc *c = static_cast<const Tc *>(pts.coord);
+      const Tc x = pts.sorted ? c[uint64_t(i) * 3 + ax]
+                              : c[int64_t(j) * pts.cs0 + int64_t(ax) * pts.cs1];
+      int i0;
+      double frac, w[W];
+      fold<Tc>(x, ax == 0 ? g.coordfct[0] : (ax == 1 ? g.coordfct[1] : g.coordfct[2]),
+               ax == 0 ? n0 : (ax == 1 ? n1 : n2),
+               ax == 0 ? g.shift[0] : (ax == 1 ? g.shift[1] : g.shift[2]),
+               ax == 0 ? g.maxi0[0] : (ax == 1 ? g.maxi0[1] : g.maxi0[2]), i0, frac);
+      kernel_weights<double, W>(kp, double(W - 1) - 2.0 * frac, w);
+      const int t = i0 + g.nsafe;
+      int *inf = reinterpret_cast<int *>(info + q);
+      inf[ax] = t >> R::LB;
+      if (ax == 0) inf[3] = int(j);
+      double *sp = st + q * R::ST + (ax == 0 ? 0 : (ax == 1 ? R::PLANES : R::PLANES + R::ROWS)) +
+                   (t & (R::BIN - 1));
+#pragma unroll
+      for (int a = 0; a < W; ++a) sp[a] = w[a];
+    }
+    __syncthreads();
+    for (int s0 = 0; s0 < np; s0 += 32) {
+      const int p0 = s0 + lane, ns = min(32, np - s0);
+      const int4 b = info[min(p0, np - 1)];
+      int pu = __shfl_up_sync(0xffffffffu, b.x, 1), pv = __shfl_up_sync(0xffffffffu, b.y, 1),
+          pw = __shfl_up_sync(0xffffffffu, b.z, 1);
+      if (lane == 0) {
+        pu = cu;
+        pv = cv;
+        pw = cw;
+      }
+      const unsigned bins =
+          __ballot_sync(0xffffffffu, p0 < np && (b.x != pu || b.y != pv || b.z != pw));
+      unsigned rest = bins & ~1u;
+      for (int s = 0; s < ns;) {
+        if ((bins >> s) & 1u) {
+          cu = __shfl_sync(0xffffffffu, b.x, s);
+          cv = __shfl_sync(0xffffffffu, b.y, s);
+          cw = __shfl_sync(0xffffffffu, b.z, s);
+          load_window();
+        }
+        const int e = rest ? __ffs(rest) - 1 : ns;
+        rest &= rest - 1;
+        for (int p = s; p < e; p += 8) {
+          const int pt = s0 + p + (lane >> 2);
+          const bool on = p + (lane >> 2) < e;
+          const double *f = st + (on ? pt : s0 + p) * R::ST;
+          const double ku = on ? f[warp] : 0.;
+          double sx = 0., sy = 0.;
+          if (__any_sync(0xffffffffu, ku != 0.)) {
+            if (finite) {
+              double a[R::KT];
+#pragma unroll
+              for (int k = 0; k < R::KT; ++k) a[k] = f[R::PLANES + R::ROWS + 4 * k + (lane & 3)];
+#pragma unroll
+              for (int r = 0; r < R::RT; ++r) {
+                double c0 = 0., c1 = 0.;
+#pragma unroll
+                for (int k = 0; k < R::KT; ++k)
+                  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, "
+                      "{%0, %1};"
+                      : "+d"(c0), "+d"(c1)
+                      : "d"(a[k]), "d"(G[r][k]));
+                const double kv = f[R::PLANES + 4 * r + (lane & 3)];
+                sx += kv * c0;
+                sy += kv * c1;
+              }
+            } else if (ku != 0.) {
+              // a value of the plane is not finite: the footprint's cells only
+              const double2 *pl =
+                  grid + int64_t(wrap2(cu * R::BIN - g.nsafe + warp, n0)) * n1 * n2;
+              for (int r = lane & 3; r < R::SPAN; r += 4) {
+                const double kv = f[R::PLANES + r];
+                if (kv == 0.) continue;
+                const double2 *row = pl + int64_t(wrap2(cv * R::BIN - g.nsafe + r, n1)) * n2;
+                for (int c = 0; c < R::SPAN; ++c) {
+                  const double wt = kv * f[R::PLANES + R::ROWS + c];
+                  if (wt == 0.) continue;
+                  const double2 gv = __ldg(row + wrap2(cw * R::BIN - g.nsafe + c, n2));
+                  sx += wt * gv.x;
+                  sy += wt * gv.y;
+                }
+              }
+            }
+            sx += __shfl_xor_sync(0xffffffffu, sx, 1);
+            sy += __shfl_xor_sync(0xffffffffu, sy, 1);
+            sx += __shfl_xor_sync(0xffffffffu, sx, 2);
+            sy += __shfl_xor_sync(0xffffffffu, sy, 2);
+          }
+          // (a plane the point does not touch: exactly zero)
+          if (on && (lane & 3) == 0)
+            part[warp * B + pt] = ku != 0. ? make_double2(ku * sx, ku * sy) : make_double2(0., 0.);
+        }
+        s = e;
+      }
+    }
+    __syncthreads();
+    for (int q = tid; q < np; q += R::THREADS) {
+      double sx = 0., sy = 0.;
+      for (int pl = 0; pl < R::SPAN; ++pl) {
+        const double2 v = part[pl * B + q];
+        sx += v.x;
+        sy += v.y;
+      }
+      out[int64_t(uint32_t(info[q].w)) * os] = make_double2(sx, sy);
+    }
+    // the next batch's zeroing touches st only; info and part are written after
+    // its first barrier
+  }
+}
+
+template <typename Tc, int W>
+void interp_run3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<double> &kp,
+                   const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
+                   int ntrans, cudaStream_t st) {
+  using R = Interp3Shape<W>;
+  auto kern = k_interp_run3<Tc, W>;
+  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(R::SMEM)));
+  // points per CTA: as the spreader
+  const uint64_t per = uint64_t(pts.npts) * uint64_t(ntrans) / (148 * 8);
+  const uint32_t ppb =
+      per >= R::BATCH ? R::BATCH * uint32_t(std::min<uint64_t>(16, per / R::BATCH))
+                      : std::max<uint32_t>(16, uint32_t(per) & ~15u);
+  dim3 grd((pts.npts + ppb - 1) / ppb, ntrans);
+  kern<<<grd, R::THREADS, R::SMEM, st>>>(pts, ppb, g, kp, static_cast<const double2 *>(grid),
+                                         gtrans, static_cast<double2 *>(out), os, otrans);
+  DN_LAUNCHED();
+}
+
+}  // namespace dnufft

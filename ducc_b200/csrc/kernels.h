@@ -128,6 +128,11 @@ void launch_interp_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts
                        int64_t gtrans, void *out, int64_t os, int64_t otrans, int ntrans,
                        cudaStream_t st);
 
+// 3D double precision (launch_interp goes here; no chunk list)
+void launch_interp_run3(const PointsDesc &pts, const Geometry &g, const KernelPoly<double> &kp,
+                        const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
+                        int ntrans, cudaStream_t st);
+
 // grad[j*gs0 + d*gs1] = Re(conj(wts[j*ws]) * d/dx_{j,d} interp(grid)(x_j)), in
 // the coordinates' dtype (interp_grad.cu)
 template <typename T>

@@ -1,14 +1,14 @@
-// Plain spreading (type 1; 1D and 3D, 2D: spread_run.cuh) and interpolation
-// (type 2) kernels.
+// Plain spreading (type 1, 1D; 2D and 3D: spread_run.cuh, spread_run3.cuh) and
+// interpolation (type 2, 1D and single precision; double in 2D and 3D:
+// interp_run.cuh, interp_run3.cuh) kernels.
 //
 // One CTA per chunk of tile-sorted points (at most CHUNK points of one tile).
 // Spreading: every warp takes 32 points at a time, each lane folds its point
-// and evaluates the W weights per axis by Horner in registers, stages them in
-// shared memory, then the warp walks the 32 points and its lanes cover the
-// W^d footprint of one point together (no two lanes touch the same cell), adding
-// into a shared-memory copy of the tile plus halo with shared-memory atomics
-// (the per-point FP32/FP64 atomics of the plain form).  The tile buffer is
-// flushed once with vectorised global atomics at wrapped grid positions.
+// and evaluates the W weights by Horner in registers, stages them in shared
+// memory, then the warp walks the 32 points, W lanes covering the W cells of a
+// point, 32 / W points together, adding into a shared-memory copy of the tile plus halo
+// with shared-memory atomics.  The tile buffer is flushed once with vectorised
+// global atomics at wrapped grid positions.
 // Interpolation: the tile plus halo is staged in shared memory and every thread
 // evaluates one point (weights in registers, W^d multiply-adds), writing the
 // result through the tile permutation.  In 2D a tile that lies inside the grid
@@ -66,9 +66,7 @@ __device__ __forceinline__ uint32_t load_point(const PointsDesc &pts, uint32_t i
 // per-lane stride of the staged weights: odd, so that the 32 lanes writing
 // their own weights hit 32 different banks; even entry count keeps the
 // following complex values aligned
-template <int NDIM, int W> constexpr int stage_stride() {
-  return ((NDIM * W) % 2 == 0) ? NDIM * W + 1 : NDIM * W;
-}
+template <int W> constexpr int stage_stride() { return W % 2 == 0 ? W + 1 : W; }
 
 template <typename T> struct BufferLayout {
   // does the tile buffer live in shared memory for this (precision, ndim)?
@@ -117,126 +115,78 @@ __device__ __forceinline__ int64_t cell_index(int c, int S, uint32_t mS, bool fa
   return gidx;
 }
 
-// One chunk of one transform (the body of k_spread).
-template <typename T, typename Tc, int NDIM, int W>
-__device__ __forceinline__ void spread_chunk(const PointsDesc &pts, const Chunk ch, const Geometry &g,
-                                             const KernelPoly<T> &kp,
-                                             const cplx<T> *__restrict__ values, int64_t vs,
-                                             cplx<T> *__restrict__ grid, unsigned char *smraw) {
-  constexpr bool SMEM = BufferLayout<T>::smem(NDIM);
-  constexpr int FP = (NDIM == 1) ? W : (NDIM == 2 ? W * W : W * W * W);
-  constexpr int NIT = (FP + 31) / 32;
-  constexpr int UNR = NIT <= 8 ? NIT : 4;
+template <typename T, typename Tc, int W>
+__global__ void __launch_bounds__(SP_THREADS)
+    k_spread(PointsDesc pts, const Chunk *__restrict__ chunks, const uint32_t *nchunks, Geometry g,
+             KernelPoly<T> kp, const cplx<T> *__restrict__ values, int64_t vs, int64_t vtrans,
+             cplx<T> *__restrict__ grid, int64_t gtrans) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  if (nchunks && blockIdx.x >= *nchunks) return;
+  const Chunk ch = chunks[blockIdx.x];
+  values += int64_t(blockIdx.y) * vtrans;
+  grid += int64_t(blockIdx.y) * gtrans;
   const int S = (1 << g.log2tile) + W;
-  int ncell = S;
-  if (NDIM >= 2) ncell *= S;
-  if (NDIM >= 3) ncell *= S;
-  int b0[NDIM];
-  tile_origin<NDIM>(ch.tile, g, b0);
-  const uint32_t mS = fastdiv_magic(uint32_t(S));
-  const bool fastwrap = fast_wrap_ok<NDIM>(g, S);
+  int b0[1];
+  tile_origin<1>(ch.tile, g, b0);
   cplx<T> *buf = reinterpret_cast<cplx<T> *>(smraw);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned char *stage = smraw + (SMEM ? size_t(ncell) * sizeof(cplx<T>) : 0);
-  constexpr int WS = stage_stride<NDIM, W>();   // per-lane weight stride (odd)
+  unsigned char *stage = smraw + size_t(S) * sizeof(cplx<T>);
+  constexpr int WS = stage_stride<W>();   // per-lane weight stride (odd)
   T *stw = reinterpret_cast<T *>(stage) + warp * 32 * WS;
   cplx<T> *stv = reinterpret_cast<cplx<T> *>(reinterpret_cast<T *>(stage) + SP_WARPS * 32 * WS) +
                  warp * 32;
   int *sto = reinterpret_cast<int *>(reinterpret_cast<cplx<T> *>(reinterpret_cast<T *>(stage) +
                                                                  SP_WARPS * 32 * WS) +
                                      SP_WARPS * 32) +
-             warp * 32 * NDIM;
-  if constexpr (SMEM) {
-    for (int c = threadIdx.x; c < ncell; c += SP_THREADS) buf[c] = mkc<T>(T(0), T(0));
-    __syncthreads();
-  }
+             warp * 32;
+  for (int c = threadIdx.x; c < S; c += SP_THREADS) buf[c] = mkc<T>(T(0), T(0));
+  __syncthreads();
   const uint32_t end = ch.start + ch.count;
   // points per warp and round: 32, or fewer for a chunk of fewer than
   // 32 * SP_WARPS points, so that every warp takes a share of a small chunk
   // (each warp walks its points one by one)
   const int pw = min(32, max(1, int((ch.count + SP_WARPS - 1) / SP_WARPS)));
   for (uint32_t base = ch.start + uint32_t(warp * pw); base < end; base += SP_WARPS * pw) {
-    uint32_t i = base + lane;
+    const uint32_t i = base + lane;
     if (lane < pw && i < end) {
-      Tc x[NDIM];
-      uint32_t j = load_point<Tc, NDIM>(pts, i, x);
+      Tc x[1];
+      const uint32_t j = load_point<Tc, 1>(pts, i, x);
       // a gather through the permutation: cached in L2 only, so a miss
       // brings one 32-byte sector instead of a whole L1 line
-      cplx<T> v = __ldcg(values + int64_t(j) * vs);
+      const cplx<T> v = __ldcg(values + int64_t(j) * vs);
+      int i0;
+      double frac;
+      fold<Tc>(x[0], g.coordfct[0], int(g.nover[0]), g.shift[0], g.maxi0[0], i0, frac);
+      T w[W];
+      kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w);
 #pragma unroll
-      for (int d = 0; d < NDIM; ++d) {
-        int i0;
-        double frac;
-        fold<Tc>(x[d], g.coordfct[d], int(g.nover[d]), g.shift[d], g.maxi0[d], i0, frac);
-        T w[W];
-        kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w);
-#pragma unroll
-        for (int a = 0; a < W; ++a) stw[lane * WS + d * W + a] = w[a];
-        sto[lane * NDIM + d] = i0 - b0[d];
-      }
+      for (int a = 0; a < W; ++a) stw[lane * WS + a] = w[a];
+      sto[lane] = i0 - b0[0];
       stv[lane] = v;
     }
     __syncwarp();
-    int np = min(pw, int(end - base));
-    for (int p = 0; p < np; ++p) {
-      const cplx<T> v = stv[p];
-      const T *wp = stw + p * WS;
-      int o[NDIM];
-#pragma unroll
-      for (int d = 0; d < NDIM; ++d) o[d] = sto[p * NDIM + d];
-#pragma unroll UNR
-      for (int c0 = 0; c0 < FP; c0 += 32) {
-        int c = c0 + lane;
-        if (FP % 32 == 0 || c < FP) {
-          T wt;
-          int cell;
-          if constexpr (NDIM == 1) {
-            wt = wp[c];
-            cell = o[0] + c;
-          } else {
-            int a = c / (W * W), r = c - a * (W * W), b = r / W, e = r - b * W;
-            wt = wp[a] * wp[W + b] * wp[2 * W + e];
-            cell = ((o[0] + a) * S + (o[1] + b)) * S + (o[2] + e);
-          }
-          T re = wt * v.x, im = wt * v.y;
-          if constexpr (SMEM) {
-            atomicAdd(&buf[cell].x, re);
-            atomicAdd(&buf[cell].y, im);
-          } else {
-            // direct global accumulation at wrapped positions
-            global_add<T>(grid + cell_index<NDIM>(cell, S, mS, fastwrap, b0, g), re, im);
-          }
-        }
+    const int np = min(pw, int(end - base));
+    // W lanes per point; in single precision 32 / W points at a time (3e6 points:
+    // 212 -> 158 us a pass; in double the atomics of more points collide, no gain)
+    constexpr int GP = sizeof(T) == 4 ? 32 / W : 1;
+    const int gp = lane / W, a = lane - gp * W;
+    for (int p = gp; p < np; p += GP) {
+      if (gp < GP) {
+        const cplx<T> v = stv[p];
+        const T wt = stw[p * WS + a];
+        const int cell = sto[p] + a;
+        atomicAdd(&buf[cell].x, wt * v.x);
+        atomicAdd(&buf[cell].y, wt * v.y);
       }
     }
     __syncwarp();
   }
-  if constexpr (SMEM) {
-    __syncthreads();
-    for (int c = threadIdx.x; c < ncell; c += SP_THREADS) {
-      cplx<T> v = buf[c];
-      if (v.x == T(0) && v.y == T(0)) continue;
-      global_add<T>(grid + cell_index<NDIM>(c, S, mS, fastwrap, b0, g), v.x, v.y);
-    }
+  __syncthreads();
+  for (int c = threadIdx.x; c < S; c += SP_THREADS) {
+    const cplx<T> v = buf[c];
+    if (v.x == T(0) && v.y == T(0)) continue;
+    global_add<T>(grid + wrapi(b0[0] + c, int(g.nover[0])), v.x, v.y);
   }
-}
-
-// four CTAs per SM for single-precision values at float64 coordinates (whose
-// exact fold takes many registers)
-template <typename T, typename Tc> constexpr int spread_min_ctas() {
-  return (sizeof(T) == 4 && sizeof(Tc) == 8) ? 4 : 1;
-}
-
-template <typename T, typename Tc, int NDIM, int W>
-__global__ void __launch_bounds__(SP_THREADS, spread_min_ctas<T, Tc>())
-    k_spread(PointsDesc pts, const Chunk *__restrict__ chunks, const uint32_t *nchunks, Geometry g,
-             KernelPoly<T> kp, const cplx<T> *__restrict__ values, int64_t vs, int64_t vtrans,
-             cplx<T> *__restrict__ grid, int64_t gtrans) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  if (nchunks && blockIdx.x >= *nchunks) return;
-  spread_chunk<T, Tc, NDIM, W>(pts, chunks[blockIdx.x], g, kp,
-                               values + int64_t(blockIdx.y) * vtrans, vs,
-                               grid + int64_t(blockIdx.y) * gtrans, smraw);
 }
 
 // One chunk of one transform (the body of k_interp; also used by the
@@ -289,7 +239,7 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
                                              unsigned char *smraw,
                                              const CUtensorMap *tmap = nullptr, int tpitch = 0,
                                              uint64_t *tbar = nullptr, int *err = nullptr) {
-  constexpr bool SMEM = BufferLayout<T>::smem(NDIM);
+  static_assert(BufferLayout<T>::smem(NDIM), "the tile is staged in shared memory");
   const int S = (1 << g.log2tile) + W;
   int ncell = S;
   if (NDIM >= 2) ncell *= S;
@@ -301,7 +251,7 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
   int pitch = S, sh = 0;
   bool tma = false;
   size_t tile_bytes = size_t(ncell) * sizeof(cplx<T>);
-  if constexpr (NDIM == 2 && SMEM) {
+  if constexpr (NDIM == 2) {
     if (tmap) {
       tile_bytes = size_t(tpitch) * size_t(S) * sizeof(cplx<T>);
       const int v0 = b0[1] & ~1;   // even start column (also for negative origins)
@@ -331,7 +281,7 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
       }
     }
   }
-  if (SMEM && !tma) {
+  if (!tma) {
     // tile + halo, LB loads in flight per thread before their stores
     // cell -> grid index by multiply-high division and division-free wrap
     constexpr int LB = 8;
@@ -353,99 +303,8 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
     }
     __syncthreads();
   }
-  auto point = [&](uint32_t i) {
-    Tc x[NDIM];
-    uint32_t j = load_point<Tc, NDIM>(pts, i, x);
-    T w[NDIM][W];
-    int o[NDIM];
-#pragma unroll
-    for (int d = 0; d < NDIM; ++d) {
-      int i0;
-      double frac;
-      fold<Tc>(x[d], g.coordfct[d], int(g.nover[d]), g.shift[d], g.maxi0[d], i0, frac);
-      kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w[d]);
-      o[d] = i0 - b0[d];
-    }
-    T ar = 0, ai = 0;
-    if constexpr (NDIM == 1) {
-#pragma unroll
-      for (int a = 0; a < W; ++a) {
-        cplx<T> gv = buf[o[0] + a];
-        ar += w[0][a] * gv.x;
-        ai += w[0][a] * gv.y;
-      }
-    } else if constexpr (NDIM == 2) {
-#pragma unroll
-      for (int a = 0; a < W; ++a) {
-        const cplx<T> *row = buf + (o[0] + a) * S + o[1];
-        T rr = 0, ri = 0;
-#pragma unroll
-        for (int b = 0; b < W; ++b) {
-          cplx<T> gv = row[b];
-          rr += w[1][b] * gv.x;
-          ri += w[1][b] * gv.y;
-        }
-        ar += w[0][a] * rr;
-        ai += w[0][a] * ri;
-      }
-    } else {
-      if constexpr (SMEM) {
-#pragma unroll 1
-        for (int a = 0; a < W; ++a) {
-          T pr = 0, pi = 0;
-#pragma unroll
-          for (int b = 0; b < W; ++b) {
-            const cplx<T> *row = buf + ((o[0] + a) * S + (o[1] + b)) * S + o[2];
-            T rr = 0, ri = 0;
-#pragma unroll
-            for (int e = 0; e < W; ++e) {
-              cplx<T> gv = row[e];
-              rr += w[2][e] * gv.x;
-              ri += w[2][e] * gv.y;
-            }
-            pr += w[1][b] * rr;
-            pi += w[1][b] * ri;
-          }
-          ar += w[0][a] * pr;
-          ai += w[0][a] * pi;
-        }
-      } else {
-        const int nu = int(g.nover[0]), nv = int(g.nover[1]), nw = int(g.nover[2]);
-        // indices stay in [-n, 2n) where every axis is at least 2S long
-        const bool fw = nu >= 2 * S && nv >= 2 * S && nw >= 2 * S;
-        auto wr = [fw](int i, int n) { return fw ? wrap1(i, n) : wrapi(i, n); };
-        int iw[W];
-#pragma unroll
-        for (int e = 0; e < W; ++e) iw[e] = wr(b0[2] + o[2] + e, nw);
-#pragma unroll 1
-        for (int a = 0; a < W; ++a) {
-          int iu = wr(b0[0] + o[0] + a, nu);
-          T pr = 0, pi = 0;
-#pragma unroll
-          for (int b = 0; b < W; ++b) {
-            int iv = wr(b0[1] + o[1] + b, nv);
-            const cplx<T> *row = grid + (int64_t(iu) * nv + iv) * nw;
-            T rr = 0, ri = 0;
-#pragma unroll
-            for (int e = 0; e < W; ++e) {
-              cplx<T> gv = __ldg(row + iw[e]);
-              rr += w[2][e] * gv.x;
-              ri += w[2][e] * gv.y;
-            }
-            pr += w[1][b] * rr;
-            pi += w[1][b] * ri;
-          }
-          ar += w[0][a] * pr;
-          ai += w[0][a] * pi;
-        }
-      }
-    }
-    out[int64_t(j) * os] = mkc<T>(ar, ai);
-  };
   const uint32_t end = ch.start + ch.count;
-  if constexpr (!SMEM) {
-    for (uint32_t i = ch.start + threadIdx.x; i < end; i += SP_THREADS) point(i);
-  } else {
+  {
     // Bank-balanced order.  At a given step of the footprint loop all lanes of
     // a warp read at the same offset from their point's first cell, so the
     // bank conflicts of that read depend only on the first cells' banks.  Each
@@ -532,6 +391,10 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
       }
       const int pl = (lane % NSLOT) * (32 / NSLOT) + lane / NSLOT;
       for (int r = warp; r < q; r += SP_WARPS) {
+        // the kernel coefficients are read again for every point: hoisted out of
+        // the loop (the multi-instance kernel has them in shared memory) they
+        // spill, 2184 against 644 bytes, 8 % of a batched pass
+        asm volatile("" ::: "memory");
         if (pl * q + r >= nb) continue;
         const int w = r * 32 + pl;
         const uint32_t j = r_j[w];
@@ -611,16 +474,11 @@ __global__ void __launch_bounds__(SP_THREADS, interp_min_ctas<T, NDIM>())
                                tpitch > 0 ? &tmap : nullptr, tpitch, &tbar, err);
 }
 
-template <typename T, int NDIM, int W>
-size_t spread_smem_bytes(const Geometry &g) {
-  int S = (1 << g.log2tile) + W;
-  size_t ncell = size_t(S);
-  for (int d = 1; d < NDIM; ++d) ncell *= size_t(S);
-  size_t buf = BufferLayout<T>::smem(NDIM) ? ncell * sizeof(cplx<T>) : 0;
-  constexpr int WS = stage_stride<NDIM, W>();
-  size_t wbytes = (size_t(SP_WARPS) * 32 * WS * sizeof(T) + 15) / 16 * 16;
-  size_t stage = wbytes + size_t(SP_WARPS) * 32 * (sizeof(cplx<T>) + NDIM * sizeof(int));
-  return buf + stage;
+template <typename T, int W> size_t spread_smem_bytes(const Geometry &g) {
+  const size_t buf = size_t((1 << g.log2tile) + W) * sizeof(cplx<T>);
+  constexpr int WS = stage_stride<W>();
+  const size_t wbytes = (size_t(SP_WARPS) * 32 * WS * sizeof(T) + 15) / 16 * 16;
+  return buf + wbytes + size_t(SP_WARPS) * 32 * (sizeof(cplx<T>) + sizeof(int));
 }
 
 // tpitch > 0: the staged 2D tile has that row pitch (TMA staging)
@@ -640,16 +498,17 @@ size_t interp_smem_bytes(const Geometry &g, int tpitch = 0) {
 bool encode_tile_map(CUtensorMap *map, const void *grid, bool f64, int64_t n0, int64_t n1,
                      int tpitch, int S);
 
-template <typename T, typename Tc, int NDIM, int W>
+template <typename T, typename Tc, int W>
 void spread_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
               const KernelPoly<T> &kp, const void *values, int64_t vs, int64_t vtrans,
               void *grid, int64_t gtrans, int ntrans, cudaStream_t st) {
-  size_t sm = spread_smem_bytes<T, NDIM, W>(g);
-  auto kern = k_spread<T, Tc, NDIM, W>;
+  size_t sm = spread_smem_bytes<T, W>(g);
+  auto kern = k_spread<T, Tc, W>;
   DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   dim3 grd(cl.nchunks, ntrans);
   kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
-                                    static_cast<const cplx<T> *>(values), vs, vtrans, static_cast<cplx<T> *>(grid), gtrans);
+                                    static_cast<const cplx<T> *>(values), vs, vtrans,
+                                    static_cast<cplx<T> *>(grid), gtrans);
   DN_LAUNCHED();
 }
 
@@ -660,7 +519,7 @@ void interp_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
   CUtensorMap map;
   memset(&map, 0, sizeof(map));
   int tpitch = 0;
-  if constexpr (NDIM == 2 && BufferLayout<T>::smem(NDIM)) {
+  if constexpr (NDIM == 2) {
     const int S = (1 << g.log2tile) + W;
     const int tp = tma_tile_pitch(S, g.nsafe);
     if (err && ntrans == 1 &&
@@ -683,12 +542,12 @@ void interp_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
 #define DN_FOR_W_DOUBLE(M) \
   M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(11) M(12) M(13) M(14) M(15) M(16)
 
-template <typename T, typename Tc, int NDIM>
+template <typename T, typename Tc>
 void spread_dispatch(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
                      const KernelPoly<T> &kp, const void *values, int64_t vs, int64_t vtrans,
                      void *grid, int64_t gtrans, int ntrans, cudaStream_t st) {
 #define DN_CASE(WW) \
-  case WW: spread_w<T, Tc, NDIM, WW>(pts, cl, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st); return;
+  case WW: spread_w<T, Tc, WW>(pts, cl, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st); return;
   if constexpr (sizeof(T) == 4) {
     switch (g.W) { DN_FOR_W_FLOAT(DN_CASE) }
   } else {
@@ -728,11 +587,11 @@ void launch_spread_impl(const PointsDesc &pts, const ChunkList &cl, const Geomet
     return;
   }
   if (cl.nchunks == 0 || ntrans == 0) return;
-#define DN_SD(TC, ND) spread_dispatch<T, TC, ND>(pts, cl, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st)
+#define DN_SD(TC) spread_dispatch<T, TC>(pts, cl, g, kp, values, vs, vtrans, grid, gtrans, ntrans, st)
   if (pts.coord_f64) {
-    DN_SD(double, 1);
+    DN_SD(double);
   } else {
-    DN_SD(float, 1);
+    DN_SD(float);
   }
 #undef DN_SD
 }
@@ -746,15 +605,21 @@ void launch_interp_impl(const PointsDesc &pts, const ChunkList &cl, const Geomet
       launch_interp_run(pts, nullptr, pts.npts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
       return;
     }
+    if (g.ndim == 3) {
+      launch_interp_run3(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
+      return;
+    }
   }
   if (cl.nchunks == 0 || ntrans == 0) return;
 #define DN_ID(TC, ND) interp_dispatch<T, TC, ND>(pts, cl, g, kp, grid, gtrans, out, os, otrans, ntrans, st, err)
   if (g.ndim == 1) {
     if (pts.coord_f64) DN_ID(double, 1); else DN_ID(float, 1);
-  } else if (g.ndim == 3) {
-    if (pts.coord_f64) DN_ID(double, 3); else DN_ID(float, 3);
   } else if constexpr (sizeof(T) == 4) {
-    if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
+    if (g.ndim == 3) {
+      if (pts.coord_f64) DN_ID(double, 3); else DN_ID(float, 3);
+    } else {
+      if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
+    }
   }
 #undef DN_ID
 }
