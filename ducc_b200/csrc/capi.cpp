@@ -681,7 +681,9 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
 
 // do type 1 / type 2 of this setup work from a chunk list?
 static bool spread_needs_chunks(const Setup &s) { return s.g.ndim == 1 || s.qbits; }
-static bool interp_needs_chunks(const Setup &s) { return s.g.ndim == 1 || !s.calc_f64; }
+static bool interp_needs_chunks(const Setup &s) {
+  return s.g.ndim == 1 || (s.g.ndim == 2 && !s.calc_f64);
+}
 
 static size_t grid_cells(const Geometry &g) {
   size_t c = 1;
@@ -1117,7 +1119,7 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   DN_REQUIRE(out.dtype == uni.dtype, ST_BADARG, "out must have the dtype of grid");
   bool f64 = uni.dtype == DNUFFT_C128;
   Setup s = make_setup(ndim, uni.shape, uint64_t(coord.shape[0]), eps, false, f64,
-                       coord.dtype == DNUFFT_F64, o, f64 && ndim >= 2);
+                       coord.dtype == DNUFFT_F64, o, ndim == 3 || (f64 && ndim == 2));
   StageTimer tm(o.verbosity > 0, st);
   if (o.verbosity > 0) report_sizes(s, false);
   if (s.npoints == 0) return;

@@ -1,5 +1,5 @@
-// Double-precision 3D interpolation (type 2) with the window of a bin in
-// registers: the transpose of spread_run3.cuh.
+// 3D interpolation (type 2) with the window of a bin in registers: the
+// transpose of spread_run3.cuh.  Double precision first, single below.
 //
 // A CTA takes consecutive sorted points and has one warp per plane of the window
 // of their bin (8^3 cells, 4^3 for W > 12).  A batch of points is staged in
@@ -210,6 +210,251 @@ void interp_run3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<do
   dim3 grd((pts.npts + ppb - 1) / ppb, ntrans);
   kern<<<grd, R::THREADS, R::SMEM, st>>>(pts, ppb, g, kp, static_cast<const double2 *>(grid),
                                          gtrans, static_cast<double2 *>(out), os, otrans);
+  DN_LAUNCHED();
+}
+
+// ---------------------------------------------------------------- single precision
+// The same with FP32 multiply-adds (packed in pairs), in the operand layout of
+// Run3Window<float>: 4 warps, warp r has planes r, r + 4, r + 8, r + 12 of the
+// window, a lane 4 rows x 2 cells of each.  A point uses two neighbouring planes
+// of a warp (loops for the three pairs, as the spreader); the lanes' parts of
+// four points are added over the warp together.
+//
+// One thread per point reading W^3 cells from a staged tile took 134 SM cycles at
+// W = 8 (32 of shared-memory bandwidth; 16 warps per SM); this takes 46 issue
+// cycles.
+template <int W> struct Interp3fShape {
+  static constexpr int PLANES = 16, ROWS = 16, CELLS = 16;
+  static constexpr int THREADS = 128, BATCH = 128;
+  static constexpr int ST = PLANES + ROWS + CELLS + 4;   // an odd number of 16-byte words
+  static constexpr size_t SMEM = size_t(BATCH) * (ST * 4 + 4 * sizeof(float2) + sizeof(int4));
+};
+
+template <int W> struct Interp3fWindow {
+  using R = Interp3fShape<W>;
+  using L = RunWindow<float, W>;
+  unsigned long long c[4][2][4];   // [plane][cell][row], (re, im)
+  // sums of points p .. p + 3 (at most e) over planes J0, J0 + 1 to part
+  template <int J0>
+  __device__ __forceinline__ void points(const float *st, float2 *part, int s, int e, int warp,
+                                         int lane) const {
+    const float *pk = st + 4 * warp + J0, *kr = st + R::PLANES + L::row0(lane),
+                *kc = st + R::PLANES + R::ROWS + L::cell0(lane);
+#pragma unroll 1
+    for (int p = s; p < e; p += 4) {
+      float2 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = min(p + q, e - 1) * R::ST;
+        const float4 k = *reinterpret_cast<const float4 *>(kr + o);
+        const unsigned long long kk[4] = {pack2(k.x, k.x), pack2(k.y, k.y), pack2(k.z, k.z),
+                                          pack2(k.w, k.w)};
+        const float w0 = kc[o], w1 = kc[o + 8];
+        const unsigned long long ww[2] = {pack2(w0, w0), pack2(w1, w1)};
+        unsigned long long sum = 0ull;
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          unsigned long long t = 0ull;
+#pragma unroll
+          for (int d = 0; d < 2; ++d) {
+            unsigned long long a;
+            asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(a) : "l"(c[J0 + j][d][0]), "l"(kk[0]));
+#pragma unroll
+            for (int i = 1; i < 4; ++i)
+              asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(c[J0 + j][d][i]), "l"(kk[i]));
+            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(t) : "l"(a), "l"(ww[d]));
+          }
+          const float kj = pk[o + j];
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum) : "l"(t), "l"(pack2(kj, kj)));
+        }
+        v[q] = unpack2(sum);
+      }
+      // lane bits 4 and 3 choose a point of the four, the others are added up
+      const bool b4 = lane & 16, b3 = lane & 8;
+      float2 x, y;
+      x.x = (b4 ? v[2].x : v[0].x) + __shfl_xor_sync(0xffffffffu, b4 ? v[0].x : v[2].x, 16);
+      x.y = (b4 ? v[2].y : v[0].y) + __shfl_xor_sync(0xffffffffu, b4 ? v[0].y : v[2].y, 16);
+      y.x = (b4 ? v[3].x : v[1].x) + __shfl_xor_sync(0xffffffffu, b4 ? v[1].x : v[3].x, 16);
+      y.y = (b4 ? v[3].y : v[1].y) + __shfl_xor_sync(0xffffffffu, b4 ? v[1].y : v[3].y, 16);
+      float2 z;
+      z.x = (b3 ? y.x : x.x) + __shfl_xor_sync(0xffffffffu, b3 ? x.x : y.x, 8);
+      z.y = (b3 ? y.y : x.y) + __shfl_xor_sync(0xffffffffu, b3 ? x.y : y.y, 8);
+#pragma unroll
+      for (int o = 4; o; o >>= 1) {
+        z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
+        z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
+      }
+      const int q = p + 2 * (b4 ? 1 : 0) + (b3 ? 1 : 0);
+      if ((lane & 7) == 0 && q < e) part[warp * R::BATCH + q] = z;
+    }
+  }
+};
+
+template <typename Tc, int W>
+__global__ void __launch_bounds__(Interp3fShape<W>::THREADS, 4)
+    k_interp_run3f(const __grid_constant__ PointsDesc pts, uint32_t ppb,
+                   const __grid_constant__ Geometry g, const __grid_constant__ KernelPoly<float> kp,
+                   const float2 *__restrict__ grid, int64_t gtrans, float2 *__restrict__ out,
+                   int64_t os, int64_t otrans) {
+  using R = Interp3fShape<W>;
+  using L = RunWindow<float, W>;
+  constexpr int B = R::BATCH;
+  extern __shared__ __align__(16) unsigned char smraw_run[];
+  float *st = reinterpret_cast<float *>(smraw_run);
+  int4 *info = reinterpret_cast<int4 *>(st + B * R::ST);   // first-axis cell, bins, output index
+  float2 *part = reinterpret_cast<float2 *>(info + B);     // [warp][point]
+  grid += int64_t(blockIdx.y) * gtrans;
+  out += int64_t(blockIdx.y) * otrans;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n0 = int(g.nover[0]), n1 = int(g.nover[1]), n2 = int(g.nover[2]);
+  const uint32_t first = blockIdx.x * ppb;
+  const uint32_t last = uint32_t(min(uint64_t(pts.npts), uint64_t(first) + ppb));
+  Interp3fWindow<W> win;
+  int cu = -1, cv = -1, cw = -1;
+  bool finite = true;
+  auto load_window = [&]() {
+    const int u0 = cu * 8 - g.nsafe, rv = cv * 8 - g.nsafe + L::row0(lane),
+              wa = cw * 8 - g.nsafe + L::cell0(lane);
+    const int ca = wrap2(wa, n2), cb = wrap2(wa + 8, n2);
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 *pl = grid + int64_t(wrap2(u0 + warp + 4 * j, n0)) * n1 * n2;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 *row = pl + int64_t(wrap2(rv + i, n1)) * n2;
+        const float2 a = __ldg(row + ca), b = __ldg(row + cb);
+        win.c[j][0][i] = pack2(a.x, a.y);
+        win.c[j][1][i] = pack2(b.x, b.y);
+        ok = ok && isfinite(a.x) && isfinite(a.y) && isfinite(b.x) && isfinite(b.y);
+      }
+    }
+    finite = __all_sync(0xffffffffu, ok);
+  };
+  for (uint32_t base = first; base < last; base += B) {
+    const int np = int(min(uint32_t(B), last - base));
+    {
+      float4 *z4 = reinterpret_cast<float4 *>(st);
+      const int nz = np * (R::ST / 4);
+      for (int i = tid; i < nz; i += R::THREADS) z4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    for (int it = tid; it < 3 * B; it += R::THREADS) {
+      const int ax = it / B, q = it - ax * B;
+      if (q >= np) continue;
+      const uint32_t i = base + uint32_t(q), j = pts.perm[i];
+      const Tc *c = static_cast<const Tc *>(pts.coord);
+      const Tc x = pts.sorted ? c[uint64_t(i) * 3 + ax]
+                              : c[int64_t(j) * pts.cs0 + int64_t(ax) * pts.cs1];
+      int i0;
+      double frac;
+      float w[W];
+      fold<Tc>(x, ax == 0 ? g.coordfct[0] : (ax == 1 ? g.coordfct[1] : g.coordfct[2]),
+               ax == 0 ? n0 : (ax == 1 ? n1 : n2),
+               ax == 0 ? g.shift[0] : (ax == 1 ? g.shift[1] : g.shift[2]),
+               ax == 0 ? g.maxi0[0] : (ax == 1 ? g.maxi0[1] : g.maxi0[2]), i0, frac);
+      kernel_weights<float, W>(kp, float(double(W - 1) - 2.0 * frac), w);
+      const int t = i0 + g.nsafe, o = t & 7;
+      int *inf = reinterpret_cast<int *>(info + q);
+      inf[ax] = ax == 0 ? t : t >> 3;
+      float *sp = st + q * R::ST;
+      if (ax == 0) {
+        inf[3] = int(j);
+#pragma unroll
+        for (int a = 0; a < W; ++a) sp[Run3Window<float, W>::plane_slot(o + a)] = w[a];
+      } else {
+        sp += (ax == 1 ? R::PLANES : R::PLANES + R::ROWS) + o;
+#pragma unroll
+        for (int a = 0; a < W; ++a) sp[a] = w[a];
+      }
+    }
+    __syncthreads();
+    for (int s0 = 0; s0 < np; s0 += 32) {
+      const int p0 = s0 + lane, ns = min(32, np - s0);
+      const int4 b = info[min(p0, np - 1)];
+      const int j0 = Run3Window<float, W>::first_plane(b.x & 7, warp);
+      int pu = __shfl_up_sync(0xffffffffu, b.x >> 3, 1), pv = __shfl_up_sync(0xffffffffu, b.y, 1),
+          pw = __shfl_up_sync(0xffffffffu, b.z, 1);
+      const int pj = __shfl_up_sync(0xffffffffu, j0, 1);
+      if (lane == 0) {
+        pu = cu;
+        pv = cv;
+        pw = cw;
+      }
+      const unsigned bins = __ballot_sync(
+          0xffffffffu, p0 < np && ((b.x >> 3) != pu || b.y != pv || b.z != pw));
+      unsigned rest = bins | __ballot_sync(0xffffffffu, p0 < np && lane > 0 && j0 != pj);
+      rest &= ~1u;
+      for (int s = 0; s < ns;) {
+        if ((bins >> s) & 1u) {
+          cu = __shfl_sync(0xffffffffu, b.x, s) >> 3;
+          cv = __shfl_sync(0xffffffffu, b.y, s);
+          cw = __shfl_sync(0xffffffffu, b.z, s);
+          load_window();
+        }
+        const int e = rest ? __ffs(rest) - 1 : ns;
+        rest &= rest - 1;
+        const int js = __shfl_sync(0xffffffffu, j0, s);
+        if (!finite) {
+          // the footprints' cells only
+          for (int p = s0 + s; p < s0 + e; ++p) {
+            const float *f = st + p * R::ST;
+            float sx = 0.f, sy = 0.f;
+            for (int k = lane; k < 4 * 256; k += 32) {
+              const int j = k >> 8, r = (k >> 4) & 15, c = k & 15;
+              const float wt = f[4 * warp + j] * f[R::PLANES + r] * f[R::PLANES + R::ROWS + c];
+              if (wt == 0.f) continue;
+              const float2 gv = __ldg(
+                  grid + (int64_t(wrap2(cu * 8 - g.nsafe + warp + 4 * j, n0)) * n1 +
+                          wrap2(cv * 8 - g.nsafe + r, n1)) * n2 + wrap2(cw * 8 - g.nsafe + c, n2));
+              sx += wt * gv.x;
+              sy += wt * gv.y;
+            }
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+              sx += __shfl_xor_sync(0xffffffffu, sx, o);
+              sy += __shfl_xor_sync(0xffffffffu, sy, o);
+            }
+            if (lane == 0) part[warp * B + p] = make_float2(sx, sy);
+          }
+        } else if (js == 0) {
+          win.template points<0>(st, part, s0 + s, s0 + e, warp, lane);
+        } else if (js == 1) {
+          win.template points<1>(st, part, s0 + s, s0 + e, warp, lane);
+        } else {
+          win.template points<2>(st, part, s0 + s, s0 + e, warp, lane);
+        }
+        s = e;
+      }
+    }
+    __syncthreads();
+    for (int q = tid; q < np; q += R::THREADS) {
+      float2 v = part[q];
+#pragma unroll
+      for (int k = 1; k < 4; ++k) {
+        const float2 a = part[k * B + q];
+        v.x += a.x;
+        v.y += a.y;
+      }
+      out[int64_t(uint32_t(info[q].w)) * os] = v;
+    }
+  }
+}
+
+template <typename Tc, int W>
+void interp_run3f_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<float> &kp,
+                    const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
+                    int ntrans, cudaStream_t st) {
+  using R = Interp3fShape<W>;
+  auto kern = k_interp_run3f<Tc, W>;
+  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(R::SMEM)));
+  const uint64_t per = uint64_t(pts.npts) * uint64_t(ntrans) / (148 * 8);
+  const uint32_t ppb =
+      per >= R::BATCH ? R::BATCH * uint32_t(std::min<uint64_t>(8, per / R::BATCH))
+                      : std::max<uint32_t>(16, uint32_t(per) & ~15u);
+  dim3 grd((pts.npts + ppb - 1) / ppb, ntrans);
+  kern<<<grd, R::THREADS, R::SMEM, st>>>(pts, ppb, g, kp, static_cast<const float2 *>(grid),
+                                         gtrans, static_cast<float2 *>(out), os, otrans);
   DN_LAUNCHED();
 }
 

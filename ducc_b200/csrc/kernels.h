@@ -128,7 +128,10 @@ void launch_interp_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts
                        int64_t gtrans, void *out, int64_t os, int64_t otrans, int ntrans,
                        cudaStream_t st);
 
-// 3D double precision (launch_interp goes here; no chunk list)
+// 3D (launch_interp goes here; no chunk list)
+void launch_interp_run3(const PointsDesc &pts, const Geometry &g, const KernelPoly<float> &kp,
+                        const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
+                        int ntrans, cudaStream_t st);
 void launch_interp_run3(const PointsDesc &pts, const Geometry &g, const KernelPoly<double> &kp,
                         const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
                         int ntrans, cudaStream_t st);

@@ -1,6 +1,6 @@
 // Plain spreading (type 1, 1D; 2D and 3D: spread_run.cuh, spread_run3.cuh) and
-// interpolation (type 2, 1D and single precision; double in 2D and 3D:
-// interp_run.cuh, interp_run3.cuh) kernels.
+// interpolation (type 2, 1D and 2D single precision; 2D double: interp_run.cuh,
+// 3D: interp_run3.cuh) kernels.
 //
 // One CTA per chunk of tile-sorted points (at most CHUNK points of one tile).
 // Spreading: every warp takes 32 points at a time, each lane folds its point
@@ -239,11 +239,9 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
                                              unsigned char *smraw,
                                              const CUtensorMap *tmap = nullptr, int tpitch = 0,
                                              uint64_t *tbar = nullptr, int *err = nullptr) {
-  static_assert(BufferLayout<T>::smem(NDIM), "the tile is staged in shared memory");
+  static_assert(NDIM <= 2, "3D: interp_run3.cuh");
   const int S = (1 << g.log2tile) + W;
-  int ncell = S;
-  if (NDIM >= 2) ncell *= S;
-  if (NDIM >= 3) ncell *= S;
+  const int ncell = NDIM == 2 ? S * S : S;
   int b0[NDIM];
   tile_origin<NDIM>(ch.tile, g, b0);
   cplx<T> *buf = reinterpret_cast<cplx<T> *>(smraw);
@@ -410,7 +408,7 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
             ar += wt[0][a] * gv.x;
             ai += wt[0][a] * gv.y;
           }
-        } else if constexpr (NDIM == 2) {
+        } else {
 #pragma unroll
           for (int a = 0; a < W; ++a) {
             const cplx<T> *row = p0 + a * pitch;
@@ -423,26 +421,6 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
             }
             ar += wt[0][a] * rr;
             ai += wt[0][a] * ri;
-          }
-        } else {
-#pragma unroll 1
-          for (int a = 0; a < W; ++a) {
-            T pr = 0, pi = 0;
-#pragma unroll
-            for (int b = 0; b < W; ++b) {
-              const cplx<T> *row = p0 + (a * S + b) * S;
-              T rr = 0, ri = 0;
-#pragma unroll
-              for (int e = 0; e < W; ++e) {
-                cplx<T> gv = row[e];
-                rr += wt[2][e] * gv.x;
-                ri += wt[2][e] * gv.y;
-              }
-              pr += wt[1][b] * rr;
-              pi += wt[1][b] * ri;
-            }
-            ar += wt[0][a] * pr;
-            ai += wt[0][a] * pi;
           }
         }
         out[int64_t(j) * os] = mkc<T>(ar, ai);
@@ -600,13 +578,13 @@ template <typename T>
 void launch_interp_impl(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
                         const KernelPoly<T> &kp, const void *grid, int64_t gtrans, void *out,
                         int64_t os, int64_t otrans, int ntrans, cudaStream_t st, int *err) {
+  if (g.ndim == 3) {
+    launch_interp_run3(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
+    return;
+  }
   if constexpr (sizeof(T) == 8) {
     if (g.ndim == 2) {
       launch_interp_run(pts, nullptr, pts.npts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
-      return;
-    }
-    if (g.ndim == 3) {
-      launch_interp_run3(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
       return;
     }
   }
@@ -615,11 +593,7 @@ void launch_interp_impl(const PointsDesc &pts, const ChunkList &cl, const Geomet
   if (g.ndim == 1) {
     if (pts.coord_f64) DN_ID(double, 1); else DN_ID(float, 1);
   } else if constexpr (sizeof(T) == 4) {
-    if (g.ndim == 3) {
-      if (pts.coord_f64) DN_ID(double, 3); else DN_ID(float, 3);
-    } else {
-      if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
-    }
+    if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
   }
 #undef DN_ID
 }

@@ -65,9 +65,11 @@ template <int W> struct Run3Window<float, W> {
   }
   // slot of plane weight i (of 16): the four planes of a warp side by side
   static __device__ __forceinline__ int plane_slot(int i) { return (i & 3) * 4 + (i >> 2); }
-  // points [s, e), whose footprints start at plane ou of the window
+  // the warp's first plane at or after plane ou of the window
+  static __device__ __forceinline__ int first_plane(int ou, int warp) { return (ou - warp + 3) >> 2; }
+  // points [s, e), whose footprints start at planes of the same first_plane
   __device__ __forceinline__ void add(const float *st, int s, int e, int ou, int warp, int lane) {
-    const int j0 = (ou - warp + 3) >> 2;   // the warp's first plane at or after ou
+    const int j0 = first_plane(ou, warp);
     if (j0 == 0) add_pair<0>(st, s, e, warp, lane);
     else if (j0 == 1) add_pair<1>(st, s, e, warp, lane);
     else add_pair<2>(st, s, e, warp, lane);
@@ -282,8 +284,8 @@ __global__ void __launch_bounds__(Run3Shape<T, W>::THREADS)
       __syncthreads();
     }
     for (int s0 = 0; s0 < np; s0 += 32) {
-      // points whose bin, or (sub-runs, float) plane in it, differs from the one
-      // before
+      // points whose bin, or (float) first plane of this warp in it, differs from
+      // the one before
       const int p = s0 + lane, ns = min(32, np - s0);
       const int4 b = info[min(p, np - 1)];
       int pu = __shfl_up_sync(0xffffffffu, b.x, 1), pv = __shfl_up_sync(0xffffffffu, b.y, 1),
@@ -296,7 +298,11 @@ __global__ void __launch_bounds__(Run3Shape<T, W>::THREADS)
       const unsigned bins = __ballot_sync(
           0xffffffffu, p < np && ((b.x >> R::LB) != (pu >> R::LB) || b.y != pv || b.z != pw));
       unsigned rest = bins;
-      if (R::F32) rest |= __ballot_sync(0xffffffffu, p < np && lane > 0 && b.x != pu);
+      if constexpr (R::F32) {
+        const int j0 = Run3Window<T, W>::first_plane(b.x & (R::BIN - 1), warp);
+        const int pj = __shfl_up_sync(0xffffffffu, j0, 1);
+        rest |= __ballot_sync(0xffffffffu, p < np && lane > 0 && j0 != pj);
+      }
       rest &= ~1u;
       for (int s = 0; s < ns;) {
         if ((bins >> s) & 1u) {

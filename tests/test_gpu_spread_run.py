@@ -113,3 +113,24 @@ def test_nonfinite_value_stays_in_its_footprint(single, shape, nover):
     vals[77] = 0
     ref = O.spread(p, coord, vals)
     assert O.l2error(got[~bad], ref[~bad]) < (3e-6 if single else 1e-10)
+
+
+@pytest.mark.parametrize("single,shape,nover", [(False, (50, 60), (110, 126)),
+                                                (False, (15, 20, 9), (36, 48, 20)),
+                                                (True, (15, 20, 9), (36, 48, 20))])
+def test_nonfinite_cell_reaches_its_points_only(single, shape, nover):
+    import torch
+    W = 6
+    p, k, nov, coord, vals = _case(W, single, shape, nover, 400, "uniform")
+    plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=shape,
+                      epsilon=1e-3, force_kernel=k, force_nover=nov)
+    rng = np.random.default_rng(6)
+    grid = (rng.standard_normal(nov) + 1j * rng.standard_normal(nov)).astype(vals.dtype)
+    ref = O.interpolate(p, grid, coord)
+    cell = tuple(n // 3 for n in nov)
+    grid[cell] = np.nan
+    got = plan.interp(grid=torch.from_numpy(grid).cuda()).cpu().numpy()
+    i0, _ = O.getpix(p, coord)
+    hit = np.all((np.array(cell) - i0) % np.array(nov) < W, axis=1)
+    assert 0 < hit.sum() < 400 and np.array_equal(~np.isfinite(got), hit)
+    assert O.l2error(got[~hit], ref[~hit]) < (3e-6 if single else 1e-10)
