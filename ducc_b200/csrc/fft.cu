@@ -336,6 +336,7 @@ struct StageInfo {
   int tstep[24];
   uint32_t mul[24];   // ceil(2^32 / Ns)
   PencilPlan pen;     // pencil passes of the line kernels (pen.L == 0: the stages above)
+  int full_tw;        // pencil passes with all n twiddles in shared memory
 };
 
 // cos / sin of 2*pi*k/R, k < R, for the odd radices 3, 5, 7, 11 (rows 0..3)
@@ -463,8 +464,9 @@ __device__ __forceinline__ void fft_lines_block(cplx<T> *__restrict__ grid, cons
   cplx<T> *s = reinterpret_cast<cplx<T> *>(smraw);
   cplx<T> *s2 = s + (n << lnl);
   cplx<T> *twl = s2 + (n << lnl);
-  cplx<T> *twh = twl + 64;
-  int64_t *lbase = reinterpret_cast<int64_t *>(twh + nh);
+  const int ntw = si.full_tw ? n : 64;
+  cplx<T> *twh = si.full_tw ? nullptr : twl + 64;
+  int64_t *lbase = reinterpret_cast<int64_t *>(twl + (si.full_tw ? (n + 1) & ~1 : 64 + nh));
   int64_t *luoff = lbase + nl;
   double *lfac = reinterpret_cast<double *>(luoff + nl);
   __shared__ int stR[24], stNs[24], stT[24];
@@ -481,8 +483,9 @@ __device__ __forceinline__ void fft_lines_block(cplx<T> *__restrict__ grid, cons
   const int nloc = min(nl, ls.nlines - L0);
   const int N = sel3(u.N, ls.ax);
   const int lo = (N + 1) / 2, hi0 = n - N / 2;
-  for (int i = threadIdx.x; i < 64; i += blockDim.x) twl[i] = (i < n) ? tw[i] : mkc<T>(T(1), T(0));
-  for (int i = threadIdx.x; i < nh; i += blockDim.x) twh[i] = (64 * i < n) ? tw[64 * i] : mkc<T>(T(1), T(0));
+  for (int i = threadIdx.x; i < ntw; i += blockDim.x) twl[i] = (i < n) ? tw[i] : mkc<T>(T(1), T(0));
+  if (!si.full_tw)
+    for (int i = threadIdx.x; i < nh; i += blockDim.x) twh[i] = (64 * i < n) ? tw[64 * i] : mkc<T>(T(1), T(0));
   for (int l = threadIdx.x; l < nl; l += blockDim.x) {
     int ia = 0, ib = 0;
     lbase[l] = (l < nloc) ? line_base(ls, u.N, u.n, L0 + l, ia, ib) : 0;
@@ -639,6 +642,17 @@ static StageInfo make_stages(const FFTAxisPlan &p, int pen_maxr) {
   return si;
 }
 
+// All twiddles in shared memory (no product of two table entries per twiddle)
+// for pencil passes of at least four lines that share them; sm: the launch's
+// shared memory, replaced
+static void full_twiddles(StageInfo &si, int n, int lnl, size_t esz, size_t &sm) {
+  if (si.pen.L == 0 || lnl < 2) return;
+  const size_t smf = size_t(2 * (n << lnl) + ((n + 1) & ~1)) * esz + size_t(1 << lnl) * 24;
+  if (smf > 100 * 1024) return;
+  si.full_tw = 1;
+  sm = smf;
+}
+
 // v2 launch if the line fits its register / shared-memory budget; false otherwise
 template <typename T>
 static bool run_lines2(cplx<T> *grid, LineSpec ls, const FFTAxisPlan &p, const UniSpec &u,
@@ -663,6 +677,7 @@ static bool run_lines2(cplx<T> *grid, LineSpec ls, const FFTAxisPlan &p, const U
   if (sm > maxsm) return false;
   ls.nl = lnl;
   StageInfo si = make_stages(p, lines_maxr<T>());
+  full_twiddles(si, n, lnl, sizeof(cplx<T>), sm);
   DN_CUDA(cudaFuncSetAttribute(k_fft_lines2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   unsigned nb = unsigned((ls.nlines + (1 << lnl) - 1) >> lnl);
   k_fft_lines2<T><<<nb, nt, sm, st>>>(grid, ls, si, static_cast<const cplx<T> *>(p.tw), u, fwd);
@@ -1533,6 +1548,8 @@ void *fft_batch_create(const std::vector<FFTBatchInst> &insts, cudaStream_t st) 
         DN_REQUIRE(lines2_config(ls.n, ls.es, ls.nlines, sizeof(cplx<T>), maxnt, lnl, nt, sm),
                    ST_UNSUPPORTED, "batched transforms: oversampled grid too large");
         ls.nl = lnl;
+        StageInfo si = make_stages(ax, lines_maxr<T>());
+        full_twiddles(si, ls.n, lnl, sizeof(cplx<T>), sm);
         bp.nt = std::max(bp.nt, nt);
         bp.sm = std::max(bp.sm, sm);
         const uint32_t blocks = uint32_t((ls.nlines + (1 << lnl) - 1) >> lnl);
@@ -1540,7 +1557,7 @@ void *fft_batch_create(const std::vector<FFTBatchInst> &insts, cudaStream_t st) 
           FFTJob jb;
           std::memset(&jb, 0, sizeof(jb));
           jb.ls = ls;
-          jb.si = make_stages(ax, lines_maxr<T>());
+          jb.si = si;
           const int64_t zero[3] = {0, 0, 0};
           jb.u = mk_uni(nullptr, zero, g, in.corfac, in.fft_order);
           jb.tw = ax.tw;
