@@ -779,7 +779,6 @@ template <typename T> constexpr int rows_maxr() { return sizeof(T) == 4 ? ROWS_M
 template <typename T> constexpr int cols_maxr() { return sizeof(T) == 4 ? COLS_MAXR_F : COLS_MAXR_D; }
 // column CTAs per SM the register allocation must allow (64 / 80 registers)
 template <typename T> constexpr int cols_min_ctas() { return sizeof(T) == 4 ? 4 : 3; }
-template <typename T> constexpr int rows_threads() { return 512; }
 
 // One row = line of n contiguous elements at grid + row*rs.  Ranges: the whole
 // line, or the kept ranges [0, lo) and [hi0, n) (zeros in between on input).
@@ -787,8 +786,12 @@ template <typename T> constexpr int rows_threads() { return 512; }
 // arrives by TMA bulk copy into the other; the result is written back by bulk
 // stores from the current buffer, which becomes the prefetch target of the
 // row after next once those stores have read it.
-template <typename T, bool FWD>
-__global__ void __launch_bounds__(rows_threads<T>(), 1)
+// NT threads per CTA, 512 / NT CTAs per SM (128 registers a thread): a row's
+// passes give every thread at most one register DFT, n / R of them, so a short
+// row leaves most of 512 threads idle and its barriers exposed; several smaller
+// CTAs per SM transform several rows at once.
+template <typename T, bool FWD, int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
     k_fft_rows(cplx<T> *__restrict__ grid, int64_t rs, int n, int nlines, int lo, int hi0,
                int in_kept, int out_kept, PencilPlan pp, const cplx<T> *__restrict__ tw,
                int full_tw, int *__restrict__ err) {
@@ -1115,19 +1118,32 @@ static bool run_rows_v3(cplx<T> *grid, int n, int nlines, int64_t rs, int Nk, bo
                         bool out_kept, const FFTAxisPlan &p, bool fwd, int *err,
                         cudaStream_t st) {
   if (err == nullptr || nlines <= 0) return false;
+  if (n < 1024) return false;
   const int nh = (n + 63) / 64 + 1;
   const size_t smfull = size_t(3 * n) * sizeof(cplx<T>);
-  const int full_tw = smfull <= 224 * 1024 ? 1 : 0;
-  const size_t sm = full_tw ? smfull : size_t(2 * n + 64 + nh) * sizeof(cplx<T>);
-  if (sm > 224 * 1024 || n < 1024) return false;
+  const size_t smtwo = size_t(2 * n + 64 + nh) * sizeof(cplx<T>);
+  // the smallest CTAs whose shared memory (with all n twiddles, except in the
+  // largest) fits as often as their registers and whose threads hold the last
+  // pass's groups
   PencilPlan pp;
-  if (!make_pencil(n, rows_maxr<T>(), rows_threads<T>(), pp)) return false;
+  const size_t smsm = 224 * 1024;
+  int nt = 0;
+  for (int t : {128, 256})
+    if (!nt && smfull + 1024 <= smsm / size_t(512 / t) && make_pencil(n, rows_maxr<T>(), t, pp)) nt = t;
+  const int full_tw = nt || smfull <= smsm ? 1 : 0;
+  const size_t sm = full_tw ? smfull : smtwo;
+  if (!nt) {
+    if (sm > smsm || !make_pencil(n, rows_maxr<T>(), 512, pp)) return false;
+    nt = 512;
+  }
   const int lo = (Nk + 1) / 2, hi0 = n - Nk / 2;
-  auto kern = fwd ? k_fft_rows<T, true> : k_fft_rows<T, false>;
+  auto kern = nt == 128 ? (fwd ? k_fft_rows<T, true, 128> : k_fft_rows<T, false, 128>)
+              : nt == 256 ? (fwd ? k_fft_rows<T, true, 256> : k_fft_rows<T, false, 256>)
+                          : (fwd ? k_fft_rows<T, true, 512> : k_fft_rows<T, false, 512>);
   DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-  const int nb = std::min(nlines, sm_count_dev());
+  const int nb = std::min(nlines, sm_count_dev() * (512 / nt));
   stage_mark(out_kept ? "FFT rows (k_fft_rows)" : "FFT rows, kept columns in (k_fft_rows)");
-  kern<<<nb, rows_threads<T>(), sm, st>>>(grid, rs, n, nlines, lo, hi0, in_kept ? 1 : 0,
+  kern<<<nb, nt, sm, st>>>(grid, rs, n, nlines, lo, hi0, in_kept ? 1 : 0,
                                           out_kept ? 1 : 0, pp, static_cast<const cplx<T> *>(p.tw),
                                           full_tw, err);
   DN_LAUNCHED();
