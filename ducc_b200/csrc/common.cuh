@@ -308,6 +308,13 @@ __device__ __forceinline__ int wrap2(int i, int n) {
   return i >= n ? i - n : i;
 }
 
+// First footprint cell i0 of a point, counted from -nsafe: 0 .. n + 1 for every
+// finite coordinate; a coordinate that is not finite is kept inside too (its
+// weights are not finite, whatever cells they reach).
+__device__ __forceinline__ int first_cell(int i0, int nsafe, int n) {
+  return min(max(i0 + nsafe, 0), n + 1);
+}
+
 // floor(x / d) for d >= 2 and x * d < 2^32 by a multiply-high with m = ceil(2^32 / d)
 __host__ __device__ __forceinline__ uint32_t fastdiv_magic(uint32_t d) {
   return uint32_t(((uint64_t(1) << 32) + d - 1) / d);
