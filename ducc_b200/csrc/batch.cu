@@ -153,8 +153,7 @@ template <typename T>
 void launch_spread_multi(const SpreadInst<T> *insts, int ninst, uint32_t nctas, uint32_t ppw,
                          int max_ntrans, size_t smem, const BatchArray *vals, cudaStream_t st) {
   if (nctas == 0) return;
-  DN_CUDA(cudaFuncSetAttribute(k_spread_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(smem)));
+  allow_smem(k_spread_multi<T>, smem);
   k_spread_multi<T><<<dim3(nctas, max_ntrans), run_threads<T>(), smem, st>>>(insts, ninst, ppw,
                                                                              vals);
   DN_LAUNCHED();
@@ -164,8 +163,7 @@ template <typename T>
 void launch_interp_multi(const SpreadInst<T> *insts, int ninst, uint32_t nchunks, int max_ntrans,
                          size_t smem, const BatchArray *outs, cudaStream_t st) {
   if (nchunks == 0) return;
-  DN_CUDA(cudaFuncSetAttribute(k_interp_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(smem)));
+  allow_smem(k_interp_multi<T>, smem);
   k_interp_multi<T><<<dim3(nchunks, max_ntrans), SP_THREADS, smem, st>>>(insts, ninst, outs);
   DN_LAUNCHED();
 }

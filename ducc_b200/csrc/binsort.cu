@@ -334,12 +334,7 @@ void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t n, int keybits, v
   uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
   size_t hsm = sizeof(uint32_t) << nbits;
   size_t ssm = size_t(RS_WARPS + 1) * hsm;
-  static bool attr_set = false;
-  if (!attr_set) {
-    DN_CUDA(cudaFuncSetAttribute(k_radix_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (RS_WARPS + 1) * (4 << RADIX_BITS)));
-    attr_set = true;
-  }
+  allow_smem(k_radix_scatter, (RS_WARPS + 1) * (4 << RADIX_BITS));
   for (int pass = 0; pass < passes; ++pass) {
     int shift = pass * nbits;
     int bits = (keybits - shift < nbits) ? keybits - shift : nbits;

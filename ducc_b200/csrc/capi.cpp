@@ -88,6 +88,18 @@ bool &bounded_wait_launched() {
   return launched;
 }
 
+void allow_smem_of(const void *kern, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void *>, size_t> limit;
+  int dev = 0;
+  DN_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  size_t &have = limit[{dev, kern}];
+  if (bytes <= have) return;
+  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  have = bytes;
+}
+
 // Kernels with bounded waits set this word instead of hanging; it is read back
 // after such a kernel (outside stream capture) and turned into ST_TIMEOUT.
 static int *device_error_word() {

@@ -678,7 +678,7 @@ static bool run_lines2(cplx<T> *grid, LineSpec ls, const FFTAxisPlan &p, const U
   ls.nl = lnl;
   StageInfo si = make_stages(p, lines_maxr<T>());
   full_twiddles(si, n, lnl, sizeof(cplx<T>), sm);
-  DN_CUDA(cudaFuncSetAttribute(k_fft_lines2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(k_fft_lines2<T>, sm);
   unsigned nb = unsigned((ls.nlines + (1 << lnl) - 1) >> lnl);
   k_fft_lines2<T><<<nb, nt, sm, st>>>(grid, ls, si, static_cast<const cplx<T> *>(p.tw), u, fwd);
   DN_LAUNCHED();
@@ -1140,7 +1140,7 @@ static bool run_rows_v3(cplx<T> *grid, int n, int nlines, int64_t rs, int Nk, bo
   auto kern = nt == 128 ? (fwd ? k_fft_rows<T, true, 128> : k_fft_rows<T, false, 128>)
               : nt == 256 ? (fwd ? k_fft_rows<T, true, 256> : k_fft_rows<T, false, 256>)
                           : (fwd ? k_fft_rows<T, true, 512> : k_fft_rows<T, false, 512>);
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(kern, sm);
   const int nb = std::min(nlines, sm_count_dev() * (512 / nt));
   stage_mark(out_kept ? "FFT rows (k_fft_rows)" : "FFT rows, kept columns in (k_fft_rows)");
   kern<<<nb, nt, sm, st>>>(grid, rs, n, nlines, lo, hi0, in_kept ? 1 : 0,
@@ -1188,7 +1188,7 @@ static bool run_cols_v3(cplx<T> *grid, cplx<T> *work, int n0, int n1, int N1,
   {
     const size_t sm = size_t(2 * P * C + P) * sizeof(cplx<T>);
     auto kern = fwd ? k_fft_colstep<T, 0, true> : k_fft_colstep<T, 0, false>;
-    DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    allow_smem(kern, sm);
     stage_mark(type1 ? "FFT columns A (k_fft_colstep)"
                      : "FFT columns A, correction + pad (k_fft_colstep)");
     kern<<<unsigned(nblk) * unsigned(Q), 256, sm, st>>>(grid, work, cs, ppP, tw, u);
@@ -1197,7 +1197,7 @@ static bool run_cols_v3(cplx<T> *grid, cplx<T> *work, int n0, int n1, int N1,
   {
     const size_t sm = size_t(2 * Q * C + Q) * sizeof(cplx<T>);
     auto kern = fwd ? k_fft_colstep<T, 1, true> : k_fft_colstep<T, 1, false>;
-    DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    allow_smem(kern, sm);
     stage_mark(type1 ? "FFT columns B, correction + crop (k_fft_colstep)"
                      : "FFT columns B (k_fft_colstep)");
     kern<<<unsigned(nblk) * unsigned(P), 256, sm, st>>>(grid, work, cs, ppQ, tw, u);
@@ -1230,8 +1230,7 @@ static void run_lines(cplx<T> *grid, LineSpec ls, const FFTAxisPlan &p, const Un
   nt = std::max(64, std::min(maxnt, nt));
   while (total > FFT_MAXE * nt) nt += 32;
   size_t sm = size_t(total) * sizeof(cplx<T>);
-  DN_CUDA(cudaFuncSetAttribute(k_fft_lines<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               int(sm)));
+  allow_smem(k_fft_lines<T>, sm);
   unsigned nb = unsigned((ls.nlines + nl - 1) / nl);
   k_fft_lines<T><<<nb, nt, sm, st>>>(grid, ls, p, u, fwd);
   DN_LAUNCHED();
@@ -1600,8 +1599,7 @@ void fft_batch_run(void *h, int type, const BatchArray *uni, bool fwd, cudaStrea
   for (int ps = 0; ps < 2; ++ps) {
     FFTBatchPass &bp = impl->pass[type][ps];
     if (bp.nblocks == 0) continue;
-    DN_CUDA(cudaFuncSetAttribute(k_fft_lines_multi<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(bp.sm)));
+    allow_smem(k_fft_lines_multi<T>, bp.sm);
     k_fft_lines_multi<T><<<bp.nblocks, bp.nt, bp.sm, st>>>(
         static_cast<const FFTJob *>(bp.jobs.p), static_cast<const uint32_t *>(bp.blk0.p),
         bp.njobs, uni, fwd);

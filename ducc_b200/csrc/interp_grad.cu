@@ -142,7 +142,7 @@ static void dcoord_w(const PointsDesc &pts, const ChunkList &cl, const Geometry 
                      void *grad, int64_t gs0, int64_t gs1, cudaStream_t st) {
   size_t sm = interp_smem_bytes<T, NDIM, W>(g);
   auto kern = k_interp_dcoord<T, Tc, NDIM, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(kern, sm);
   kern<<<cl.nchunks, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
                                           static_cast<const cplx<T> *>(grid),
                                           static_cast<const cplx<T> *>(wts), ws,

@@ -195,7 +195,7 @@ void interp_run_w(const PointsDesc &pts, const uint32_t *sel, uint32_t npts, con
   constexpr uint32_t NW = IR_THREADS / 32;
   const size_t sm = NW * InterpShape<W>::WARP_BYTES;
   auto kern = k_interp_run<Tc, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(kern, sm);
   const uint32_t ppw = run_points_per_warp(uint64_t(npts) * uint64_t(ntrans));
   const uint64_t per = uint64_t(NW) * ppw;
   dim3 grd(unsigned((npts + per - 1) / per), ntrans);

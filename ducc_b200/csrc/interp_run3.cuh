@@ -201,7 +201,7 @@ void interp_run3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<do
                    int ntrans, cudaStream_t st) {
   using R = Interp3Shape<W>;
   auto kern = k_interp_run3<Tc, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(R::SMEM)));
+  allow_smem(kern, R::SMEM);
   // points per CTA: as the spreader
   const uint64_t per = uint64_t(pts.npts) * uint64_t(ntrans) / (148 * 8);
   const uint32_t ppb =
@@ -447,7 +447,7 @@ void interp_run3f_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<f
                     int ntrans, cudaStream_t st) {
   using R = Interp3fShape<W>;
   auto kern = k_interp_run3f<Tc, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(R::SMEM)));
+  allow_smem(kern, R::SMEM);
   const uint64_t per = uint64_t(pts.npts) * uint64_t(ntrans) / (148 * 8);
   const uint32_t ppb =
       per >= R::BATCH ? R::BATCH * uint32_t(std::min<uint64_t>(8, per / R::BATCH))

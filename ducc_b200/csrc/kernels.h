@@ -10,6 +10,15 @@ namespace dnufft {
 // is read back
 bool &bounded_wait_launched();
 
+// Lets launches of kern on the current device use `bytes` of dynamic shared
+// memory.  The limit belongs to the kernel, not to the launch: it is only ever
+// raised, as another host thread may be about to launch the same kernel with more.
+void allow_smem_of(const void *kern, size_t bytes);
+template <typename K>
+inline void allow_smem(K *kern, size_t bytes) {
+  allow_smem_of(reinterpret_cast<const void *>(kern), bytes);
+}
+
 // ---- binning / sorting (binsort.cu)
 // Order of the points inside a 2D or 3D tile, as key bits below the tile:
 // tensor core (2D, quadrant): the point's quadrant within its tile and below it

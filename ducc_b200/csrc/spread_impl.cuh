@@ -482,7 +482,7 @@ void spread_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
               void *grid, int64_t gtrans, int ntrans, cudaStream_t st) {
   size_t sm = spread_smem_bytes<T, W>(g);
   auto kern = k_spread<T, Tc, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(kern, sm);
   dim3 grd(cl.nchunks, ntrans);
   kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
                                     static_cast<const cplx<T> *>(values), vs, vtrans,
@@ -506,7 +506,7 @@ void interp_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
   }
   size_t sm = interp_smem_bytes<T, NDIM, W>(g, tpitch);
   auto kern = k_interp<T, Tc, NDIM, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(kern, sm);
   dim3 grd(cl.nchunks, ntrans);
   kern<<<grd, SP_THREADS, sm, st>>>(pts, cl.chunks, cl.count, g, kp,
                                     static_cast<const cplx<T> *>(grid), gtrans, static_cast<cplx<T> *>(out), os, otrans, map, tpitch,

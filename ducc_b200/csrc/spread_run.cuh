@@ -346,7 +346,7 @@ void spread_run_w(const PointsDesc &pts, const uint32_t *sel, uint32_t npts, con
   constexpr uint32_t NW = run_threads<T>() / 32;
   const size_t sm = NW * RunShape<T, W>::WARP_BYTES;
   auto kern = k_spread_run<T, Tc, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  allow_smem(kern, sm);
   const uint32_t ppw = run_points_per_warp(uint64_t(npts) * uint64_t(ntrans));
   const uint64_t per = uint64_t(NW) * ppw;
   dim3 grd(unsigned((npts + per - 1) / per), ntrans);

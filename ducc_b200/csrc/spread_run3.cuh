@@ -329,7 +329,7 @@ void spread_run3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<T>
                    int ntrans, cudaStream_t st) {
   using R = Run3Shape<T, W>;
   auto kern = k_spread_run3<T, Tc, W>;
-  DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(R::SMEM)));
+  allow_smem(kern, R::SMEM);
   // points per CTA: up to eight batches where that leaves 8 CTAs per SM, down
   // to 16 points for few points (the CTAs walk them one after the other)
   const uint64_t per = uint64_t(pts.npts) * uint64_t(ntrans) / (148 * 8);

@@ -998,7 +998,7 @@ void launch_spread_tc(const PointsDesc &pts, const TcBlocks &tb, const Geometry 
   {                                                                                             \
     auto kern = k_spread_tc<TC, WW>;                                                            \
     constexpr int smem = tc::smem_bytes<TC>();                                                  \
-    DN_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));     \
+    allow_smem(kern, smem);                                                                  \
     kern<<<tb.groups, tc::THREADS, smem, st>>>(pts, tb.kblk, tb.range, g, kp,                   \
                                                static_cast<const float2 *>(values), vs, absmax, \
                                                static_cast<float2 *>(grid), err);               \

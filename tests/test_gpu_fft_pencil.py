@@ -55,3 +55,39 @@ def test_pencil_lengths(nover, single):
         got2 = p.u2nu(grid=grid, forward=forward)
         ref2 = O.direct_u2nu(grid, coord, forward)
         assert O.l2error(got2, ref2) < 4 * eps
+
+
+def test_two_threads_of_different_shared_memory():
+    """Plans of long and short lines run the same kernels with different amounts
+    of shared memory from two host threads; neither may lower the other's limit."""
+    import threading
+    import torch
+    from ducc_b200 import nufft
+    plans = []
+    for i, shape in enumerate([(2000,), (40,)]):
+        rng = np.random.default_rng(i)
+        coord = torch.from_numpy(rng.uniform(-np.pi, np.pi, (50, 1))).cuda()
+        vals = torch.from_numpy(rng.standard_normal(50) + 0j).cuda()
+        p = nufft.plan(nu2u=True, coord=coord, grid_shape=shape, epsilon=1e-9)
+        out = torch.empty(shape, dtype=torch.complex128, device="cuda")
+        p.nu2u(points=vals, forward=True, out=out)
+        plans.append((p, vals, out, out.clone(), torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    errs = []
+
+    def work(p, vals, out, ref, stream):
+        try:
+            for _ in range(200):
+                p.nu2u(points=vals, forward=True, out=out, stream=stream.cuda_stream)
+        except Exception as e:
+            errs.append(e)
+
+    th = [threading.Thread(target=work, args=a) for a in plans]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not errs, errs
+    for p, vals, out, ref, stream in plans:
+        # the spreader's order of additions differs from run to run
+        assert torch.linalg.norm(out - ref) < 1e-12 * torch.linalg.norm(ref)
