@@ -693,8 +693,15 @@ static void build_index(const Setup &s, const View &coord, Index &ix, cudaStream
 
 // do type 1 / type 2 of this setup work from a chunk list?
 static bool spread_needs_chunks(const Setup &s) { return s.g.ndim == 1 || s.qbits; }
+// Two CTAs with a tile of 16 + W cells per axis fit an SM up to W = 7 in single
+// precision, and the tile kernel is the faster one at every density (ms, windows /
+// tiles: 128^3, W = 7, 3e5 points 0.29 / 0.23, 1e7 points 3.05 / 1.82; W = 5, 1e7
+// points 2.96 / 0.93); from W = 8 one fits and the windows are (3e5 points 0.38 /
+// 0.74, 1e7 points 3.19 / 3.56; 256^3, 1e7 points 3.79 / 4.77).  No complex128 tile fits.
+bool interp3_in_windows(const Geometry &g, bool f64) { return f64 || g.W >= 8; }
 static bool interp_needs_chunks(const Setup &s) {
-  return s.g.ndim == 1 || (s.g.ndim == 2 && !s.calc_f64);
+  if (s.g.ndim == 3) return !interp3_in_windows(s.g, s.calc_f64);
+  return s.g.ndim == 1 || !s.calc_f64;
 }
 
 static size_t grid_cells(const Geometry &g) {

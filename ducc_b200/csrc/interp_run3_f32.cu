@@ -7,15 +7,14 @@ void launch_interp_run3(const PointsDesc &pts, const Geometry &g, const KernelPo
                         const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
                         int ntrans, cudaStream_t st) {
   if (pts.npts == 0 || ntrans == 0) return;
-#define DN_CASE(WW)                                                                          \
-  case WW:                                                                                   \
-    if (pts.coord_f64)                                                                       \
-      interp_run3f_w<double, WW>(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);     \
-    else                                                                                     \
-      interp_run3f_w<float, WW>(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);      \
+  // the one support for which interp3_in_windows (capi.cpp) holds in single precision
+  if (g.W == 8) {
+    if (pts.coord_f64)
+      interp_run3f_w<double, 8>(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
+    else
+      interp_run3f_w<float, 8>(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
     return;
-  switch (g.W) { DN_FOR_W_FLOAT(DN_CASE) }
-#undef DN_CASE
+  }
   throw Error(ST_UNSUPPORTED, "kernel support not supported by this build");
 }
 

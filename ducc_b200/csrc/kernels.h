@@ -137,7 +137,10 @@ void launch_interp_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts
                        int64_t gtrans, void *out, int64_t os, int64_t otrans, int ntrans,
                        cudaStream_t st);
 
-// 3D (launch_interp goes here; no chunk list)
+// Does 3D type 2 work bin by bin from the grid (launch_interp_run3; no chunk
+// list) or from tiles staged in shared memory (k_interp, single precision only)?
+bool interp3_in_windows(const Geometry &g, bool f64);
+// 3D (launch_interp goes here where interp3_in_windows)
 void launch_interp_run3(const PointsDesc &pts, const Geometry &g, const KernelPoly<float> &kp,
                         const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,
                         int ntrans, cudaStream_t st);

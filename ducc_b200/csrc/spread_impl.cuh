@@ -1,6 +1,6 @@
 // Plain spreading (type 1, 1D; 2D and 3D: spread_run.cuh, spread_run3.cuh) and
-// interpolation (type 2, 1D and 2D single precision; 2D double: interp_run.cuh,
-// 3D: interp_run3.cuh) kernels.
+// interpolation (type 2, 1D and single precision; 2D double: interp_run.cuh, 3D
+// where interp3_in_windows: interp_run3.cuh) kernels.
 //
 // One CTA per chunk of tile-sorted points (at most CHUNK points of one tile).
 // Spreading: every warp takes 32 points at a time, each lane folds its point
@@ -239,9 +239,11 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
                                              unsigned char *smraw,
                                              const CUtensorMap *tmap = nullptr, int tpitch = 0,
                                              uint64_t *tbar = nullptr, int *err = nullptr) {
-  static_assert(NDIM <= 2, "3D: interp_run3.cuh");
+  static_assert(BufferLayout<T>::smem(NDIM), "the tile is staged in shared memory");
   const int S = (1 << g.log2tile) + W;
-  const int ncell = NDIM == 2 ? S * S : S;
+  int ncell = S;
+  if (NDIM >= 2) ncell *= S;
+  if (NDIM >= 3) ncell *= S;
   int b0[NDIM];
   tile_origin<NDIM>(ch.tile, g, b0);
   cplx<T> *buf = reinterpret_cast<cplx<T> *>(smraw);
@@ -408,7 +410,7 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
             ar += wt[0][a] * gv.x;
             ai += wt[0][a] * gv.y;
           }
-        } else {
+        } else if constexpr (NDIM == 2) {
 #pragma unroll
           for (int a = 0; a < W; ++a) {
             const cplx<T> *row = p0 + a * pitch;
@@ -421,6 +423,26 @@ __device__ __forceinline__ void interp_chunk(const PointsDesc &pts, const Chunk 
             }
             ar += wt[0][a] * rr;
             ai += wt[0][a] * ri;
+          }
+        } else {
+#pragma unroll 1
+          for (int a = 0; a < W; ++a) {
+            T pr = 0, pi = 0;
+#pragma unroll
+            for (int b = 0; b < W; ++b) {
+              const cplx<T> *row = p0 + (a * S + b) * S;
+              T rr = 0, ri = 0;
+#pragma unroll
+              for (int e = 0; e < W; ++e) {
+                cplx<T> gv = row[e];
+                rr += wt[2][e] * gv.x;
+                ri += wt[2][e] * gv.y;
+              }
+              pr += wt[1][b] * rr;
+              pi += wt[1][b] * ri;
+            }
+            ar += wt[0][a] * pr;
+            ai += wt[0][a] * pi;
           }
         }
         out[int64_t(j) * os] = mkc<T>(ar, ai);
@@ -578,7 +600,7 @@ template <typename T>
 void launch_interp_impl(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
                         const KernelPoly<T> &kp, const void *grid, int64_t gtrans, void *out,
                         int64_t os, int64_t otrans, int ntrans, cudaStream_t st, int *err) {
-  if (g.ndim == 3) {
+  if (g.ndim == 3 && interp3_in_windows(g, sizeof(T) == 8)) {
     launch_interp_run3(pts, g, kp, grid, gtrans, out, os, otrans, ntrans, st);
     return;
   }
@@ -593,7 +615,11 @@ void launch_interp_impl(const PointsDesc &pts, const ChunkList &cl, const Geomet
   if (g.ndim == 1) {
     if (pts.coord_f64) DN_ID(double, 1); else DN_ID(float, 1);
   } else if constexpr (sizeof(T) == 4) {
-    if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
+    if (g.ndim == 3) {
+      if (pts.coord_f64) DN_ID(double, 3); else DN_ID(float, 3);
+    } else {
+      if (pts.coord_f64) DN_ID(double, 2); else DN_ID(float, 2);
+    }
   }
 #undef DN_ID
 }

@@ -115,12 +115,12 @@ def test_nonfinite_value_stays_in_its_footprint(single, shape, nover):
     assert O.l2error(got[~bad], ref[~bad]) < (3e-6 if single else 1e-10)
 
 
-@pytest.mark.parametrize("single,shape,nover", [(False, (50, 60), (110, 126)),
-                                                (False, (15, 20, 9), (36, 48, 20)),
-                                                (True, (15, 20, 9), (36, 48, 20))])
-def test_nonfinite_cell_reaches_its_points_only(single, shape, nover):
+@pytest.mark.parametrize("single,W,shape,nover", [(False, 6, (50, 60), (110, 126)),
+                                                  (False, 6, (15, 20, 9), (36, 48, 20)),
+                                                  (True, 6, (15, 20, 9), (36, 48, 20)),
+                                                  (True, 8, (15, 20, 9), (36, 48, 20))])
+def test_nonfinite_cell_reaches_its_points_only(single, W, shape, nover):
     import torch
-    W = 6
     p, k, nov, coord, vals = _case(W, single, shape, nover, 400, "uniform")
     plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=shape,
                       epsilon=1e-3, force_kernel=k, force_nover=nov)
