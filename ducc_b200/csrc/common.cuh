@@ -35,30 +35,6 @@ __device__ __forceinline__ cplx<T> csub(cplx<T> a, cplx<T> b) {
   return mkc<T>(a.x - b.x, a.y - b.y);
 }
 
-// ---------------------------------------------------------------------------
-// Coordinate fold: DUCC's Nufft_ancestor::getpix (src/ducc0/nufft/nufft.h:285-298)
-//   tmp  = x * (1/period);  f = tmp - floor(tmp)
-//   tmp2 = f * n            (long double for float64 coords, double otherwise)
-//   i0   = min(int(tmp2 + shift) - n, maxi0)
-//   frac = tmp2 - i0
-// For float32 coordinates DUCC's optimised build evaluates frac as one fused
-// multiply-add, fma(f, n, -i0); that is reproduced here.  For float64
-// coordinates the x87 80-bit arithmetic (64-bit significand, round to nearest
-// even) is emulated exactly with 128-bit integers.
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ void fold_f32(double x, double coordfct, int n, double shift,
-                                         int maxi0, int &i0, double &frac) {
-  double tmp = __dmul_rn(x, coordfct);
-  double f = tmp - floor(tmp);
-  double tmp2 = __dmul_rn(f, double(n));
-  int s = int(__dadd_rn(tmp2, shift));
-  i0 = min(s - n, maxi0);
-  frac = __fma_rn(f, double(n), -double(i0));
-}
-
-typedef unsigned __int128 u128;
-
 __host__ __device__ __forceinline__ int clz64(uint64_t v) {
 #ifdef __CUDA_ARCH__
   return __clzll((long long)v);
@@ -101,6 +77,38 @@ __host__ __device__ __forceinline__ double of_bits(uint64_t a) {
   return r;
 #endif
 }
+__host__ __device__ __forceinline__ double nan_f64() { return of_bits(0x7ff8000000000000ull); }
+
+// ---------------------------------------------------------------------------
+// Coordinate fold: DUCC's Nufft_ancestor::getpix (src/ducc0/nufft/nufft.h:285-298)
+//   tmp  = x * (1/period);  f = tmp - floor(tmp)
+//   tmp2 = f * n            (long double for float64 coords, double otherwise)
+//   i0   = min(int(tmp2 + shift) - n, maxi0)
+//   frac = tmp2 - i0
+// For float32 coordinates DUCC's optimised build evaluates frac as one fused
+// multiply-add, fma(f, n, -i0); that is reproduced here.  For float64
+// coordinates the x87 80-bit arithmetic (64-bit significand, round to nearest
+// even) is emulated exactly with 128-bit integers.
+//
+// For every x, i0 lies in [-nsafe, n + 1 - nsafe], nsafe = (W + 1) / 2: shift is
+// n + 1 - W / 2 and maxi0 is n + nsafe - W.  Tile keys, chunks and the cells that
+// a kernel touches rest on that.  An x that is not finite gets the cell of
+// position 0 and a frac that is not a number, so that its weights are not either.
+// ---------------------------------------------------------------------------
+
+__host__ __device__ __forceinline__ void fold_f32(double x, double coordfct, int n, double shift,
+                                                  int maxi0, int &i0, double &frac) {
+  const double tmp = mul_rn(x, coordfct);
+  double f = add_rn(tmp, -floor(tmp));
+  const bool nan = !(f == f);
+  if (nan) f = 0.;
+  const double tmp2 = mul_rn(f, double(n));
+  const int s = int(add_rn(tmp2, shift)) - n;
+  i0 = s < maxi0 ? s : maxi0;
+  frac = nan ? nan_f64() : fma(f, double(n), -double(i0));
+}
+
+typedef unsigned __int128 u128;
 
 __host__ __device__ __forceinline__ int bitlen128(u128 v) {
   uint64_t hi = uint64_t(v >> 64), lo = uint64_t(v);
@@ -132,7 +140,7 @@ __host__ __device__ __forceinline__ u128 round_sig(u128 v, bool sticky, int keep
   return r;
 }
 
-// the fold of a fractional position f in 128-bit integers (any f)
+// the fold of a fractional position f in 128-bit integers (any f in [0, 1])
 __host__ __device__ __noinline__ inline void fold_f64_int(double f, int n, double shift, int maxi0,
                                                           int *i0_, double *frac_) {
   int i0;
@@ -199,7 +207,9 @@ __host__ __device__ __forceinline__ double round64_magic(double a) {
 __host__ __device__ __forceinline__ void fold_f64(double x, double coordfct, int n, double shift,
                                                   int maxi0, int &i0, double &frac) {
   const double tmp = mul_rn(x, coordfct);
-  const double f = add_rn(tmp, -floor(tmp));
+  double f = add_rn(tmp, -floor(tmp));
+  const bool nan = !(f == f);
+  if (nan) f = 0.;
   const double dn = double(n);
   const double hi = mul_rn(f, dn), lo = fma(f, dn, -hi);
   const double m1 = round64_magic(hi);
@@ -224,10 +234,11 @@ __host__ __device__ __forceinline__ void fold_f64(double x, double coordfct, int
   ok = ok && s > 0x1p-38 && (bits_of(s) & 0x000fffffffffffffull) != 0;
   frac = add_rn(s, l64);
   if (!ok) fold_f64_int(f, n, shift, maxi0, &i0, &frac);
+  if (nan) frac = nan_f64();
 }
 
 template <typename Tc>
-__device__ __forceinline__ void fold(Tc x, double coordfct, int n, double shift, int maxi0,
+__host__ __device__ __forceinline__ void fold(Tc x, double coordfct, int n, double shift, int maxi0,
                                      int &i0, double &frac) {
   if constexpr (sizeof(Tc) == 4)
     fold_f32(double(x), coordfct, n, shift, maxi0, i0, frac);
@@ -306,13 +317,6 @@ __device__ __forceinline__ int wrap2(int i, int n) {
   i = i < 0 ? i + n : i;
   i = i >= n ? i - n : i;
   return i >= n ? i - n : i;
-}
-
-// First footprint cell i0 of a point, counted from -nsafe: 0 .. n + 1 for every
-// finite coordinate; a coordinate that is not finite is kept inside too (its
-// weights are not finite, whatever cells they reach).
-__device__ __forceinline__ int first_cell(int i0, int nsafe, int n) {
-  return min(max(i0 + nsafe, 0), n + 1);
 }
 
 // floor(x / d) for d >= 2 and x * d < 2^32 by a multiply-high with m = ceil(2^32 / d)

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(IR_THREADS, W <= 9 ? 4 : 3)
       double frac, w[W];
       fold<Tc>(x, ax ? g.coordfct[1] : g.coordfct[0], ax ? n1 : n0, ax ? g.shift[1] : g.shift[0],
                ax ? g.maxi0[1] : g.maxi0[0], i0, frac);
-      t = first_cell(i0, g.nsafe, ax ? n1 : n0);
+      t = i0 + g.nsafe;
       kernel_weights<double, W>(kp, double(W - 1) - 2.0 * frac, w);
       double *sp = st + q * R::ST + (ax ? R::ROWS : 0) + (t & 7);
 #pragma unroll

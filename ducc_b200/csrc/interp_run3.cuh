@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(Interp3Shape<W>::THREADS)
                ax == 0 ? g.shift[0] : (ax == 1 ? g.shift[1] : g.shift[2]),
                ax == 0 ? g.maxi0[0] : (ax == 1 ? g.maxi0[1] : g.maxi0[2]), i0, frac);
       kernel_weights<double, W>(kp, double(W - 1) - 2.0 * frac, w);
-      const int t = first_cell(i0, g.nsafe, ax == 0 ? n0 : (ax == 1 ? n1 : n2));
+      const int t = i0 + g.nsafe;
       int *inf = reinterpret_cast<int *>(info + q);
       inf[ax] = t >> R::LB;
       if (ax == 0) inf[3] = int(j);
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(Interp3fShape<W>::THREADS, 4)
                ax == 0 ? g.shift[0] : (ax == 1 ? g.shift[1] : g.shift[2]),
                ax == 0 ? g.maxi0[0] : (ax == 1 ? g.maxi0[1] : g.maxi0[2]), i0, frac);
       kernel_weights<float, W>(kp, float(double(W - 1) - 2.0 * frac), w);
-      const int t = first_cell(i0, g.nsafe, ax == 0 ? n0 : (ax == 1 ? n1 : n2)), o = t & 7;
+      const int t = i0 + g.nsafe, o = t & 7;
       int *inf = reinterpret_cast<int *>(info + q);
       inf[ax] = ax == 0 ? t : t >> 3;
       float *sp = st + q * R::ST;

@@ -232,13 +232,13 @@ __device__ __forceinline__ void spread_run(const PointsDesc &pts, const uint32_t
       T w[W];
       if constexpr (R::F32) {
         fold<Tc>(x[0], g.coordfct[0], n0, g.shift[0], g.maxi0[0], i0, frac);
-        tu = first_cell(i0, g.nsafe, n0);
+        tu = i0 + g.nsafe;
         kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w);
         T *sr = sp + (tu & 7);
 #pragma unroll
         for (int a = 0; a < W; ++a) sr[a] = w[a];
         fold<Tc>(x[1], g.coordfct[1], n1, g.shift[1], g.maxi0[1], i0, frac);
-        tv = first_cell(i0, g.nsafe, n1);
+        tv = i0 + g.nsafe;
         kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w);
         cplx<T> *sc = reinterpret_cast<cplx<T> *>(sp + R::ROWS) + (tv & 7);
 #pragma unroll
@@ -246,7 +246,7 @@ __device__ __forceinline__ void spread_run(const PointsDesc &pts, const uint32_t
       } else {
         fold<Tc>(ax ? x[1] : x[0], ax ? g.coordfct[1] : g.coordfct[0], ax ? n1 : n0,
                  ax ? g.shift[1] : g.shift[0], ax ? g.maxi0[1] : g.maxi0[0], i0, frac);
-        tu = first_cell(i0, g.nsafe, ax ? n1 : n0);
+        tu = i0 + g.nsafe;
         kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w);
         if (ax == 0) {
           T *sr = sp + (tu & 7);

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(Run3Shape<T, W>::THREADS)
                ax == 0 ? g.shift[0] : (ax == 1 ? g.shift[1] : g.shift[2]),
                ax == 0 ? g.maxi0[0] : (ax == 1 ? g.maxi0[1] : g.maxi0[2]), i0, frac);
       kernel_weights<T, W>(kp, T(double(W - 1) - 2.0 * frac), w);
-      const int t = first_cell(i0, g.nsafe, ax == 0 ? n0 : (ax == 1 ? n1 : n2)),
+      const int t = i0 + g.nsafe,
                 o = t & (R::BIN - 1);
       T *sp = st + q * R::ST;
       int *inf = reinterpret_cast<int *>(info + q);
