@@ -313,9 +313,16 @@ __device__ __forceinline__ int wrapi(int i, int n) {
 __device__ __forceinline__ int wrap1(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
 // periodic wrap of i in [-n, 3n) without a division
-__device__ __forceinline__ int wrap2(int i, int n) {
+__host__ __device__ __forceinline__ int wrap2(int i, int n) {
   i = i < 0 ? i + n : i;
   i = i >= n ? i - n : i;
+  return i >= n ? i - n : i;
+}
+
+// the same for i in [-n, 4n)
+__host__ __device__ __forceinline__ int wrap3(int i, int n) {
+  i = i < 0 ? i + n : i;
+  i = i >= 2 * n ? i - 2 * n : i;
   return i >= n ? i - n : i;
 }
 

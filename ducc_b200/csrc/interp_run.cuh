@@ -69,10 +69,10 @@ __global__ void __launch_bounds__(IR_THREADS, W <= 9 ? 4 : 3)
     const double *gd = reinterpret_cast<const double *>(grid) + ((lane >> 2) & 1);
 #pragma unroll
     for (int r = 0; r < R::RT; ++r) {
-      const double *row = gd + 2 * int64_t(wrap2(u0 + 4 * r + (lane >> 3), n0)) * n1;
+      const double *row = gd + 2 * int64_t(wrap3(u0 + 4 * r + (lane >> 3), n0)) * n1;
 #pragma unroll
       for (int k = 0; k < R::KT; ++k) {
-        G[r][k] = __ldg(row + 2 * wrap2(v0 + 4 * k + (lane & 3), n1));
+        G[r][k] = __ldg(row + 2 * wrap3(v0 + 4 * k + (lane & 3), n1));
         ok = ok && isfinite(G[r][k]);
       }
     }
@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(IR_THREADS, W <= 9 ? 4 : 3)
           for (int c = lane; c < W * W; c += 32) {
             const int a = c / W, b = c - a * W;
             const double wt = f[(tu & 7) + a] * f[R::ROWS + (tv & 7) + b];
-            const double2 gv = __ldg(grid + int64_t(wrap2(tu - g.nsafe + a, n0)) * n1 +
-                                     wrap2(tv - g.nsafe + b, n1));
+            const double2 gv = __ldg(grid + int64_t(wrap3(tu - g.nsafe + a, n0)) * n1 +
+                                     wrap3(tv - g.nsafe + b, n1));
             sx += wt * gv.x;
             sy += wt * gv.y;
           }

@@ -56,17 +56,17 @@ __global__ void __launch_bounds__(Interp3Shape<W>::THREADS)
   int cu = -1, cv = -1, cw = -1;
   bool finite = true;
   auto load_window = [&]() {
-    const int u = wrap2(cu * R::BIN - g.nsafe + warp, n0), v0 = cv * R::BIN - g.nsafe,
+    const int u = wrap3(cu * R::BIN - g.nsafe + warp, n0), v0 = cv * R::BIN - g.nsafe,
               w0 = cw * R::BIN - g.nsafe;
     const double *pl = reinterpret_cast<const double *>(grid + int64_t(u) * n1 * n2) +
                        ((lane >> 2) & 1);
     bool ok = true;
 #pragma unroll
     for (int r = 0; r < R::RT; ++r) {
-      const double *row = pl + 2 * int64_t(wrap2(v0 + 4 * r + (lane >> 3), n1)) * n2;
+      const double *row = pl + 2 * int64_t(wrap3(v0 + 4 * r + (lane >> 3), n1)) * n2;
 #pragma unroll
       for (int k = 0; k < R::KT; ++k) {
-        G[r][k] = __ldg(row + 2 * wrap2(w0 + 4 * k + (lane & 3), n2));
+        G[r][k] = __ldg(row + 2 * wrap3(w0 + 4 * k + (lane & 3), n2));
         ok = ok && isfinite(G[r][k]);
       }
     }
@@ -154,15 +154,15 @@ __global__ void __launch_bounds__(Interp3Shape<W>::THREADS)
             } else if (ku != 0.) {
               // a value of the plane is not finite: the footprint's cells only
               const double2 *pl =
-                  grid + int64_t(wrap2(cu * R::BIN - g.nsafe + warp, n0)) * n1 * n2;
+                  grid + int64_t(wrap3(cu * R::BIN - g.nsafe + warp, n0)) * n1 * n2;
               for (int r = lane & 3; r < R::SPAN; r += 4) {
                 const double kv = f[R::PLANES + r];
                 if (kv == 0.) continue;
-                const double2 *row = pl + int64_t(wrap2(cv * R::BIN - g.nsafe + r, n1)) * n2;
+                const double2 *row = pl + int64_t(wrap3(cv * R::BIN - g.nsafe + r, n1)) * n2;
                 for (int c = 0; c < R::SPAN; ++c) {
                   const double wt = kv * f[R::PLANES + R::ROWS + c];
                   if (wt == 0.) continue;
-                  const double2 gv = __ldg(row + wrap2(cw * R::BIN - g.nsafe + c, n2));
+                  const double2 gv = __ldg(row + wrap3(cw * R::BIN - g.nsafe + c, n2));
                   sx += wt * gv.x;
                   sy += wt * gv.y;
                 }
@@ -315,14 +315,14 @@ __global__ void __launch_bounds__(Interp3fShape<W>::THREADS, 4)
   auto load_window = [&]() {
     const int u0 = cu * 8 - g.nsafe, rv = cv * 8 - g.nsafe + L::row0(lane),
               wa = cw * 8 - g.nsafe + L::cell0(lane);
-    const int ca = wrap2(wa, n2), cb = wrap2(wa + 8, n2);
+    const int ca = wrap3(wa, n2), cb = wrap3(wa + 8, n2);
     bool ok = true;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float2 *pl = grid + int64_t(wrap2(u0 + warp + 4 * j, n0)) * n1 * n2;
+      const float2 *pl = grid + int64_t(wrap3(u0 + warp + 4 * j, n0)) * n1 * n2;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float2 *row = pl + int64_t(wrap2(rv + i, n1)) * n2;
+        const float2 *row = pl + int64_t(wrap3(rv + i, n1)) * n2;
         const float2 a = __ldg(row + ca), b = __ldg(row + cb);
         win.c[j][0][i] = pack2(a.x, a.y);
         win.c[j][1][i] = pack2(b.x, b.y);
@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(Interp3fShape<W>::THREADS, 4)
               const float wt = f[4 * warp + j] * f[R::PLANES + r] * f[R::PLANES + R::ROWS + c];
               if (wt == 0.f) continue;
               const float2 gv = __ldg(
-                  grid + (int64_t(wrap2(cu * 8 - g.nsafe + warp + 4 * j, n0)) * n1 +
-                          wrap2(cv * 8 - g.nsafe + r, n1)) * n2 + wrap2(cw * 8 - g.nsafe + c, n2));
+                  grid + (int64_t(wrap3(cu * 8 - g.nsafe + warp + 4 * j, n0)) * n1 +
+                          wrap3(cv * 8 - g.nsafe + r, n1)) * n2 + wrap3(cw * 8 - g.nsafe + c, n2));
               sx += wt * gv.x;
               sy += wt * gv.y;
             }

@@ -79,9 +79,14 @@ __device__ __forceinline__ float2 unpack2(unsigned long long a) {
 }
 
 // The window of the current bin: adds points [s, e) of the staged batch,
-// flushes itself to the grid.  A window starts in [-8, n + 1) and is at most 24
-// cells wide (n >= 16), so its cells lie in [-n, 3n).
+// flushes itself to the grid.  A window starts in [-nsafe, n + 1 - nsafe], n >= 2
+// nsafe, and is at most 24 cells wide, so its cells lie in [-n, 4n); beyond 3n only
+// those of 16 cells at n = 4, which only W = 4 has.
 template <typename T, int W> struct RunWindow;
+
+template <int W> __host__ __device__ __forceinline__ int run_wrap(int i, int n) {
+  return W == 4 ? wrap3(i, n) : wrap2(i, n);
+}
 
 // float: each lane has rows 4 rg .. + 3 of the cells cg and cg + 8, with rg =
 // lane bit 0 and bit 4, cg = lane bits 1..3: at most two addresses among four
@@ -116,10 +121,10 @@ template <int W> struct RunWindow<float, W> {
   __device__ __forceinline__ void flush(float2 *grid, int u0, int v0, int n0, int n1, bool inside,
                                         int lane) {
     const int ru = u0 + row0(lane), va = v0 + cell0(lane);
-    float2 *pa = grid + (inside ? va : wrap2(va, n1)), *pb = grid + (inside ? va + 8 : wrap2(va + 8, n1));
+    float2 *pa = grid + (inside ? va : run_wrap<W>(va, n1)), *pb = grid + (inside ? va + 8 : run_wrap<W>(va + 8, n1));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int64_t off = int64_t(inside ? ru + i : wrap2(ru + i, n0)) * n1;
+      const int64_t off = int64_t(inside ? ru + i : run_wrap<W>(ru + i, n0)) * n1;
       const float2 a = unpack2(c[0][i]), b = unpack2(c[1][i]);
       if (a.x != 0.f || a.y != 0.f) atomicAdd(pa + off, a);
       if (b.x != 0.f || b.y != 0.f) atomicAdd(pb + off, b);
@@ -164,10 +169,10 @@ template <int W> struct RunWindow<double, W> {
     const int ru = u0 + (lane >> 2), cv = v0 + (lane & 3);
 #pragma unroll
     for (int m = 0; m < R::MT; ++m) {
-      double2 *row = grid + int64_t(inside ? ru + 8 * m : wrap2(ru + 8 * m, n0)) * n1;
+      double2 *row = grid + int64_t(inside ? ru + 8 * m : wrap3(ru + 8 * m, n0)) * n1;
 #pragma unroll
       for (int n = 0; n < R::NT; ++n) {
-        double2 *q = row + (inside ? cv + 4 * n : wrap2(cv + 4 * n, n1));
+        double2 *q = row + (inside ? cv + 4 * n : wrap3(cv + 4 * n, n1));
         if (c[m][n][0] != 0.) atomicAdd(&q->x, c[m][n][0]);
         if (c[m][n][1] != 0.) atomicAdd(&q->y, c[m][n][1]);
       }

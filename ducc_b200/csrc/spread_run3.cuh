@@ -104,13 +104,13 @@ template <int W> struct Run3Window<float, W> {
   __device__ __forceinline__ void flush(float2 *grid, int u0, int v0, int w0, int n0, int n1,
                                         int n2, int warp, int lane) {
     const int rv = v0 + L::row0(lane), wa = w0 + L::cell0(lane);
-    const int ca = wrap2(wa, n2), cb = wrap2(wa + 8, n2);
+    const int ca = wrap3(wa, n2), cb = wrap3(wa + 8, n2);
     int64_t row[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) row[i] = int64_t(wrap2(rv + i, n1)) * n2;
+    for (int i = 0; i < 4; ++i) row[i] = int64_t(wrap3(rv + i, n1)) * n2;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      float2 *pl = grid + int64_t(wrap2(u0 + warp + 4 * j, n0)) * n1 * n2;
+      float2 *pl = grid + int64_t(wrap3(u0 + warp + 4 * j, n0)) * n1 * n2;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float2 a = unpack2(c[j][0][i]), b = unpack2(c[j][1][i]);
@@ -158,14 +158,14 @@ template <int W> struct Run3Window<double, W> {
   }
   __device__ __forceinline__ void flush(double2 *grid, int u0, int v0, int w0, int n0, int n1,
                                         int n2, int warp, int lane) {
-    double2 *pl = grid + int64_t(wrap2(u0 + warp, n0)) * n1 * n2;
+    double2 *pl = grid + int64_t(wrap3(u0 + warp, n0)) * n1 * n2;
     const int rv = v0 + (lane >> 2), cw = w0 + (lane & 3);
 #pragma unroll
     for (int m = 0; m < R::MT; ++m) {
-      double2 *row = pl + int64_t(wrap2(rv + 8 * m, n1)) * n2;
+      double2 *row = pl + int64_t(wrap3(rv + 8 * m, n1)) * n2;
 #pragma unroll
       for (int n = 0; n < R::NT; ++n) {
-        double2 *q = row + wrap2(cw + 4 * n, n2);
+        double2 *q = row + wrap3(cw + 4 * n, n2);
         if (c[m][n][0] != 0.) atomicAdd(&q->x, c[m][n][0]);
         if (c[m][n][1] != 0.) atomicAdd(&q->y, c[m][n][1]);
       }
@@ -272,8 +272,8 @@ __global__ void __launch_bounds__(Run3Shape<T, W>::THREADS)
           const T wt = sp[Run3Window<T, W>::plane_slot(a)] * sp[R::PLANES + b] *
                        sp[R::PLANES + R::ROWS + 2 * e];
           if (wt != T(0))
-            global_add<T>(grid + (int64_t(wrap2(u0 + a, n0)) * n1 + wrap2(v0 + b, n1)) * n2 +
-                              wrap2(w0 + e, n2),
+            global_add<T>(grid + (int64_t(wrap3(u0 + a, n0)) * n1 + wrap3(v0 + b, n1)) * n2 +
+                              wrap3(w0 + e, n2),
                           wt * v.x, wt * v.y);
         }
       }

@@ -134,3 +134,14 @@ def test_nonfinite_cell_reaches_its_points_only(single, W, shape, nover):
     hit = np.all((np.array(cell) - i0) % np.array(nov) < W, axis=1)
     assert 0 < hit.sum() < 400 and np.array_equal(~np.isfinite(got), hit)
     assert O.l2error(got[~hit], ref[~hit]) < (3e-6 if single else 1e-10)
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+@pytest.mark.parametrize("single,W", [(True, w) for w in range(4, 9)] +
+                         [(False, w) for w in range(4, 17)])
+def test_smallest_grids(single, W, ndim):
+    """Oversampled axes of 2 nsafe cells, the shortest that are accepted: the
+    windows go around them more than once."""
+    n = 2 * ((W + 1) // 2)
+    _run(W, single, (2, 3, 2)[:ndim], (n, n, n + 2 if n + 2 != 14 else n)[:ndim], 200, "edges")
+    _run(W, single, (2, 3, 2)[:ndim], (n,) * ndim, 200, "uniform")
