@@ -60,14 +60,16 @@ __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t c
             (uint32_t(t[1] >> 3) & bm);
     }
   } else if (order.bin_bits) {
-    // bin inside the tile, then the first axis inside the bin
+    // bin inside the tile, then the cell inside the bin along the first axes
     const int L = g.log2tile, lb = order.bin_log2, ab = L - lb;
     const uint32_t bm = (1u << ab) - 1u;
     key = uint32_t(t[0] >> L) * uint32_t(g.ntiles[1] * g.ntiles[2]) +
           uint32_t(t[1] >> L) * uint32_t(g.ntiles[2]) + uint32_t(t[2] >> L);
 #pragma unroll
     for (int d = 0; d < NDIM; ++d) key = (key << ab) | (uint32_t(t[d] >> lb) & bm);
-    key = (key << lb) | (uint32_t(t[0]) & ((1u << lb) - 1u));
+#pragma unroll
+    for (int d = 0; d < NDIM; ++d)
+      if (d < order.cell_axes) key = (key << lb) | (uint32_t(t[d]) & ((1u << lb) - 1u));
   } else {
     uint32_t ss = uint32_t(g.ssmall), ms = (1u << ss) - 1u;
     uint32_t a = uint32_t(t[0] >> g.lsq2), b = uint32_t(t[1] >> g.lsq2),

@@ -403,9 +403,21 @@ static int bitlen64(uint64_t v) {
   return b;
 }
 
+// Digits up to which the sort also orders the points of a 3D bin by cell
+// (make_setup).  The kernels with one thread per point (k_interp_direct3, k_interp,
+// k_interp_dcoord) read fewer lines per warp then: complex128, 2e6 clustered points,
+// 176^3 cells, W = 8: interpolation 1348 -> 896 us, gradient 1886 -> 1578; complex64,
+// 132^3 cells, W = 6: gradient 451 -> 378.  Longer digits make the sort slower (5e6
+// points, 11 bits for 10: plan 411 -> 543 us), which complex64 plans do not pay for;
+// unplanned complex64 calls and type 1 keep the shortest key (20,000 points: 9 us).
+constexpr int CELL_DIGIT_F64 = RADIX_BITS, CELL_DIGIT_F32 = 10;
+
+// run_order: sort the points by bin inside their tile.  cell_digit: in 3D by cell
+// inside the bin too, as far as the passes of the sort keep to digits of so many bits
+// (0: by the first axis only).
 static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double epsilon,
                         bool gridding, bool calc_f64, bool coord_f64, const dnufft_opts &o,
-                        bool run_order = false) {
+                        bool run_order = false, int cell_digit = 0) {
   DN_REQUIRE(ndim >= 1 && ndim <= 3, ST_BADARG, "transform must be 1D/2D/3D");
   DN_REQUIRE(npoints <= 0xffffffffull, ST_BADARG, "too many nonuniform points");
   DN_REQUIRE(epsilon > 0, ST_BADARG, "epsilon must be positive");
@@ -514,11 +526,14 @@ static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double 
   } else if (run_order && ndim == 3) {
     // bins and, inside them, the first axis, where the key has room for them
     const int lb = spread_run3_bin_log2(g.W), bb = 3 * (g.log2tile - lb);
-    if (bitlen64(s.max_tiles) + bb + lb <= 32) {
+    const int bits = bitlen64(s.max_tiles) + bb + lb;
+    if (bits <= 32) {
       s.order.bin_bits = bb;
       s.order.bin_log2 = lb;
-      s.tile_shift = bb + lb;
-      maxkey = s.max_tiles << lb;   // (bin_bits are added below)
+      const int room = std::min(32, (bits + RADIX_BITS - 1) / RADIX_BITS * cell_digit);
+      while (s.order.cell_axes < 3 && bits + s.order.cell_axes * lb <= room) ++s.order.cell_axes;
+      s.tile_shift = bb + lb * s.order.cell_axes;
+      maxkey = s.max_tiles << (lb * s.order.cell_axes);   // (bin_bits are added below)
     }
   }
   DN_REQUIRE(maxkey < (uint64_t(1) << 32), ST_UNSUPPORTED, "tile key space too large");
@@ -1138,7 +1153,8 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   DN_REQUIRE(out.dtype == uni.dtype, ST_BADARG, "out must have the dtype of grid");
   bool f64 = uni.dtype == DNUFFT_C128;
   Setup s = make_setup(ndim, uni.shape, uint64_t(coord.shape[0]), eps, false, f64,
-                       coord.dtype == DNUFFT_F64, o, ndim == 3 || (f64 && ndim == 2));
+                       coord.dtype == DNUFFT_F64, o, ndim == 3 || (f64 && ndim == 2),
+                       f64 ? CELL_DIGIT_F64 : 0);
   StageTimer tm(o.verbosity > 0, st);
   if (o.verbosity > 0) report_sizes(s, false);
   if (s.npoints == 0) return;
@@ -1263,7 +1279,8 @@ static void plan_create_impl(int nu2u, const dnufft_array *coord_, const int64_t
   bool f64 = coord.dtype == DNUFFT_F64;
   auto p = std::make_unique<dnufft_plan>();
   p->o = o;
-  p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o, true);
+  p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o, true,
+                    f64 ? CELL_DIGIT_F64 : CELL_DIGIT_F32);
   DN_CUDA(cudaGetDevice(&p->device));
   p->dc = &consts_for(p->s, p->own, st);
   if (p->s.npoints > 0) {

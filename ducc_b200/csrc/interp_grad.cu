@@ -18,8 +18,18 @@
 
 namespace dnufft {
 
+// CTAs per SM asked for in 3D: two up to W = 7 (at most 128 registers: with 132 only
+// one fits, 1.3 times the time), one from W = 11, where the compiler otherwise keeps
+// to 122 to 170 registers and fewer loads in flight (complex128, 1e5 points, 80^3
+// cells, W = 12: 748 -> 537 us); nothing for W = 8 to 10 (2e6 points, 112^3 cells,
+// W = 9: 1786 us against 2320 with one) and in 2D (2e6 points, 640^2 cells, W = 5:
+// 174 against 255 us).
+template <int NDIM, int W> constexpr int dcoord_min_ctas() {
+  return NDIM < 3 || (W >= 8 && W <= 10) ? 0 : (W <= 7 ? 2 : 1);
+}
+
 template <typename T, typename Tc, int NDIM, int W>
-__global__ void __launch_bounds__(SP_THREADS)
+__global__ void __launch_bounds__(SP_THREADS, dcoord_min_ctas<NDIM, W>())
     k_interp_dcoord(PointsDesc pts, const Chunk *__restrict__ chunks,
                     const uint32_t *nchunks, Geometry g,
                     KernelPoly<T> kp, const cplx<T> *__restrict__ grid,

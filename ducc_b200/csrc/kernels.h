@@ -24,10 +24,11 @@ inline void allow_smem(K *kern, size_t bytes) {
 // tensor core (2D, quadrant): the point's quadrant within its tile and below it
 // the Morton code of its cell within the quadrant (2 * (log2tile - 1) bits);
 // runs: its bin of (2^bin_log2)^d cells within the tile (bin_bits), and in 3D
-// its first-axis position in the bin (the order of k_spread_run, k_spread_run3)
+// its position in the bin along the first cell_axes axes (the order of
+// k_spread_run, k_spread_run3)
 struct TileOrder {
   bool quadrant = false;
-  int bin_bits = 0, bin_log2 = 3;
+  int bin_bits = 0, bin_log2 = 3, cell_axes = 1;
 };
 int spread_run3_bin_log2(int W);
 void launch_fold_keys(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
