@@ -145,3 +145,57 @@ def test_smallest_grids(single, W, ndim):
     n = 2 * ((W + 1) // 2)
     _run(W, single, (2, 3, 2)[:ndim], (n, n, n + 2 if n + 2 != 14 else n)[:ndim], 200, "edges")
     _run(W, single, (2, 3, 2)[:ndim], (n,) * ndim, 200, "uniform")
+
+
+@pytest.mark.parametrize("W,nover,M", [(8, (36, 48, 20), 4500), (9, (36, 48, 20), 4500),
+                                       (10, (20, 40, 36), 4500), (11, (30, 40, 36), 35000),
+                                       (11, (110, 120, 126), 17000), (12, (126, 120, 128), 17000),
+                                       (13, (72, 70, 80), 17000), (14, (72, 70, 80), 17000),
+                                       (15, (90, 88, 80), 17000)])
+def test_3d_double_direct(W, nover, M):
+    """3D double-precision interpolation cell by cell (few points per bin, small
+    supports, and W = 11 with many points per bin)."""
+    _run(W, False, tuple(n // 2 - 3 for n in nover), nover, M, "uniform")
+    if M < 5000:
+        _run(W, False, tuple(n // 2 - 3 for n in nover), nover, M, "edges")
+
+
+@pytest.mark.parametrize("single,shape,M", [(True, (20, 24, 18), 3000), (True, (500,), 3000),
+                                            (False, (20, 24, 18), 3000),
+                                            (False, (20, 24, 18), 6000), (False, (40, 36), 3000)])
+@pytest.mark.parametrize("eps", [1e-2, 1e-5])
+def test_strided_unplanned(single, shape, M, eps):
+    """Unplanned calls read unsorted coordinates through their strides; values and
+    results may be strided as well."""
+    import torch
+    rng = np.random.default_rng(8)
+    ct = torch.complex64 if single else torch.complex128
+    nd = len(shape)
+    coord = rng.uniform(-np.pi, np.pi, (M, nd)).astype(np.float32 if single else np.float64)
+    vals = torch.from_numpy(rng.standard_normal((M, 2))).cuda().to(ct) + 1j
+    grid = torch.from_numpy(rng.standard_normal(shape)).cuda().to(ct) + 1j
+    c = torch.from_numpy(coord).cuda()
+    cs = torch.from_numpy(np.ascontiguousarray(coord.T)).cuda().T[:, :]
+    assert nd == 1 or not cs.is_contiguous()
+    kw = dict(forward=True, epsilon=eps)
+    ref = nufft.u2nu(grid=grid, coord=c, **kw)
+    out = torch.zeros((M, 3), dtype=ct, device="cuda")
+    nufft.u2nu(grid=grid, coord=cs, out=out[:, 1], **kw)
+    assert torch.equal(out[:, 1], ref) and not out[:, ::2].any()
+    u0 = nufft.nu2u(points=vals[:, 0].contiguous(), coord=c,
+                    out=torch.empty(shape, dtype=ct, device="cuda"), **kw)
+    u1 = nufft.nu2u(points=vals[:, 0], coord=cs,
+                    out=torch.empty(shape, dtype=ct, device="cuda"), **kw)
+    # (sums in another order)
+    assert torch.linalg.vector_norm(u1 - u0) <= 2 * eps * torch.linalg.vector_norm(u0)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "bin"])
+@pytest.mark.parametrize("W", range(4, 17))
+@pytest.mark.parametrize("single", [True, False])
+def test_1d(single, W, kind):
+    """1D: several points at a time (single precision, spread points) and one."""
+    if single and W > 8:
+        pytest.skip("no kernel of this support")
+    for M in (1, 70, 3000):
+        _run(W, single, (400,), (900,), M, kind)
