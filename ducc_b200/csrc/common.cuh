@@ -77,7 +77,14 @@ __host__ __device__ __forceinline__ double of_bits(uint64_t a) {
   return r;
 #endif
 }
-__host__ __device__ __forceinline__ double nan_f64() { return of_bits(0x7ff8000000000000ull); }
+// integer part of a that is not too large; 0 for a that is not a number
+__host__ __device__ __forceinline__ int to_int(double a) {
+#ifdef __CUDA_ARCH__
+  return __double2int_rz(a);
+#else
+  return a == a ? int(a) : 0;
+#endif
+}
 
 // ---------------------------------------------------------------------------
 // Coordinate fold: DUCC's Nufft_ancestor::getpix (src/ducc0/nufft/nufft.h:285-298)
@@ -92,20 +99,19 @@ __host__ __device__ __forceinline__ double nan_f64() { return of_bits(0x7ff80000
 //
 // For every x, i0 lies in [-nsafe, n + 1 - nsafe], nsafe = (W + 1) / 2: shift is
 // n + 1 - W / 2 and maxi0 is n + nsafe - W.  Tile keys, chunks and the cells that
-// a kernel touches rest on that.  An x that is not finite gets the cell of
-// position 0 and a frac that is not a number, so that its weights are not either.
+// a kernel touches rest on that.  An x that is not finite gets cell 0 and a frac
+// that is not a number, so that its weights are not either.
 // ---------------------------------------------------------------------------
 
 __host__ __device__ __forceinline__ void fold_f32(double x, double coordfct, int n, double shift,
                                                   int maxi0, int &i0, double &frac) {
   const double tmp = mul_rn(x, coordfct);
-  double f = add_rn(tmp, -floor(tmp));
-  const bool nan = !(f == f);
-  if (nan) f = 0.;
+  const double f = add_rn(tmp, -floor(tmp));
   const double tmp2 = mul_rn(f, double(n));
-  const int s = int(add_rn(tmp2, shift)) - n;
-  i0 = s < maxi0 ? s : maxi0;
-  frac = nan ? nan_f64() : fma(f, double(n), -double(i0));
+  int t = to_int(add_rn(tmp2, shift));
+  t = t > 0 ? t : n;   // (0 is not a number's; shift >= 3)
+  i0 = t - n < maxi0 ? t - n : maxi0;
+  frac = fma(f, double(n), -double(i0));
 }
 
 typedef unsigned __int128 u128;
@@ -140,9 +146,15 @@ __host__ __device__ __forceinline__ u128 round_sig(u128 v, bool sticky, int keep
   return r;
 }
 
-// the fold of a fractional position f in 128-bit integers (any f in [0, 1])
+// the fold of a fractional position f in 128-bit integers (any f in [0, 1], or not a
+// number)
 __host__ __device__ __noinline__ inline void fold_f64_int(double f, int n, double shift, int maxi0,
                                                           int *i0_, double *frac_) {
+  if (!(f == f)) {
+    *i0_ = 0;
+    *frac_ = f;
+    return;
+  }
   int i0;
   // exact f = mant * 2^e
   uint64_t bits = bits_of(f);
@@ -203,13 +215,11 @@ __host__ __device__ __forceinline__ double round64_magic(double a) {
 // and every following sum stays exact in two doubles as long as the operands'
 // exponents are within 38 of one another.  Where that, or the exponent of a sum
 // (its upper part a power of two), or the integer part (within 2^-29 of an
-// integer) is in doubt, the integer version decides.
+// integer) is in doubt, or f is not a number, the integer version decides.
 __host__ __device__ __forceinline__ void fold_f64(double x, double coordfct, int n, double shift,
                                                   int maxi0, int &i0, double &frac) {
   const double tmp = mul_rn(x, coordfct);
-  double f = add_rn(tmp, -floor(tmp));
-  const bool nan = !(f == f);
-  if (nan) f = 0.;
+  const double f = add_rn(tmp, -floor(tmp));
   const double dn = double(n);
   const double hi = mul_rn(f, dn), lo = fma(f, dn, -hi);
   const double m1 = round64_magic(hi);
@@ -218,7 +228,7 @@ __host__ __device__ __forceinline__ void fold_f64(double x, double coordfct, int
   const double ih = floor(hi), is = floor(shift);
   const double r = add_rn(add_rn(add_rn(hi, -ih), add_rn(shift, -is)), lo64);
   const double fr = floor(r);
-  const int k = int(ih) + (int(is) - n) + int(fr);
+  const int k = to_int(ih) + (int(is) - n) + to_int(fr);
   const double off = add_rn(r, -fr);
   bool ok = hi >= 0x1p-38 && (bits_of(hi) & 0x000fffffffffffffull) != 0 && off > 0x1p-29 &&
             off < 1. - 0x1p-29;
@@ -234,7 +244,6 @@ __host__ __device__ __forceinline__ void fold_f64(double x, double coordfct, int
   ok = ok && s > 0x1p-38 && (bits_of(s) & 0x000fffffffffffffull) != 0;
   frac = add_rn(s, l64);
   if (!ok) fold_f64_int(f, n, shift, maxi0, &i0, &frac);
-  if (nan) frac = nan_f64();
 }
 
 template <typename Tc>
