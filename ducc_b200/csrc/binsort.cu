@@ -448,9 +448,21 @@ void read_words(const uint32_t *const *src, int n, uint32_t *out, cudaStream_t s
   for (int i = 0; i < n; ++i) out[i] = h[i];
 }
 
+// the last k of [lo, hi] with pos[k] <= i, for ascending pos with pos[lo] <= i
+__device__ __forceinline__ uint32_t last_at_or_before(const uint32_t *pos, uint32_t lo, uint32_t hi,
+                                                      uint32_t i) {
+  while (lo < hi) {
+    const uint32_t mid = lo + (hi - lo + 1) / 2;
+    if (pos[mid] <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
 // The chunk list of up to CHUNK_TILES tiles: where every tile starts (a binary
-// search each), then one block counts, scans and writes.  Two launches over the
-// tiles instead of seven over the points.
+// search each), then one block counts, scans (into shared memory) and writes, one
+// thread per chunk, so that a tile with most of the points does not take longer.
+// Two launches over the tiles instead of seven over the points.
 constexpr uint32_t CHUNK_TILES = 16384;
 constexpr int CT_THREADS = 1024;
 
@@ -471,6 +483,7 @@ __global__ void __launch_bounds__(CT_THREADS)
     k_tile_chunks(const uint32_t *__restrict__ start, uint32_t ntiles, uint32_t chunk,
                   Chunk *__restrict__ chunks, uint32_t *__restrict__ count) {
   __shared__ uint32_t ws[32];
+  extern __shared__ uint32_t first[];   // first chunk of every tile
   const uint32_t per = (ntiles + CT_THREADS - 1) / CT_THREADS;
   const uint32_t t0 = min(ntiles, threadIdx.x * per), t1 = min(ntiles, t0 + per);
   uint32_t s = 0;
@@ -478,15 +491,18 @@ __global__ void __launch_bounds__(CT_THREADS)
   uint32_t tot;
   uint32_t pos = block_excl_scan(s, ws, &tot);
   for (uint32_t t = t0; t < t1; ++t) {
-    const uint32_t e = start[t + 1];
-    for (uint32_t b = start[t]; b < e; b += chunk) {
-      Chunk c;
-      c.start = b;
-      c.count = min(chunk, e - b);
-      c.tile = t;
-      c.pad = 0;
-      chunks[pos++] = c;
-    }
+    first[t] = pos;
+    pos += (start[t + 1] - start[t] + chunk - 1) / chunk;
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < tot; i += CT_THREADS) {
+    const uint32_t lo = last_at_or_before(first, 0, ntiles - 1, i);
+    Chunk c;
+    c.start = start[lo] + (i - first[lo]) * chunk;
+    c.count = min(chunk, start[lo + 1] - c.start);
+    c.tile = lo;
+    c.pad = 0;
+    chunks[i] = c;
   }
   if (threadIdx.x == 0) *count = tot;
 }
@@ -501,7 +517,9 @@ uint32_t build_chunks(const uint32_t *skeys, uint32_t n, int tile_shift, uint32_
     k_tile_starts<<<unsigned(ntiles / 256 + 1), 256, 0, st>>>(skeys, n, tile_shift,
                                                               uint32_t(ntiles), start);
     DN_LAUNCHED();
-    k_tile_chunks<<<1, CT_THREADS, 0, st>>>(start, uint32_t(ntiles), chunk, chunks, d_count);
+    allow_smem(k_tile_chunks, CHUNK_TILES * sizeof(uint32_t));
+    k_tile_chunks<<<1, CT_THREADS, size_t(ntiles) * sizeof(uint32_t), st>>>(
+        start, uint32_t(ntiles), chunk, chunks, d_count);
     DN_LAUNCHED();
   } else {
     uint32_t *flags = static_cast<uint32_t *>(ws);
@@ -679,36 +697,79 @@ const uint32_t *build_group_chunks(const uint32_t *start, uint32_t ntiles, int g
 // sorted positions of the points of groups [g0, g1), bin after bin: counts
 // per bin, then (after a scan into pos) the positions
 __global__ void k_gsel_count(const uint32_t *__restrict__ start, uint32_t nbins, int gbits,
-                             uint32_t g0, uint32_t g1, uint32_t *__restrict__ cnt) {
+                             uint32_t g0, uint32_t g1, uint32_t *__restrict__ cnt,
+                             uint32_t *__restrict__ nlarge) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *nlarge = 0;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nbins; t += gridDim.x * blockDim.x)
     cnt[t] = start[(uint64_t(t) << gbits) + g1] - start[(uint64_t(t) << gbits) + g0];
 }
 
-__global__ void k_gsel_fill(const uint32_t *__restrict__ start, const uint32_t *__restrict__ cnt,
-                            const uint32_t *__restrict__ pos, uint32_t nbins, int gbits,
-                            uint32_t g0, uint32_t *__restrict__ sel) {
-  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nbins;
-       t += gridDim.x * blockDim.x) {
-    const uint32_t s = start[(uint64_t(t) << gbits) + g0], n = cnt[t];
-    uint32_t *d = sel + pos[t];
-    for (uint32_t k = 0; k < n; ++k) d[k] = s + k;
+// One thread per bin writes the positions of a small bin, a warp those of a larger
+// one together; a bin of more than GSEL_LARGE is put on a list for the next launch,
+// where 32 CTAs share it.  (One thread for every bin took 21 ms instead of 9.6 for a
+// gridding call with most points in a few bins; a search for every position's bin 1 %
+// more than this for evenly spread points.)
+constexpr uint32_t GSEL_SMALL = 32, GSEL_LARGE = 2048, GSEL_SPLIT = 32;
+
+__global__ void k_gsel_fill(const uint32_t *__restrict__ start, const uint32_t *__restrict__ pos,
+                            uint32_t nbins, int gbits, uint32_t g0, uint32_t n,
+                            uint32_t *__restrict__ sel, uint32_t *__restrict__ nlarge,
+                            uint32_t *__restrict__ large) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t t0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); t0 < nbins;
+       t0 += gridDim.x * blockDim.x) {
+    const uint32_t t = t0 + lane;
+    uint32_t s = 0, p = 0, c = 0;
+    if (t < nbins) {
+      s = start[(uint64_t(t) << gbits) + g0];
+      p = pos[t];
+      c = (t + 1 < nbins ? pos[t + 1] : n) - p;
+    }
+    if (c <= GSEL_SMALL)
+      for (uint32_t k = 0; k < c; ++k) sel[p + k] = s + k;
+    else if (c > GSEL_LARGE)
+      large[atomicAdd(nlarge, 1u)] = t;
+    for (unsigned m = __ballot_sync(0xffffffffu, c > GSEL_SMALL && c <= GSEL_LARGE); m; m &= m - 1) {
+      const int l = __ffs(m) - 1;
+      const uint32_t ls = __shfl_sync(0xffffffffu, s, l), lp = __shfl_sync(0xffffffffu, p, l),
+                     lc = __shfl_sync(0xffffffffu, c, l);
+      for (uint32_t k = lane; k < lc; k += 32) sel[lp + k] = ls + k;
+    }
+  }
+}
+
+__global__ void k_gsel_large(const uint32_t *__restrict__ start, const uint32_t *__restrict__ pos,
+                             uint32_t nbins, int gbits, uint32_t g0, uint32_t n,
+                             uint32_t *__restrict__ sel, const uint32_t *__restrict__ nlarge,
+                             const uint32_t *__restrict__ large) {
+  const uint32_t nl = *nlarge;
+  for (uint32_t i = blockIdx.x; i < nl; i += gridDim.x) {
+    const uint32_t t = large[i], s = start[(uint64_t(t) << gbits) + g0], p = pos[t];
+    const uint32_t c = (t + 1 < nbins ? pos[t + 1] : n) - p;
+    for (uint64_t k = uint64_t(blockIdx.y) * blockDim.x + threadIdx.x; k < c;
+         k += gridDim.y * blockDim.x)
+      sel[p + k] = s + uint32_t(k);
   }
 }
 
 size_t group_select_workspace_bytes(uint32_t nbins) {
-  return size_t(2) * nbins * 4 + 256 + scan_workspace_bytes(nbins);
+  return size_t(2) * nbins * 4 + 4 + 256 + scan_workspace_bytes(nbins);
 }
 
 void build_group_select(const uint32_t *start, uint32_t nbins, int gbits, uint32_t g0, uint32_t g1,
-                        uint32_t *sel, void *ws, cudaStream_t st) {
-  uint32_t *cnt = static_cast<uint32_t *>(ws);
-  uint32_t *pos = cnt + nbins;
+                        uint32_t n, uint32_t *sel, void *ws, cudaStream_t st) {
+  if (n == 0) return;
+  uint32_t *cnt = static_cast<uint32_t *>(ws);   // the list of large bins after the scan
+  uint32_t *pos = cnt + nbins, *nlarge = pos + nbins;
   uint32_t *sws = reinterpret_cast<uint32_t *>(
-      (reinterpret_cast<uintptr_t>(pos + nbins) + 255) & ~uintptr_t(255));
-  k_gsel_count<<<grid_of(nbins), 256, 0, st>>>(start, nbins, gbits, g0, g1, cnt);
+      (reinterpret_cast<uintptr_t>(nlarge + 1) + 255) & ~uintptr_t(255));
+  k_gsel_count<<<grid_of(nbins), 256, 0, st>>>(start, nbins, gbits, g0, g1, cnt, nlarge);
   DN_LAUNCHED();
   exclusive_scan(cnt, pos, nbins, sws, st);
-  k_gsel_fill<<<grid_of(nbins), 256, 0, st>>>(start, cnt, pos, nbins, gbits, g0, sel);
+  k_gsel_fill<<<grid_of(nbins), 256, 0, st>>>(start, pos, nbins, gbits, g0, n, sel, nlarge, cnt);
+  DN_LAUNCHED();
+  k_gsel_large<<<dim3(64, GSEL_SPLIT), 256, 0, st>>>(start, pos, nbins, gbits, g0, n, sel, nlarge,
+                                                     cnt);
   DN_LAUNCHED();
 }
 

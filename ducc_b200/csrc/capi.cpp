@@ -2114,7 +2114,7 @@ static ChunkList grouped_chunks(GroupedPlan *gp, uint32_t g0, uint32_t g1, uint6
 static uint32_t grouped_select(GroupedPlan *gp, uint32_t g0, uint32_t g1, cudaStream_t st) {
   const uint32_t n = uint32_t(gp->run_points(g0, g1));
   if (n > 0 && (gp->g1 == 0 || gp->g0 != g0 || gp->g1 != g1)) {
-    build_group_select(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1,
+    build_group_select(gp->start.as<uint32_t>(), gp->ntiles, gp->gbits, g0, g1, n,
                        gp->sel.as<uint32_t>(), gp->cws.p, st);
     gp->g0 = g0;
     gp->g1 = g1;

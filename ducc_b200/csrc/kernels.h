@@ -74,11 +74,11 @@ const uint32_t *build_group_chunks(const uint32_t *start, uint32_t ntiles, int g
 void launch_scatter_coords(bool coord_f64, const void *sorted, int ndim, const uint32_t *perm,
                            uint32_t n, void *out, cudaStream_t st);
 
-// the points of groups [g0, g1) of a grouped index, in key order: their sorted
-// positions into sel (one entry per point)
+// the n points of groups [g0, g1) of a grouped index, in key order: their sorted
+// positions into sel
 size_t group_select_workspace_bytes(uint32_t nbins);
 void build_group_select(const uint32_t *start, uint32_t nbins, int gbits, uint32_t g0, uint32_t g1,
-                        uint32_t *sel, void *ws, cudaStream_t st);
+                        uint32_t n, uint32_t *sel, void *ws, cudaStream_t st);
 // counts[k] = number of points with group k < ngroups (counts zeroed first)
 void launch_group_counts(const uint32_t *group, uint32_t n, uint32_t ngroups, uint32_t *counts,
                          cudaStream_t st);

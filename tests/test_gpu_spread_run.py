@@ -199,3 +199,23 @@ def test_1d(single, W, kind):
         pytest.skip("no kernel of this support")
     for M in (1, 70, 3000):
         _run(W, single, (400,), (900,), M, kind)
+
+
+@pytest.mark.parametrize("shape,nover,W", [((400,), (900,), 7), ((3000,), (6480,), 5),
+                                           ((30, 40), (64, 90), 6)])
+def test_many_chunks_of_one_tile(shape, nover, W):
+    """Most points in one tile (some fifty chunks) and a few all over the grid."""
+    import torch
+    rng = np.random.default_rng(9)
+    M = 50000
+    coord = np.where(rng.random((M, 1)) < 0.99, rng.uniform(0.1, 0.12, (M, len(shape))),
+                     rng.uniform(-np.pi, np.pi, (M, len(shape)))).astype(np.float32)
+    p, k, nov, _, vals = _case(W, True, shape, nover, M, "uniform")
+    plan = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=shape,
+                      epsilon=1e-3, force_kernel=k, force_nover=nov)
+    grid = (rng.standard_normal(nov) + 1j * rng.standard_normal(nov)).astype(np.complex64)
+    out = plan.interp(grid=torch.from_numpy(grid).cuda()).cpu().numpy()
+    assert O.l2error(out, O.interpolate(p, grid, coord)) < 3e-6
+    got = plan.spread(points=torch.from_numpy(vals).cuda()).cpu().numpy()
+    # 5e4 values of size 1 summed in one order or another in a few cells
+    assert O.l2error(got, O.spread(p, coord, vals)) < 3e-6 + 50000 ** 0.5 * 2 ** -23

@@ -461,3 +461,27 @@ def test_plane_shares_sum_to_whole(ng, singleprec):
     # (the spreader's atomic additions come in a different order each call)
     assert O.l2error(ng.vis2dirty(vis=vis, npix_x=200, npix_y=200, planes=(0, 1), **args),
                      ng.vis2dirty(vis=vis, npix_x=200, npix_y=200, **args)) < tol
+
+
+@pmp("singleprec,epsilon", [(True, 1e-5), (False, 1e-9)])
+@pmp("fov", (2., 20.))
+def test_concentrated_baselines(ng, singleprec, epsilon, fov):
+    """Most visibilities in a few bins of the uv grid (short baselines), the others
+    far out: the position lists of the planes have bins with one point, with most of
+    them and with none."""
+    rng = np.random.default_rng(61)
+    nrow, nchan, npix = 3000, 2, 26
+    ps = fov * np.pi / 180 / npix
+    freq = 1e9 * (1 + 0.2 * np.arange(nchan))
+    umax = 0.4 * SPEEDOFLIGHT / (ps * freq[-1])
+    r, phi = umax * rng.random(nrow) ** 8, 2 * np.pi * rng.random(nrow)
+    uvw = np.stack([r * np.cos(phi), r * np.sin(phi), (2 * rng.random(nrow) - 1) * umax], 1)
+    ms = rng.random((nrow, nchan)) - 0.5 + 1j * (rng.random((nrow, nchan)) - 0.5)
+    dirty = rng.random((npix, npix)) - 0.5
+    if singleprec:
+        ms, dirty = ms.astype("c8"), dirty.astype("f4")
+    dirty2 = ng.ms2dirty(uvw, freq, ms, None, npix, npix, ps, ps, 0, 0, epsilon, True, 1, 0)
+    ref = O.explicit_gridder(uvw, freq, ms.astype("c16"), None, npix, npix, ps, ps, True, None)
+    assert O.l2error(dirty2, ref) <= epsilon
+    ms2 = ng.dirty2ms(uvw, freq, dirty, None, ps, ps, 0, 0, epsilon, True, 1, 0)
+    _adjoint_check(ms, dirty, dirty2.astype("f8"), ms2.astype("c16"), singleprec)
