@@ -1821,13 +1821,49 @@ struct Carver {
   char *base;
   size_t cap, used = 0;
   Carver(void *b, size_t c) : base(static_cast<char *>(b)), cap(c) {}
+  // null where the area is too small (used then says how large it has to be)
   void *take(size_t bytes) {
-    size_t off = (used + 255) & ~size_t(255);
-    if (off + bytes > cap) return nullptr;
+    const size_t off = (used + 255) & ~size_t(255);
     used = off + bytes;
-    return base + off;
+    return used <= cap ? base + off : nullptr;
+  }
+  bool fits() const { return used <= cap; }
+};
+
+// the temporaries of a type 1 transform in one area; chunks only where the
+// spreader works from them
+struct ScratchLayout {
+  double *cf[3] = {nullptr, nullptr, nullptr};
+  void *tw[3] = {nullptr, nullptr, nullptr};
+  uint32_t *keys = nullptr, *perm = nullptr, *count = nullptr;
+  void *rws = nullptr, *cws = nullptr, *grid = nullptr;
+  Chunk *chunks = nullptr;
+  ScratchLayout(const Setup &s, Carver &cv) {
+    const Geometry &g = s.g;
+    const uint32_t M = s.npoints;
+    const size_t csz = s.calc_f64 ? 16 : 8;
+    for (int d = 0; d < g.ndim; ++d) {
+      cf[d] = static_cast<double *>(cv.take(size_t(g.nuni[d] / 2 + 1) * sizeof(double)));
+      tw[d] = cv.take(size_t(g.nover[d]) * csz);
+    }
+    keys = static_cast<uint32_t *>(cv.take(size_t(M) * 4));
+    perm = static_cast<uint32_t *>(cv.take(size_t(M) * 4));
+    rws = cv.take(radix_workspace_bytes(M, s.keybits));
+    if (spread_needs_chunks(s)) {
+      const uint64_t maxchunks = std::min<uint64_t>(M, s.max_tiles) + M / s.chunk + 2;
+      cws = cv.take(chunk_workspace_bytes(M));
+      chunks = static_cast<Chunk *>(cv.take(size_t(maxchunks) * sizeof(Chunk)));
+      count = static_cast<uint32_t *>(cv.take(16));
+    }
+    grid = cv.take(grid_cells(g) * csz);
   }
 };
+
+static size_t scratch_needed(const Setup &s) {
+  Carver cv(nullptr, 0);
+  ScratchLayout l(s, cv);
+  return cv.used;
+}
 
 template <typename T>
 static void nu2u_scratch_typed(const Setup &s, const View &points, const View &coord,
@@ -1836,50 +1872,19 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
   const Geometry &g = s.g;
   const uint32_t M = s.npoints;
   const size_t csz = sizeof(T) * 2;
-  uint64_t maxchunks = std::min<uint64_t>(M, s.max_tiles) + M / s.chunk + 2;
   Carver cv(scratch, cap);
-  double *cf[3] = {nullptr, nullptr, nullptr};
-  void *tw[3] = {nullptr, nullptr, nullptr};
-  std::vector<double> corfac[3];
-  for (int d = 0; d < g.ndim; ++d) {
-    corfac[d] = corfac_of(s, d);
-    cf[d] = static_cast<double *>(cv.take(corfac[d].size() * sizeof(double)));
-    tw[d] = cv.take(size_t(g.nover[d]) * csz);
-  }
-  uint32_t *keys = static_cast<uint32_t *>(cv.take(size_t(M) * 4));
-  uint32_t *perm = static_cast<uint32_t *>(cv.take(size_t(M) * 4));
-  void *rws = cv.take(radix_workspace_bytes(M, s.keybits));
-  void *cws = cv.take(chunk_workspace_bytes(M));
-  Chunk *chunks = static_cast<Chunk *>(cv.take(size_t(maxchunks) * sizeof(Chunk)));
-  uint32_t *count = static_cast<uint32_t *>(cv.take(16));
-  void *grid = cv.take(grid_cells(g) * csz);
-  bool fits = grid != nullptr;
-  for (int d = 0; d < g.ndim; ++d) fits = fits && cf[d] && tw[d];
-  fits = fits && keys && perm && rws && cws && chunks && count;
-  if (!fits) {
-    // measure what would have been needed for the message
-    Carver probe(nullptr, ~size_t(0));
-    for (int d = 0; d < g.ndim; ++d) {
-      probe.take(corfac[d].size() * sizeof(double));
-      probe.take(size_t(g.nover[d]) * csz);
-    }
-    probe.take(size_t(M) * 4);
-    probe.take(size_t(M) * 4);
-    probe.take(radix_workspace_bytes(M, s.keybits));
-    probe.take(chunk_workspace_bytes(M));
-    probe.take(size_t(maxchunks) * sizeof(Chunk));
-    probe.take(16);
-    probe.take(grid_cells(g) * csz);
-    throw Error(ST_BADARG, "problem needs " + std::to_string(probe.used) +
-                               " bytes of scratch, more than the " + std::to_string(cap) +
-                               " bytes of the no-allocation scratch area");
-  }
+  const ScratchLayout l(s, cv);
+  DN_REQUIRE(cv.fits(), ST_BADARG,
+             "problem needs " + std::to_string(cv.used) + " bytes of scratch, more than the " +
+                 std::to_string(cap) + " bytes of the no-allocation scratch area");
   // constants: correction factors and FP64-accurate twiddles
   FFTAxisPlan ax[3];
+  std::vector<double> corfac[3];
   std::vector<std::vector<double>> hd(g.ndim);
   std::vector<std::vector<float>> hf(g.ndim);
   for (int d = 0; d < g.ndim; ++d) {
-    DN_CUDA(cudaMemcpyAsync(cf[d], corfac[d].data(), corfac[d].size() * sizeof(double),
+    corfac[d] = corfac_of(s, d);
+    DN_CUDA(cudaMemcpyAsync(l.cf[d], corfac[d].data(), corfac[d].size() * sizeof(double),
                             cudaMemcpyHostToDevice, st));
     const int n = int(g.nover[d]);
     if (sizeof(T) == 8) {
@@ -1889,7 +1894,7 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
         hd[d][2 * k] = std::cos(a);
         hd[d][2 * k + 1] = std::sin(a);
       }
-      DN_CUDA(cudaMemcpyAsync(tw[d], hd[d].data(), hd[d].size() * 8, cudaMemcpyHostToDevice, st));
+      DN_CUDA(cudaMemcpyAsync(l.tw[d], hd[d].data(), hd[d].size() * 8, cudaMemcpyHostToDevice, st));
     } else {
       hf[d].resize(2 * size_t(n));
       for (int k = 0; k < n; ++k) {
@@ -1897,33 +1902,34 @@ static void nu2u_scratch_typed(const Setup &s, const View &points, const View &c
         hf[d][2 * k] = float(std::cos(a));
         hf[d][2 * k + 1] = float(std::sin(a));
       }
-      DN_CUDA(cudaMemcpyAsync(tw[d], hf[d].data(), hf[d].size() * 4, cudaMemcpyHostToDevice, st));
+      DN_CUDA(cudaMemcpyAsync(l.tw[d], hf[d].data(), hf[d].size() * 4, cudaMemcpyHostToDevice, st));
     }
     ax[d].n = n;
     ax[d].nfac = int(s.factors[d].size());
     for (int i = 0; i < ax[d].nfac; ++i) ax[d].fac[i] = s.factors[d][i];
-    ax[d].tw = tw[d];
+    ax[d].tw = l.tw[d];
   }
-  // index: fold + stable sort by tile + chunks (1D, 3D); the stream is
-  // synchronised here (chunk count read-back), after which the host constant
-  // buffers may be released
-  launch_fold_keys(s.coord_f64, coord.data, coord.stride[0], coord.stride[1], M, g, keys, perm, st);
-  radix_sort_pairs(keys, perm, M, s.keybits, rws, st);
+  // index: fold + sort + (1D) chunks; the stream is synchronised here (in 1D by
+  // the read-back of the chunk count), after which the host constant buffers may
+  // be released
+  launch_fold_keys(s.coord_f64, coord.data, coord.stride[0], coord.stride[1], M, g, l.keys, l.perm,
+                   st, s.order);
+  radix_sort_pairs(l.keys, l.perm, M, s.keybits, l.rws, st);
   uint32_t nch = 0;
   if (spread_needs_chunks(s))
-    nch = build_chunks(keys, M, s.tile_shift, s.chunk, chunks, count, cws, st,
+    nch = build_chunks(l.keys, M, s.tile_shift, s.chunk, l.chunks, l.count, l.cws, st,
                        /*zero_copy=*/false);
   else
     DN_CUDA(cudaStreamSynchronize(st));
-  PointsDesc pts{coord.data, coord.stride[0], coord.stride[1], false, s.coord_f64, perm, M};
-  ChunkList cl{chunks, nch};
+  PointsDesc pts{coord.data, coord.stride[0], coord.stride[1], false, s.coord_f64, l.perm, M};
+  ChunkList cl{l.chunks, nch};
   // the scratch keeps the previous call's contents: the grid must start at zero
-  DN_CUDA(cudaMemsetAsync(grid, 0, grid_cells(g) * csz, st));
+  DN_CUDA(cudaMemsetAsync(l.grid, 0, grid_cells(g) * csz, st));
   const KernelPoly<T> &kp = *reinterpret_cast<const KernelPoly<T> *>(
       sizeof(T) == 4 ? static_cast<const void *>(&s.kpf) : static_cast<const void *>(&s.kpd));
-  launch_spread<T>(pts, cl, g, kp, points.data, points.stride[0], 0, grid, 0, 1, st);
-  const double *cfc[3] = {cf[0], cf[1], cf[2]};
-  fft_nu2u_tail<T>(grid, g, ax, forward, cfc, fft_order, out.data, out.stride, st);
+  launch_spread<T>(pts, cl, g, kp, points.data, points.stride[0], 0, l.grid, 0, 1, st);
+  const double *cfc[3] = {l.cf[0], l.cf[1], l.cf[2]};
+  fft_nu2u_tail<T>(l.grid, g, ax, forward, cfc, fft_order, out.data, out.stride, st);
 }
 
 static void nu2u_scratch_impl(const dnufft_array *points_, const dnufft_array *coord_, int forward,
@@ -1949,7 +1955,11 @@ static void nu2u_scratch_impl(const dnufft_array *points_, const dnufft_array *c
   DN_REQUIRE(out.dtype == points.dtype, ST_BADARG, "out must have the dtype of points");
   bool f64 = points.dtype == DNUFFT_C128;
   Setup s = make_setup(ndim, out.shape, uint64_t(points.shape[0]), eps, true, f64,
-                       coord.dtype == DNUFFT_F64, o);
+                       coord.dtype == DNUFFT_F64, o, true);
+  // a longer key may need a larger table of the sort: near the limit, sort by tile
+  if (scratch_needed(s) > cap)
+    s = make_setup(ndim, out.shape, uint64_t(points.shape[0]), eps, true, f64,
+                   coord.dtype == DNUFFT_F64, o);
   if (s.npoints == 0) {
     zero_view(out, st);
     return;

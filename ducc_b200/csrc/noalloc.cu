@@ -9,12 +9,10 @@
 // library: a file-scope device array of NOALLOC_SCRATCH_BYTES bytes, which
 // every GPU that loads the library holds until the process exits.
 //
-// The call waits on its stream once, part-way through, to read the number of
-// point chunks back to the host (a 4-byte copy into a host variable), and it
-// uploads the correction factors from host vectors; the host thread therefore
-// returns only after the sort has run on the GPU.
-#include <cuda_runtime.h>
-
+// The call waits on its stream once, part-way through: it uploads the correction
+// factors from host vectors, and in 1D it reads the number of point chunks back to
+// the host (a 4-byte copy into a host variable).  The host thread therefore returns
+// only after the sort has run on the GPU.
 #include <cuda_runtime.h>
 
 #include <mutex>

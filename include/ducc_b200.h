@@ -253,8 +253,8 @@ int dnufft_plan_get_permutation(const dnufft_plan *plan, uint32_t *out, void *st
  * The first call on a device looks up the area's address and keeps it for the
  * life of the process, so make that first call before any stream capture, and
  * do not call this entry point on a device after resetting it.  The call waits
- * on its stream once, part-way through, to read the number of point chunks
- * back to the host.  All calls share the one area and it keeps the previous
+ * on its stream once, part-way through, for the uploads of its constants (in 1D
+ * also to read a count back).  All calls share the one area and it keeps the previous
  * call's contents: calls that can overlap on the GPU (other streams, other
  * host threads) race, so serialise them.  Plain spreader only; 2D rows run in
  * the line FFT kernel. */

@@ -118,3 +118,27 @@ def test_noalloc_allocates_no_device_memory():
     s1, ref = call(L.dnufft_nu2u, coord, vals, shape, eps)
     assert s1 == 0
     assert O.l2error(arrays[1][2].cpu().numpy(), ref) < eps
+
+
+def test_noalloc_near_the_limit():
+    """A problem whose scratch holds the short sort keys' table (points sorted by
+    tile) and not the longer keys' (by bin inside the tile) is still taken."""
+    import torch
+    L = C.lib()
+    # 33,497,600 and 33,573,632 of 33,554,432 bytes
+    M, shape, nover = 200000, (40, 50), (1800, 2100)
+    coord, vals = problem(7, M, shape, np.float32, np.complex64)
+    k = [i for i, r in enumerate(O.kernel_db()) if r[0] == 6 and r[6] and r[5] == 2][0]
+    opts = C.make_opts(False, ndim=2, force_kernel=k, force_nover=nover)
+    dc, dv = torch.from_numpy(coord).cuda(), torch.from_numpy(vals).cuda()
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    res = []
+    for fn in (L.dnufft_nu2u, L.dnufft_nu2u_noalloc):
+        out = torch.full(shape, float("nan"), dtype=torch.complex64, device="cuda")
+        a = [C.describe(x) for x in (dv, dc, out)]
+        s = fn(ctypes.byref(a[0]), ctypes.byref(a[1]), 1, 1e-3, ctypes.byref(a[2]),
+               ctypes.byref(opts), st)
+        assert s == 0, L.dnufft_last_error()
+        torch.cuda.synchronize()
+        res.append(out.cpu().numpy())
+    assert O.l2error(res[1], res[0]) < 1e-5
