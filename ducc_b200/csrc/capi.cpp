@@ -10,6 +10,7 @@
 // C interface, julia/ducc_julia.cc:58-59); argument errors never launch kernels.
 #include "../../include/ducc_b200.h"
 
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -83,10 +84,42 @@ struct DevBuf {
 };
 
 // ---------------------------------------------------------------- device error word
-bool &bounded_wait_launched() {
-  static thread_local bool launched = false;
-  return launched;
+constexpr int MAX_DEVICES = 64;
+
+static int current_device() {
+  int dev = 0;
+  DN_CUDA(cudaGetDevice(&dev));
+  DN_REQUIRE(dev >= 0 && dev < MAX_DEVICES, ST_INTERNAL, "device index out of range");
+  return dev;
 }
+
+// has this host thread launched a bounded wait on the current device since it last
+// read the device's error word?
+static bool &bounded_wait_launched() {
+  static thread_local bool launched[MAX_DEVICES] = {false};
+  return launched[current_device()];
+}
+
+// is there a graph with a bounded wait of this device?
+static std::atomic<bool> g_wait_captured[MAX_DEVICES];
+
+void note_bounded_wait(cudaStream_t st) {
+  bounded_wait_launched() = true;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  DN_CUDA(cudaStreamIsCapturing(st, &cs));
+  if (cs != cudaStreamCaptureStatusNone) g_wait_captured[current_device()] = true;
+}
+
+// the bounded waits launched in its lifetime
+struct WaitScope {
+  bool &launched;
+  const bool before;
+  WaitScope() : launched(bounded_wait_launched()), before(launched) { launched = false; }
+  WaitScope(const WaitScope &) = delete;
+  WaitScope &operator=(const WaitScope &) = delete;
+  ~WaitScope() { launched = launched || before; }
+  bool any() const { return launched; }
+};
 
 void allow_smem_of(const void *kern, size_t bytes) {
   static std::mutex mu;
@@ -103,29 +136,25 @@ void allow_smem_of(const void *kern, size_t bytes) {
 // Kernels with bounded waits set this word instead of hanging; it is read back
 // after such a kernel (outside stream capture) and turned into ST_TIMEOUT.
 static int *device_error_word() {
-  static thread_local int dev_cached = -1;
-  static int *words[64] = {nullptr};
-  int dev = 0;
-  DN_CUDA(cudaGetDevice(&dev));
-  DN_REQUIRE(dev >= 0 && dev < 64, ST_INTERNAL, "device index out of range");
+  static int *words[MAX_DEVICES] = {nullptr};
+  const int dev = current_device();
   if (!words[dev]) {
     // word 0: error flag; word 1: scratch for the operand-scale reduction
     DN_CUDA(cudaMalloc(&words[dev], 4 * sizeof(int)));
     DN_CUDA(cudaMemset(words[dev], 0, 4 * sizeof(int)));
   }
-  dev_cached = dev;
   return words[dev];
 }
 
 // Every call ends here, waiting for its stream (plans share their grid between
 // calls on any streams; arrays may be reused once a call returns).  Only kernels
-// with bounded waits (marked by their launchers in bounded_wait_launched) can set
-// the word: without one there is nothing to read.
+// with bounded waits (note_bounded_wait) can set the word: without one in this call
+// and in any graph there is nothing to read.
 static void check_device_error(int *word, cudaStream_t st) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   DN_CUDA(cudaStreamIsCapturing(st, &cs));
   if (cs != cudaStreamCaptureStatusNone) return;
-  if (!bounded_wait_launched()) {
+  if (!bounded_wait_launched() && !g_wait_captured[current_device()]) {
     DN_CUDA(cudaStreamSynchronize(st));
     return;
   }
@@ -814,15 +843,15 @@ static void do_fft_interp(const Setup &s, const DevConst &dc, const PointsDesc &
   if (wb && !work.p) work = DevBuf(wb, st);
   int *err = device_error_word();
   tm.mark("correction + FFT");
-  if (side) {
-    DN_REQUIRE(ws && wk, ST_INTERNAL, "side-stream FFT without preallocated buffers");
+  bool fft_waits;
+  {
+    const WaitScope waits;
+    DN_REQUIRE(!side || (ws && wk), ST_INTERNAL, "side-stream FFT without preallocated buffers");
     fft_u2nu_head<T>(uni.data, uni.stride, s.g, dc.ax, forward, dc.cf, fft_order, grid.p,
-                     side->s, work.p, err);
-    side->merge();
-  } else {
-    fft_u2nu_head<T>(uni.data, uni.stride, s.g, dc.ax, forward, dc.cf, fft_order, grid.p, st,
-                     work.p, err);
+                     side ? side->s : st, work.p, err);
+    fft_waits = waits.any();
   }
+  if (side) side->merge();
   tm.mark("interpolation");
   const KernelPoly<T> &kp = *reinterpret_cast<const KernelPoly<T> *>(
       sizeof(T) == 4 ? static_cast<const void *>(&s.kpf) : static_cast<const void *>(&s.kpd));
@@ -837,7 +866,7 @@ static void do_fft_interp(const Setup &s, const DevConst &dc, const PointsDesc &
   // anyway (the same time per launch, and no tensor map for small grids)
   if (!done)
     launch_interp<T>(pts, cl, s.g, kp, grid.p, 0, out.data, out.stride[0], 0, 1, st,
-                     bounded_wait_launched() ? err : nullptr);
+                     fft_waits ? err : nullptr);
   tm.mark("output copy");
   if (check) check_device_error(err, st);
 }
@@ -2457,7 +2486,6 @@ int dnufft_selftest_wait_timeout(int64_t limit_ns, void *stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     int *err = dnufft::device_error_word();
     dnufft::launch_wait_selftest(err, (unsigned long long)limit_ns, st);
-    dnufft::bounded_wait_launched() = true;
     dnufft::check_device_error(err, st);
   })
 }

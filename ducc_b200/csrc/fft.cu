@@ -1147,7 +1147,7 @@ static bool run_rows_v3(cplx<T> *grid, int n, int nlines, int64_t rs, int Nk, bo
                                           out_kept ? 1 : 0, pp, static_cast<const cplx<T> *>(p.tw),
                                           full_tw, err);
   DN_LAUNCHED();
-  bounded_wait_launched() = true;
+  note_bounded_wait(st);
   return true;
 }
 

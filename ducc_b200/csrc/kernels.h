@@ -5,10 +5,11 @@
 
 namespace dnufft {
 
-// set by the launchers of kernels that wait on mbarriers with a time limit and
-// report through the device error word; per host thread, cleared where the word
-// is read back
-bool &bounded_wait_launched();
+// Called by the launchers of kernels that wait on mbarriers with a time limit and
+// report through the device error word: the word is read at the end of the call,
+// and where the launch is recorded into a graph, at the end of every later call on
+// the device (the graph may be replayed at any time, from any thread).
+void note_bounded_wait(cudaStream_t st);
 
 // Lets launches of kern on the current device use `bytes` of dynamic shared
 // memory.  The limit belongs to the kernel, not to the launch: it is only ever

@@ -555,7 +555,7 @@ void interp_w(const PointsDesc &pts, const ChunkList &cl, const Geometry &g,
                                     static_cast<const cplx<T> *>(grid), gtrans, static_cast<cplx<T> *>(out), os, otrans, map, tpitch,
                                     err);
   DN_LAUNCHED();
-  if (tpitch > 0) bounded_wait_launched() = true;
+  if (tpitch > 0) note_bounded_wait(st);
 }
 
 // W dispatch: float supports W 4..8, double 4..16 (the kernel table's ranges)

@@ -975,6 +975,7 @@ __global__ void k_wait_selftest(int *err, unsigned long long limit_ns) {
 void launch_wait_selftest(int *err, unsigned long long limit_ns, cudaStream_t st) {
   k_wait_selftest<<<1, 32, 0, st>>>(err, limit_ns);
   DN_LAUNCHED();
+  note_bounded_wait(st);
 }
 
 bool spread_tc_supported(const Geometry &g, bool calc_f64) {
@@ -998,12 +999,12 @@ void launch_spread_tc(const PointsDesc &pts, const TcBlocks &tb, const Geometry 
   {                                                                                             \
     auto kern = k_spread_tc<TC, WW>;                                                            \
     constexpr int smem = tc::smem_bytes<TC>();                                                  \
-    allow_smem(kern, smem);                                                                  \
+    allow_smem(kern, smem);                                                                     \
     kern<<<tb.groups, tc::THREADS, smem, st>>>(pts, tb.kblk, tb.range, g, kp,                   \
                                                static_cast<const float2 *>(values), vs, absmax, \
                                                static_cast<float2 *>(grid), err);               \
     DN_LAUNCHED();                                                                              \
-    bounded_wait_launched() = true;                                                             \
+    note_bounded_wait(st);                                                                      \
     return;                                                                                     \
   }
   if (pts.coord_f64) {

@@ -38,3 +38,49 @@ def test_bounded_wait_reports_timeout_and_context_survives():
     nufft.nu2u(points=vals, coord=coord, forward=True, epsilon=1e-5, out=out, spreader="tc")
     torch.cuda.synchronize()
     assert torch.isfinite(torch.view_as_real(out)).all()
+
+
+def test_timeout_in_a_replayed_graph_is_reported_by_the_next_call():
+    """A bounded wait recorded into a graph may give up at any replay: the next call
+    on the device reports it, also one that launches no such wait itself, from
+    another thread, and not just the first after the capture."""
+    import threading
+    import torch
+    L = C.lib()
+    rng = np.random.default_rng(0)
+    coord = torch.from_numpy(rng.uniform(-np.pi, np.pi, (500, 1))).cuda()
+    vals = torch.randn(500, dtype=torch.complex128, device="cuda")
+    out = torch.empty(60, dtype=torch.complex128, device="cuda")
+
+    def small_call():
+        nufft.nu2u(points=vals, coord=coord, forward=True, epsilon=1e-7, out=out)
+
+    small_call()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        status = L.dnufft_selftest_wait_timeout(2_000_000,
+                                                torch.cuda.current_stream().cuda_stream)
+    assert status == 0        # recorded, not run
+    small_call()
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        with pytest.raises(RuntimeError, match="bounded device-side wait"):
+            small_call()
+        small_call()
+    g.replay()
+    torch.cuda.synchronize()
+    err = []
+
+    def run():
+        try:
+            small_call()
+        except RuntimeError as e:
+            err.append(str(e))
+
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    assert len(err) == 1 and "bounded device-side wait" in err[0]
+    small_call()
+    assert torch.isfinite(torch.view_as_real(out)).all()
