@@ -591,17 +591,21 @@ struct DevConst {
 };
 
 static void upload_consts(const Setup &s, DevConst &dc, cudaStream_t st) {
+  // sources of the copies, alive until the stream has been synchronised
+  std::vector<double> cf[3], twd[3];
+  std::vector<float> twf[3];
   for (int d = 0; d < s.g.ndim; ++d) {
-    const std::vector<double> cf = corfac_of(s, d);
-    size_t nb = cf.size() * sizeof(double);
+    cf[d] = corfac_of(s, d);
+    size_t nb = cf[d].size() * sizeof(double);
     dc.corfac[d] = DevBuf(nb, st);
-    DN_CUDA(cudaMemcpyAsync(dc.corfac[d].p, cf.data(), nb, cudaMemcpyHostToDevice, st));
+    DN_CUDA(cudaMemcpyAsync(dc.corfac[d].p, cf[d].data(), nb, cudaMemcpyHostToDevice, st));
     dc.cf[d] = dc.corfac[d].as<double>();
     int n = int(s.g.nover[d]);
     size_t esz = s.calc_f64 ? 16 : 8;
     dc.tw[d] = DevBuf(size_t(n) * esz, st);
     if (s.calc_f64) {
-      std::vector<double> t(2 * size_t(n));
+      std::vector<double> &t = twd[d];
+      t.resize(2 * size_t(n));
       for (int k = 0; k < n; ++k) {
         double a = -2.0 * M_PI * double(k) / double(n);
         t[2 * k] = std::cos(a);
@@ -609,7 +613,8 @@ static void upload_consts(const Setup &s, DevConst &dc, cudaStream_t st) {
       }
       DN_CUDA(cudaMemcpyAsync(dc.tw[d].p, t.data(), t.size() * 8, cudaMemcpyHostToDevice, st));
     } else {
-      std::vector<float> t(2 * size_t(n));
+      std::vector<float> &t = twf[d];
+      t.resize(2 * size_t(n));
       for (int k = 0; k < n; ++k) {
         double a = -2.0 * M_PI * double(k) / double(n);
         t[2 * k] = float(std::cos(a));
@@ -623,7 +628,6 @@ static void upload_consts(const Setup &s, DevConst &dc, cudaStream_t st) {
     for (int i = 0; i < p.nfac; ++i) p.fac[i] = s.factors[d][i];
     p.tw = dc.tw[d].p;
   }
-  // host vectors must stay alive until the copies ran
   DN_CUDA(cudaStreamSynchronize(st));
 }
 
