@@ -21,6 +21,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "const_table.h"
 #include "dnufft_internal.h"
 #include "kernels.h"
 
@@ -631,48 +632,62 @@ static void upload_consts(const Setup &s, DevConst &dc, cudaStream_t st) {
   DN_CUDA(cudaStreamSynchronize(st));
 }
 
-// Constants of an unplanned call or a plan, shared by later calls and plans with
-// the same geometry on the same device: the upload (host cosines, pageable
-// copies and a stream synchronisation) then happens once.  Up to MAX_SHARED
-// geometries per process are kept (about the size of their twiddle tables
-// each) for the life of the process; beyond that a call uploads into the
-// caller's `local`.  An entry is complete (its stream was
-// synchronised) before it is published, so any stream may read it.
-static const DevConst &consts_for(const Setup &s, DevConst &local, cudaStream_t st) {
-  constexpr size_t MAX_SHARED = 32;
-  struct Key {
-    int dev, ndim, f64, W;
-    double beta, e0;
-    int64_t nover[3], nuni[3];
-    bool operator<(const Key &o) const {
-      return std::memcmp(this, &o, sizeof(Key)) < 0;
+struct ConstKey {
+  int dev, ndim, f64, W;
+  double beta, e0;
+  int64_t nover[3], nuni[3];
+  explicit ConstKey(const Setup &s) {
+    std::memset(this, 0, sizeof(*this));   // padding bytes take part in the comparison
+    dev = current_device();
+    ndim = s.g.ndim;
+    f64 = s.calc_f64 ? 1 : 0;
+    W = s.g.W;
+    beta = s.beta;
+    e0 = s.e0;
+    for (int d = 0; d < s.g.ndim; ++d) {
+      nover[d] = s.g.nover[d];
+      nuni[d] = s.g.nuni[d];
     }
-  };
-  Key k;
-  std::memset(&k, 0, sizeof(k));   // padding bytes take part in the comparison
-  DN_CUDA(cudaGetDevice(&k.dev));
-  k.ndim = s.g.ndim;
-  k.f64 = s.calc_f64 ? 1 : 0;
-  k.W = s.g.W;
-  k.beta = s.beta;
-  k.e0 = s.e0;
-  for (int d = 0; d < s.g.ndim; ++d) {
-    k.nover[d] = s.g.nover[d];
-    k.nuni[d] = s.g.nuni[d];
   }
-  static std::mutex mu;
-  static std::map<Key, DevConst *> *cache = new std::map<Key, DevConst *>();   // never freed
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = cache->find(k);
-  if (it != cache->end()) return *it->second;
-  if (cache->size() >= MAX_SHARED) {
-    upload_consts(s, local, st);
-    return local;
-  }
-  DevConst *dc = new DevConst();   // kept until exit (not destroyed: no frees at teardown)
-  upload_consts(s, *dc, st);
-  (*cache)[k] = dc;
-  return *dc;
+  bool operator<(const ConstKey &o) const { return std::memcmp(this, &o, sizeof(ConstKey)) < 0; }
+};
+
+using Consts = ConstTable<ConstKey, DevConst>;
+
+static Consts &const_table() {
+  static Consts *t = new Consts();   // never destroyed: no frees at teardown
+  return *t;
+}
+
+static DevConst *make_consts(const Setup &s, cudaStream_t st) {
+  auto dc = std::make_unique<DevConst>();
+  upload_consts(s, *dc, st);   // (synchronises st: any stream may read it then)
+  return dc.release();
+}
+
+// The upload (host cosines, pageable copies and a stream synchronisation) happens
+// once per geometry; local: of a call for which the table has no place.
+static const DevConst &consts_for(const Setup &s, DevConst &local, cudaStream_t st) {
+  const ConstKey k(s);
+  if (const DevConst *dc = const_table().for_call(k, k.dev, [&] { return make_consts(s, st); }))
+    return *dc;
+  upload_consts(s, local, st);
+  return local;
+}
+
+// buffers go back to the pool in the order of st
+static void free_consts_on(DevConst &dc, cudaStream_t st) {
+  for (int d = 0; d < 3; ++d) dc.corfac[d].st = dc.tw[d].st = st;
+}
+
+static Consts::Ptr consts_for_plan(const Setup &s, cudaStream_t st) {
+  const ConstKey k(s);
+  return const_table().for_plan(
+      k, k.dev, [&] { return make_consts(s, st); }, [&](DevConst &dc) { free_consts_on(dc, st); });
+}
+
+static void release_consts(Consts::Ptr &p) {
+  const_table().release(p, [](DevConst &dc) { free_consts_on(dc, nullptr); });
 }
 
 // index: tile permutation, sorted keys and chunk list
@@ -1287,8 +1302,7 @@ struct PlanGroup {
 
 struct dnufft_plan {
   dnufft::Setup s;
-  dnufft::DevConst own;                      // constants where the shared ones are full
-  const dnufft::DevConst *dc = nullptr;
+  dnufft::Consts::Ptr dc;
   dnufft::Index ix;
   dnufft::DevBuf sorted_coord;
   dnufft::DevBuf grid;   // oversampled grid, allocated on first execution
@@ -1296,6 +1310,12 @@ struct dnufft_plan {
   std::vector<dnufft::PlanGroup> groups;   // host-coordinate plans with many points
   dnufft_opts o;
   int device = 0;
+  dnufft_plan() = default;
+  dnufft_plan(const dnufft_plan &) = delete;
+  dnufft_plan &operator=(const dnufft_plan &) = delete;
+  ~dnufft_plan() {
+    if (dc) dnufft::release_consts(dc);
+  }
 };
 
 namespace dnufft {
@@ -1315,7 +1335,7 @@ static void plan_create_impl(int nu2u, const dnufft_array *coord_, const int64_t
   p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o, true,
                     f64 ? CELL_DIGIT_F64 : CELL_DIGIT_F32);
   DN_CUDA(cudaGetDevice(&p->device));
-  p->dc = &consts_for(p->s, p->own, st);
+  p->dc = consts_for_plan(p->s, st);
   if (p->s.npoints > 0) {
     Staged sc(coord, true, false, st);
     build_index(p->s, sc.dev, p->ix, st);
@@ -2408,7 +2428,6 @@ int dnufft_plan_destroy(dnufft_plan *plan) {
       plan->sorted_coord.st = st;
       plan->grid.st = st;
       plan->work.st = st;
-      for (int d = 0; d < 3; ++d) plan->own.corfac[d].st = plan->own.tw[d].st = st;
       for (auto &pg : plan->groups) {
         pg.ix.perm.st = pg.ix.chunks.st = pg.ix.count.st = pg.ix.keys.st = st;
         pg.ix.kblk.st = pg.ix.kbrange.st = st;
