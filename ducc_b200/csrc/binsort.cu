@@ -24,7 +24,8 @@ namespace dnufft {
 template <typename Tc, int NDIM>
 __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t cs1,
                             uint32_t npts, Geometry g, uint32_t *__restrict__ keys,
-                            uint32_t *__restrict__ idx, TileOrder order) {
+                            uint32_t *__restrict__ idx, TileOrder order,
+                            const uint32_t *__restrict__ to) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= npts) return;
   int t[NDIM];
@@ -79,18 +80,19 @@ __global__ void k_fold_keys(const Tc *__restrict__ coord, int64_t cs0, int64_t c
                   (b >> ss) * uint32_t(g.ntiles[2]) + (c >> ss);
     key = (hi << (3 * ss)) | low;
   }
-  keys[i] = key;
-  idx[i] = i;
+  const uint32_t j = to ? to[i] : i;
+  keys[j] = key;
+  idx[j] = j;
 }
 
 void launch_fold_keys(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
                       uint32_t npts, const Geometry &g, uint32_t *keys, uint32_t *idx,
-                      cudaStream_t st, TileOrder order) {
+                      cudaStream_t st, TileOrder order, const uint32_t *to) {
   if (npts == 0) return;
   dim3 block(256), grid((npts + 255) / 256);
 #define FK(TC, ND) \
   k_fold_keys<TC, ND><<<grid, block, 0, st>>>((const TC *)coord, cs0, cs1, npts, g, keys, idx, \
-                                               order)
+                                               order, to)
   if (coord_f64) {
     if (g.ndim == 1) FK(double, 1); else if (g.ndim == 2) FK(double, 2); else FK(double, 3);
   } else {
@@ -570,27 +572,6 @@ void launch_gather_coords(bool coord_f64, const void *coord, int64_t cs0, int64_
   else
     k_gather_coords<float><<<g, 256, 0, st>>>((const float *)coord, cs0, cs1, ndim, perm, n,
                                               (float *)out);
-  DN_LAUNCHED();
-}
-
-// inverse of the gather: out[perm[i]] = sorted[i]
-template <typename Tc>
-__global__ void k_scatter_coords(const Tc *__restrict__ sorted, int ndim,
-                                 const uint32_t *__restrict__ perm, uint32_t n, Tc *__restrict__ out) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t j = perm[i];
-  for (int d = 0; d < ndim; ++d) out[uint64_t(j) * ndim + d] = sorted[uint64_t(i) * ndim + d];
-}
-
-void launch_scatter_coords(bool coord_f64, const void *sorted, int ndim, const uint32_t *perm,
-                           uint32_t n, void *out, cudaStream_t st) {
-  if (n == 0) return;
-  unsigned g = (n + 255) / 256;
-  if (coord_f64)
-    k_scatter_coords<double><<<g, 256, 0, st>>>((const double *)sorted, ndim, perm, n, (double *)out);
-  else
-    k_scatter_coords<float><<<g, 256, 0, st>>>((const float *)sorted, ndim, perm, n, (float *)out);
   DN_LAUNCHED();
 }
 

@@ -2471,24 +2471,19 @@ int dnufft_plan_get_permutation(const dnufft_plan *p, uint32_t *out, void *strea
       DN_CUDA(cudaMemcpyAsync(out, p->ix.perm.p, size_t(p->s.npoints) * 4, cudaMemcpyDefault, st));
     } else {
       // the plan processes points in an order of its own inside every tile;
-      // DUCC's permutation is the stable order by tile alone: re-sort the
-      // original coordinates
+      // DUCC's permutation is the stable order by tile alone: the tile keys, put
+      // back to the caller's order, sorted again
       dnufft::Setup s2 = p->s;
-      s2.qbits = false;
       s2.order = dnufft::TileOrder();
       s2.keybits = s2.ducc_keybits;
-      s2.chunk = dnufft::CHUNK;
       const uint32_t M = s2.npoints;
       const int nd = s2.g.ndim;
-      // sorted coordinates in original order: scatter back through perm
       dnufft::Index ix2;
       ix2.perm = dnufft::DevBuf(size_t(M) * 4, st);
       ix2.keys = dnufft::DevBuf(size_t(M) * 4, st);
-      dnufft::DevBuf orig(size_t(M) * nd * (s2.coord_f64 ? 8 : 4), st);
-      dnufft::launch_scatter_coords(s2.coord_f64, p->sorted_coord.p, nd, p->ix.perm.as<uint32_t>(),
-                                    M, orig.p, st);
-      dnufft::launch_fold_keys(s2.coord_f64, orig.p, nd, 1, M, s2.g, ix2.keys.as<uint32_t>(),
-                               ix2.perm.as<uint32_t>(), st);
+      dnufft::launch_fold_keys(s2.coord_f64, p->sorted_coord.p, nd, 1, M, s2.g,
+                               ix2.keys.as<uint32_t>(), ix2.perm.as<uint32_t>(), st, s2.order,
+                               p->ix.perm.as<uint32_t>());
       dnufft::DevBuf ws(dnufft::radix_workspace_bytes(M, s2.keybits), st);
       dnufft::radix_sort_pairs(ix2.keys.as<uint32_t>(), ix2.perm.as<uint32_t>(), M, s2.keybits,
                                ws.p, st);

@@ -32,9 +32,11 @@ struct TileOrder {
   int bin_bits = 0, bin_log2 = 3, cell_axes = 1;
 };
 int spread_run3_bin_log2(int W);
+// the key of point i and its index j, at place j = to[i] (i where to is null)
 void launch_fold_keys(bool coord_f64, const void *coord, int64_t cs0, int64_t cs1,
                       uint32_t npts, const Geometry &g, uint32_t *keys, uint32_t *idx,
-                      cudaStream_t st, TileOrder order = TileOrder());
+                      cudaStream_t st, TileOrder order = TileOrder(),
+                      const uint32_t *to = nullptr);
 // bits of the within-quadrant cell order in a tensor-core sort key
 inline int tc_cell_bits(const Geometry &g) { return 2 * (g.log2tile - 1); }
 size_t scan_workspace_bytes(uint64_t n);
@@ -71,9 +73,6 @@ size_t group_chunk_workspace_bytes(uint32_t ntiles);
 const uint32_t *build_group_chunks(const uint32_t *start, uint32_t ntiles, int gbits, uint32_t g0,
                             uint32_t g1, uint32_t chunk, Chunk *chunks, void *ws,
                             cudaStream_t st);
-
-void launch_scatter_coords(bool coord_f64, const void *sorted, int ndim, const uint32_t *perm,
-                           uint32_t n, void *out, cudaStream_t st);
 
 // the n points of groups [g0, g1) of a grouped index, in key order: their sorted
 // positions into sel
