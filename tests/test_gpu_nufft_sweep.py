@@ -149,7 +149,8 @@ def test_nufft_3d(nx, ny, nz, npoints, epsilon, forward, singleprec, periodicity
 def test_nufft_2d_tensor_core_spreader(nx, ny, npoints, epsilon, forward, periodicity,
                                        fft_order):
     """The single-precision 2D cases of the sweep with the tensor-core
-    spreader forced (the automatic choice is the plain one): the same criterion against the direct sum, unplanned and planned."""
+    spreader forced (the automatic choice is the plain one): the same criterion
+    against the direct sum, unplanned and planned."""
     shape = (nx, ny)
     uvw, ms, dirty = case_data(shape, npoints, periodicity, True)
     # float64 coordinates with complex64 values, as the reference's single

@@ -2,8 +2,8 @@
 groups whose host->device copies (and, for type 2, device->host copies of the
 results) overlap the sorting and spreading / interpolation of the other
 groups.  Checked against the same calls on device arrays (one group, no
-overlap), in complex64 and complex128, both signs, and against the direct NUDFT on a sample of
-modes / points.
+overlap), in complex64 (both spreaders) and complex128, both signs, and against
+the direct NUDFT on a sample of modes / points.
 """
 import numpy as np
 import pytest
@@ -17,8 +17,8 @@ M = 5_000_000          # above the pipelining threshold (4M points): 2 groups
 SHAPE = (320, 288)
 
 
-@pytest.mark.parametrize("single", [True, False])
-def test_pipelined_host_calls_match_device_calls(single):
+@pytest.mark.parametrize("single,spreader", [(True, "plain"), (True, "tc"), (False, "auto")])
+def test_pipelined_host_calls_match_device_calls(single, spreader):
     import torch
     rng = np.random.default_rng(11)
     cdt, vdt = (np.float32, np.complex64) if single else (np.float64, np.complex128)
@@ -31,9 +31,11 @@ def test_pipelined_host_calls_match_device_calls(single):
     for forward in (True, False):
         # type 1
         h_out = np.zeros(SHAPE, vdt)
-        nufft.nu2u(points=vals, coord=coord, forward=forward, epsilon=eps, out=h_out)
+        nufft.nu2u(points=vals, coord=coord, forward=forward, epsilon=eps, out=h_out,
+                   spreader=spreader)
         d_out = torch.zeros(SHAPE, dtype=dv.dtype, device="cuda")
-        nufft.nu2u(points=dv, coord=dc, forward=forward, epsilon=eps, out=d_out)
+        nufft.nu2u(points=dv, coord=dc, forward=forward, epsilon=eps, out=d_out,
+                   spreader=spreader)
         assert O.l2error(h_out, d_out.cpu().numpy()) < tol
         # a few modes against the direct sum over all points
         s = -1 if forward else 1

@@ -22,19 +22,22 @@ def _problem(ndim, M, single, seed):
     return coord, vals
 
 
-CASES = [((256, 240), 400_000, True, 1e-6),     # dense
-         ((96, 80), 30_000, True, 1e-5),        # plain
-         ((96, 80), 30_000, False, 1e-11),
-         ((400,), 20_000, False, 1e-10),
-         ((24, 20, 16), 20_000, True, 1e-5)]
+CASES = [((256, 240), 400_000, True, 1e-6, "tc"),
+         ((256, 240), 400_000, True, 1e-6, "plain"),
+         ((96, 80), 30_000, True, 1e-5, "tc"),
+         ((96, 80), 30_000, True, 1e-5, "plain"),
+         ((96, 80), 30_000, False, 1e-11, "auto"),
+         ((400,), 20_000, False, 1e-10, "auto"),
+         ((24, 20, 16), 20_000, True, 1e-5, "auto")]
 
 
-@pytest.mark.parametrize("shape,M,single,eps", CASES)
-def test_halves_equal_one_piece(shape, M, single, eps):
+@pytest.mark.parametrize("shape,M,single,eps,spreader", CASES)
+def test_halves_equal_one_piece(shape, M, single, eps, spreader):
     import torch
     coord, vals = _problem(len(shape), M, single, 3)
     dc, dv = torch.from_numpy(coord).cuda(), torch.from_numpy(vals).cuda()
-    p = nufft.plan(nu2u=True, coord=dc, grid_shape=shape, epsilon=eps)
+    p = nufft.plan(nu2u=True, coord=dc, grid_shape=shape, epsilon=eps, spreader=spreader)
+    assert (p.info()["tc_records"] > 0) == (spreader == "tc")
     for forward in (True, False):
         ref = p.nu2u(points=dv, forward=forward).cpu().numpy()
         g = p.spread(points=dv)
@@ -44,8 +47,8 @@ def test_halves_equal_one_piece(shape, M, single, eps):
         assert O.l2error(got, ref) < (1e-6 if single else 1e-14)
 
 
-@pytest.mark.parametrize("shape,M,single,eps", CASES)
-def test_two_shards_sum_to_whole(shape, M, single, eps):
+@pytest.mark.parametrize("shape,M,single,eps,spreader", CASES)
+def test_two_shards_sum_to_whole(shape, M, single, eps, spreader):
     import torch
     coord, vals = _problem(len(shape), M, single, 4)
     k, n = nufft.find_parameters(nu2u=True, grid_shape=shape, npoints=M, epsilon=eps,
@@ -55,10 +58,10 @@ def test_two_shards_sum_to_whole(shape, M, single, eps):
     for sl in (slice(0, cut), slice(cut, M)):
         dc = torch.from_numpy(np.ascontiguousarray(coord[sl])).cuda()
         parts.append((nufft.plan(nu2u=True, coord=dc, grid_shape=shape, epsilon=eps,
-                                 force_kernel=k, force_nover=n),
+                                 force_kernel=k, force_nover=n, spreader=spreader),
                       torch.from_numpy(np.ascontiguousarray(vals[sl])).cuda()))
     whole = nufft.plan(nu2u=True, coord=torch.from_numpy(coord).cuda(), grid_shape=shape,
-                       epsilon=eps, force_kernel=k, force_nover=n)
+                       epsilon=eps, force_kernel=k, force_nover=n, spreader=spreader)
     g = parts[0][0].spread(points=parts[0][1])
     g += parts[1][0].spread(points=parts[1][1])
     got = parts[0][0].grid_to_uniform(forward=True, grid=g).cpu().numpy()
@@ -67,7 +70,8 @@ def test_two_shards_sum_to_whole(shape, M, single, eps):
     # against the direct sum over a sample of points (all modes)
     sub = slice(0, 2000)
     p_sub = nufft.plan(nu2u=True, coord=torch.from_numpy(np.ascontiguousarray(coord[sub])).cuda(),
-                       grid_shape=shape, epsilon=eps, force_kernel=k, force_nover=n)
+                       grid_shape=shape, epsilon=eps, force_kernel=k, force_nover=n,
+                       spreader=spreader)
     ga = p_sub.spread(points=torch.from_numpy(np.ascontiguousarray(vals[sub])).cuda())
     got_sub = p_sub.grid_to_uniform(forward=True, grid=ga).cpu().numpy()
     exact = O.direct_nu2u(coord[sub].astype(np.float64), vals[sub].astype(np.complex128), shape,
