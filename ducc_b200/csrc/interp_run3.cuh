@@ -208,7 +208,7 @@ void interp_run3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<do
   const uint32_t ppb =
       per >= R::BATCH ? R::BATCH * uint32_t(std::min<uint64_t>(16, per / R::BATCH))
                       : std::max<uint32_t>(16, uint32_t(per) & ~15u);
-  dim3 grd((pts.npts + ppb - 1) / ppb, ntrans);
+  dim3 grd(unsigned((uint64_t(pts.npts) + ppb - 1) / ppb), ntrans);
   kern<<<grd, R::THREADS, R::SMEM, st>>>(pts, ppb, g, kp, static_cast<const double2 *>(grid),
                                          gtrans, static_cast<double2 *>(out), os, otrans);
   DN_LAUNCHED();
@@ -521,7 +521,7 @@ void interp_run3f_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<f
   const uint32_t ppb =
       per >= R::BATCH ? R::BATCH * uint32_t(std::min<uint64_t>(8, per / R::BATCH))
                       : std::max<uint32_t>(16, uint32_t(per) & ~15u);
-  dim3 grd((pts.npts + ppb - 1) / ppb, ntrans);
+  dim3 grd(unsigned((uint64_t(pts.npts) + ppb - 1) / ppb), ntrans);
   kern<<<grd, R::THREADS, R::SMEM, st>>>(pts, ppb, g, kp, static_cast<const float2 *>(grid),
                                          gtrans, static_cast<float2 *>(out), os, otrans);
   DN_LAUNCHED();

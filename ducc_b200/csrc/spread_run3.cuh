@@ -341,7 +341,7 @@ void spread_run3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly<T>
   const uint32_t ppb =
       per >= R::BATCH ? R::BATCH * uint32_t(std::min<uint64_t>(8, per / R::BATCH))
                       : std::max<uint32_t>(16, uint32_t(per) & ~15u);
-  dim3 grd((pts.npts + ppb - 1) / ppb, ntrans);
+  dim3 grd(unsigned((uint64_t(pts.npts) + ppb - 1) / ppb), ntrans);
   kern<<<grd, R::THREADS, R::SMEM, st>>>(pts, ppb, g, kp, static_cast<const cplx<T> *>(values), vs,
                                          vtrans, static_cast<cplx<T> *>(grid), gtrans);
   DN_LAUNCHED();
