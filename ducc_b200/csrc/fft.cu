@@ -688,8 +688,8 @@ static bool run_lines2(cplx<T> *grid, LineSpec ls, const FFTAxisPlan &p, const U
 // ---------------------------------------------------------------------------
 // FFT v3 for 2D grids.
 //
-// Rows (the contiguous axis): a persistent kernel, one CTA per SM, walks its
-// rows with three shared-memory line buffers: the next row is fetched by a TMA
+// Rows (the contiguous axis): a persistent kernel, one to four CTAs per SM (more for
+// shorter rows, run_rows_v3), walks its rows with three shared-memory line buffers: the next row is fetched by a TMA
 // bulk copy (cp.async.bulk, completion on an mbarrier) while the current one
 // runs its Stockham stages (ping-pong between the other two buffers), and the
 // result is written back by bulk stores.  Kept ranges (type 1 output, type 2

@@ -1,13 +1,14 @@
 // Plain spreading (type 1, 1D; 2D and 3D: spread_run.cuh, spread_run3.cuh) and
 // interpolation (type 2, 1D and single precision; 2D double: interp_run.cuh, 3D
-// where interp3_in_windows: interp_run3.cuh) kernels.
+// double and where interp3_in_windows: interp_run3.cuh) kernels.
 //
 // One CTA per chunk of tile-sorted points (at most CHUNK points of one tile).
 // Spreading: every warp takes 32 points at a time, each lane folds its point
 // and evaluates the W weights by Horner in registers, stages them in shared
 // memory, then the warp walks the 32 points, W lanes covering the W cells of a
-// point, 32 / W points together, adding into a shared-memory copy of the tile plus halo
-// with shared-memory atomics.  The tile buffer is flushed once with vectorised
+// point (32 / W points together in single precision), adding into a shared-memory
+// copy of the tile plus halo with shared-memory atomics; points within a few cells
+// are summed in registers first.  The tile buffer is flushed once with vectorised
 // global atomics at wrapped grid positions.
 // Interpolation: the tile plus halo is staged in shared memory and every thread
 // evaluates one point (weights in registers, W^d multiply-adds), writing the

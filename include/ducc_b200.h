@@ -45,7 +45,7 @@ extern "C" {
 /* spreader selection (type 1) */
 /* AUTO: plain (measured faster than the tensor-core form everywhere) */
 #define DNUFFT_SPREAD_AUTO 0
-#define DNUFFT_SPREAD_PLAIN 1  /* FP32/FP64 sums, in registers (2D) or shared memory */
+#define DNUFFT_SPREAD_PLAIN 1  /* FP32/FP64 sums in registers (2D, 3D) or shared memory */
 #define DNUFFT_SPREAD_TC 2     /* split-precision FP16 tcgen05 tile contraction  */
 
 typedef struct dnufft_array {
