@@ -4,7 +4,9 @@
 // Unplanned calls: the first KEPT geometries are kept for the life of the process
 // (a captured graph of a call may use them at any time); beyond that a call makes
 // its own.  Plans: an entry is shared with the calls' and the other plans' of the
-// same geometry; the last RECENT ones of a device are kept for plans to come and the
+// same geometry; the last RECENT ones of a device are kept for plans to come (about
+// 16 bytes per cell of the oversampled axes each; a batch of 64 different plans that
+// is made again and again finds all of its own) and the
 // oldest is given up first, freed when no plan holds it any more.  Plans take no
 // place of the calls': a program that makes many different plans does not make its
 // unplanned calls upload every time.
@@ -23,7 +25,7 @@ namespace dnufft {
 // use it at once).  drop(V &): called before the last reference to an entry goes.
 template <typename Key, typename V> class ConstTable {
  public:
-  static constexpr size_t KEPT = 32, RECENT = 32;
+  static constexpr size_t KEPT = 32, RECENT = 128;
   using Ptr = std::shared_ptr<V>;
 
   // for an unplanned call; null: no place left

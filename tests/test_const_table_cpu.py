@@ -27,13 +27,13 @@ int main() {
   auto mk = [&](int k) { return [&made, k] { ++made; return new V{k}; }; };
   auto drop = [&](V &v) { dropped.insert(v.k); };
   // many plans, all destroyed again
-  for (int k = 0; k < 200; ++k) {
+  for (int k = 0; k < 400; ++k) {
     T::Ptr p = t.for_plan(k, 0, mk(k), drop);
     CHECK(p->k == k);
     t.release(p, drop);
     CHECK(!p);
   }
-  CHECK(made == 200 && dropped.size() == 200 - T::RECENT);
+  CHECK(made == 400 && dropped.size() == 400 - T::RECENT);
   // new geometries of unplanned calls are kept all the same, for good
   const V *first = nullptr;
   for (int r = 0; r < 3; ++r)
@@ -41,8 +41,8 @@ int main() {
       const V *v = t.for_call(k, 0, mk(k));
       CHECK(v && v->k == k);
       if (k == 1000) { CHECK(!first || v == first); first = v; }
-      for (int j = 0; j < 40; ++j) {
-        T::Ptr p = t.for_plan(2000 + (r * 7 + j), 0, mk(2000), drop);
+      for (int j = 0; j < 150; ++j) {
+        T::Ptr p = t.for_plan(2000 + (r * 70 + j), 0, mk(2000), drop);
         t.release(p, drop);
       }
     }
@@ -65,8 +65,8 @@ int main() {
   before = made;
   { T::Ptr p = u.for_plan(1, 0, mk(1), drop); u.release(p, drop); }   // 1 is young again
   CHECK(made == before);
-  { T::Ptr p = u.for_plan(100, 0, mk(100), drop); u.release(p, drop); }   // evicts 0 (held)
-  { T::Ptr p = u.for_plan(101, 0, mk(101), drop); u.release(p, drop); }   // evicts 2
+  { T::Ptr p = u.for_plan(10000, 0, mk(10000), drop); u.release(p, drop); }   // evicts 0 (held)
+  { T::Ptr p = u.for_plan(10001, 0, mk(10001), drop); u.release(p, drop); }   // evicts 2
   CHECK(dropped == std::multiset<int>{2});
   u.release(a, drop);
   CHECK(dropped.count(0) == 0);
@@ -76,7 +76,7 @@ int main() {
   before = made;
   CHECK(u.for_call(1, 0, mk(1))->k == 1 && made == before);
   // devices apart
-  { T::Ptr p = u.for_plan(101, 1, mk(101), drop); CHECK(made == before + 1); u.release(p, drop); }
+  { T::Ptr p = u.for_plan(10001, 1, mk(10001), drop); CHECK(made == before + 1); u.release(p, drop); }
   // from several threads
   std::vector<std::thread> th;
   std::mutex m;
@@ -84,7 +84,7 @@ int main() {
   for (int i = 0; i < 8; ++i)
     th.emplace_back([&, i] {
       for (int r = 0; r < 2000; ++r) {
-        const int k = (r * 13 + i) % 90;
+        const int k = (r * 13 + i) % 300;
         T::Ptr p = u.for_plan(k, 0, [k] { return new V{k}; }, [&](V &v) { v.k = -1; });
         if (p->k != k) { std::lock_guard<std::mutex> l(m); ++bad; }
         u.release(p, [&](V &v) { v.k = -1; });

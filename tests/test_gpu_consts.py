@@ -58,7 +58,7 @@ def test_plans_outlive_their_place_in_the_table():
     del twin
 
     def churn(k):
-        for i in range(30):
+        for i in range(40):
             s = (10 + 2 * i, 12 + 2 * k)
             c, v = _problem(s, 60, seed=k)
             p = nufft.plan(nu2u=True, coord=c, grid_shape=s, epsilon=1e-9)
@@ -75,7 +75,7 @@ def test_plans_outlive_their_place_in_the_table():
         t.start()
     for t in threads:
         t.join()
-    assert len(ok) == 120 and all(ok)
+    assert len(ok) == 160 and all(ok)
     plan.nu2u(points=vals, forward=True, out=out[1])
     # (sums in another order)
     assert torch.linalg.vector_norm(out[1] - out[0]) <= 2e-9 * torch.linalg.vector_norm(out[0])
