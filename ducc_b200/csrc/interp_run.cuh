@@ -11,8 +11,10 @@
 //
 // Staging a tile in shared memory and reading W^2 cells of 16 bytes per point
 // took 132 SM cycles per point at W = 15 (28 of shared-memory bandwidth, the rest
-// bank conflicts and latency at 255 registers); this takes 18 cycles of FP64
-// per point, and the window's loads come from L2 once per bin.
+// bank conflicts and latency at 255 registers); this takes 18 cycles of matrix
+// instructions per point, and the window's loads come from L2 once per bin: 5e6
+// points 2.32 -> 0.80 ms, 46 cycles in all (12 warps per SM; the matrix pipe is
+// active 39 % of the cycles, the rest is the latency of staging and of the loads).
 //
 // A window with a value that is not finite is not multiplied (zero weights
 // would spread it to points that do not touch it): its points read their own

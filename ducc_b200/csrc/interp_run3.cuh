@@ -10,7 +10,9 @@
 // plane weight, in shared memory, where they are added over the planes.
 //
 // Reading W^3 cells of 16 bytes through L1 per point took 700 SM cycles per point
-// at W = 12; the matrix instructions take 165.  Small supports and thinly spread
+// at W = 12; the matrix instructions take 165, all of it 426 (1e6 points, 1.5 ms: the
+// matrix pipe is active 45 % of the cycles, the warps of the one CTA that fits an SM
+// wait for staging and at its barriers).  Small supports and thinly spread
 // points are left to that direct form (k_interp_direct3).
 //
 // Mirrors HelperU2nu / interpolation_helper (src/ducc0/nufft/nufft.h:1508-1729).
@@ -291,7 +293,8 @@ void interp_direct3_w(const PointsDesc &pts, const Geometry &g, const KernelPoly
 //
 // One thread per point reading W^3 cells from a staged tile took 134 SM cycles at
 // W = 8 (32 of shared-memory bandwidth; 16 warps per SM); this takes 46 issue
-// cycles.
+// cycles for the sums and their 12 shuffles per four points, 108 cycles in all (1e7
+// points, 256^3 cells, 3.8 ms; issue active 59 %).
 template <int W> struct Interp3fShape {
   static constexpr int PLANES = 16, ROWS = 16, CELLS = 16;
   static constexpr int THREADS = 128, BATCH = 128;
