@@ -142,7 +142,7 @@ template <typename T> size_t interp_multi_smem(const Geometry &g) {
   return r;
 }
 
-uint32_t spread_multi_ppw(uint64_t total_points) { return run_points_per_warp(total_points); }
+uint32_t spread_multi_ppw(uint64_t total_points) { return run_points_per_warp(total_points, false); }
 
 template <typename T> uint32_t spread_multi_ctas(uint32_t npts, uint32_t ppw) {
   const uint64_t per = uint64_t(run_threads<T>() / 32) * ppw;

@@ -198,7 +198,7 @@ void interp_run_w(const PointsDesc &pts, const uint32_t *sel, uint32_t npts, con
   const size_t sm = NW * InterpShape<W>::WARP_BYTES;
   auto kern = k_interp_run<Tc, W>;
   allow_smem(kern, sm);
-  const uint32_t ppw = run_points_per_warp(uint64_t(npts) * uint64_t(ntrans));
+  const uint32_t ppw = run_points_per_warp(uint64_t(npts) * uint64_t(ntrans), true);
   const uint64_t per = uint64_t(NW) * ppw;
   dim3 grd(unsigned((npts + per - 1) / per), ntrans);
   kern<<<grd, IR_THREADS, sm, st>>>(pts, sel, npts, ppw, g, kp, static_cast<const double2 *>(grid),

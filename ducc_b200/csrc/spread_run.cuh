@@ -318,11 +318,19 @@ __device__ __forceinline__ void spread_run(const PointsDesc &pts, const uint32_t
   if (cu >= 0) flush();
 }
 
-// points per warp: about 24 warps per SM get work before longer runs save
-// flushes; a multiple of 32 from 32 up, at least 8 (few points: a warp adds its
-// points one after the other, so more warps finish sooner)
-inline uint32_t run_points_per_warp(uint64_t npts) {
-  const uint64_t p = npts / (148 * 24);
+// Points per warp: about 24 warps per SM get work before longer runs save flushes; a
+// multiple of 32 from 32 up, at least 8 (few points: a warp adds its points one after
+// the other, so more warps finish sooner).  waves: where runs of 128 points and more
+// would make little more than one wave of warps, a third of that length: warps in
+// thin and in dense places take times of their own, and a wave lasts as long as its
+// slowest (1e6 points, one wave / three, us: complex64 spreading of clustered points
+// on 2420^2 cells 188 / 96, 4116^2 222 / 121, evenly spread 203 / 167, complex128
+// interpolation of clustered points on 1890^2 211 / 109).  Not for complex128
+// spreading, whose flushes cost more (clustered on 224^2: 118 / 211; thinly spread
+// ones would gain, 248 / 139 on 1890^2), nor for fewer points (3e5 on 1050^2: 50 / 53).
+inline uint32_t run_points_per_warp(uint64_t npts, bool waves) {
+  uint64_t p = npts / (148 * 24);
+  if (waves && p >= 128) p = std::max<uint64_t>(64, p / 3);
   return uint32_t(p < 32 ? std::max<uint64_t>(8, p & ~uint64_t(7))
                          : std::min<uint64_t>(256, p & ~uint64_t(31)));
 }
@@ -352,7 +360,7 @@ void spread_run_w(const PointsDesc &pts, const uint32_t *sel, uint32_t npts, con
   const size_t sm = NW * RunShape<T, W>::WARP_BYTES;
   auto kern = k_spread_run<T, Tc, W>;
   allow_smem(kern, sm);
-  const uint32_t ppw = run_points_per_warp(uint64_t(npts) * uint64_t(ntrans));
+  const uint32_t ppw = run_points_per_warp(uint64_t(npts) * uint64_t(ntrans), sizeof(T) == 4);
   const uint64_t per = uint64_t(NW) * ppw;
   dim3 grd(unsigned((npts + per - 1) / per), ntrans);
   kern<<<grd, run_threads<T>(), sm, st>>>(pts, sel, npts, ppw, g, kp,
