@@ -433,21 +433,21 @@ static int bitlen64(uint64_t v) {
   return b;
 }
 
-// Digits up to which the sort also orders the points of a 3D bin by cell
-// (make_setup).  The kernels with one thread per point (k_interp_direct3, k_interp,
-// k_interp_dcoord) read fewer lines per warp then: complex128, 2e6 clustered points,
-// 176^3 cells, W = 8: interpolation 1348 -> 896 us, gradient 1886 -> 1578; complex64,
-// 132^3 cells, W = 6: gradient 451 -> 378.  Longer digits make the sort slower (5e6
-// points, 11 bits for 10: plan 411 -> 543 us), which complex64 plans do not pay for;
-// unplanned complex64 calls and type 1 keep the shortest key (20,000 points: 9 us).
+// Which calls sort the points of a 3D bin by cell too, as far as the passes of the
+// sort keep to digits of so many bits: the kernels with one thread per point
+// (k_interp_direct3, k_interp, k_interp_dcoord) read fewer lines per warp then
+// (complex128, 2e6 clustered points, 176^3 cells, W = 8: interpolation 1348 -> 896 us,
+// gradient 1886 -> 1578; complex64, 132^3 cells, W = 6: gradient 451 -> 378).  Longer
+// digits make the sort slower (5e6 points, 11 bits for 10: plan 411 -> 543 us; 7e4
+// points: 20 us), so complex64 plans stop at 10 bits, and of the unplanned calls only
+// those do it whose interpolation goes cell by cell.
+enum class CellOrder { FIRST_AXIS, FOR_DIRECT, FOR_PLAN };
 constexpr int CELL_DIGIT_F64 = RADIX_BITS, CELL_DIGIT_F32 = 10;
 
-// run_order: sort the points by bin inside their tile.  cell_digit: in 3D by cell
-// inside the bin too, as far as the passes of the sort keep to digits of so many bits
-// (0: by the first axis only).
+// run_order: sort the points by bin inside their tile (3D: cells as above).
 static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double epsilon,
                         bool gridding, bool calc_f64, bool coord_f64, const dnufft_opts &o,
-                        bool run_order = false, int cell_digit = 0) {
+                        bool run_order = false, CellOrder cells = CellOrder::FIRST_AXIS) {
   DN_REQUIRE(ndim >= 1 && ndim <= 3, ST_BADARG, "transform must be 1D/2D/3D");
   DN_REQUIRE(npoints <= 0xffffffffull, ST_BADARG, "too many nonuniform points");
   DN_REQUIRE(epsilon > 0, ST_BADARG, "epsilon must be positive");
@@ -560,7 +560,11 @@ static Setup make_setup(int ndim, const int64_t *nuni, uint64_t npoints, double 
     if (bits <= 32) {
       s.order.bin_bits = bb;
       s.order.bin_log2 = lb;
-      const int room = std::min(32, (bits + RADIX_BITS - 1) / RADIX_BITS * cell_digit);
+      const bool by_cell = cells == CellOrder::FOR_PLAN ||
+                           (cells == CellOrder::FOR_DIRECT && calc_f64 &&
+                            interp3_direct(g, s.npoints));
+      const int digit = !by_cell ? 0 : (calc_f64 ? CELL_DIGIT_F64 : CELL_DIGIT_F32);
+      const int room = std::min(32, (bits + RADIX_BITS - 1) / RADIX_BITS * digit);
       while (s.order.cell_axes < 3 && bits + s.order.cell_axes * lb <= room) ++s.order.cell_axes;
       s.tile_shift = bb + lb * s.order.cell_axes;
       maxkey = s.max_tiles << (lb * s.order.cell_axes);   // (bin_bits are added below)
@@ -1202,7 +1206,7 @@ static void u2nu_impl(const dnufft_array *grid_, const dnufft_array *coord_, int
   bool f64 = uni.dtype == DNUFFT_C128;
   Setup s = make_setup(ndim, uni.shape, uint64_t(coord.shape[0]), eps, false, f64,
                        coord.dtype == DNUFFT_F64, o, ndim == 3 || (f64 && ndim == 2),
-                       f64 ? CELL_DIGIT_F64 : 0);
+                       CellOrder::FOR_DIRECT);
   StageTimer tm(o.verbosity > 0, st);
   if (o.verbosity > 0) report_sizes(s, false);
   if (s.npoints == 0) return;
@@ -1333,7 +1337,7 @@ static void plan_create_impl(int nu2u, const dnufft_array *coord_, const int64_t
   auto p = std::make_unique<dnufft_plan>();
   p->o = o;
   p->s = make_setup(ndim, shape, uint64_t(coord.shape[0]), eps, nu2u != 0, f64, f64, o, true,
-                    f64 ? CELL_DIGIT_F64 : CELL_DIGIT_F32);
+                    CellOrder::FOR_PLAN);
   DN_CUDA(cudaGetDevice(&p->device));
   p->dc = consts_for_plan(p->s, st);
   if (p->s.npoints > 0) {

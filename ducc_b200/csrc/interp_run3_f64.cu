@@ -22,12 +22,12 @@ namespace dnufft {
 //   W = 16  p = 7: 1 / 0.85, else more
 // A few thousand points are latency: from W = 8 the windows' many warps per point
 // finish sooner (1000 points: 1 / 1.03-1.2 at W = 8, 1 / 2.5 at W = 14).
-static bool interp3_direct(const Geometry &g, uint32_t npts) {
+bool interp3_direct(const Geometry &g, uint32_t npts) {
   const int W = g.W;
   if (W > 15 || (W >= 8 && npts < (W <= 10 ? 4096u : 16384u))) return false;
   if (W <= 10) return true;
   const double p = double(npts) * 512. / (double(g.nover[0]) * double(g.nover[1]) * double(g.nover[2]));
-  if (W == 11) return p < 8. || p > 400.;
+  if (W == 11) return p < 8. || p > 500.;
   if (W == 12) return p < 6.;
   return p < (W <= 14 ? 30. : 18.);
 }

@@ -141,6 +141,8 @@ void launch_interp_run(const PointsDesc &pts, const uint32_t *sel, uint32_t npts
 // Does 3D type 2 work bin by bin from the grid (launch_interp_run3; no chunk
 // list) or from tiles staged in shared memory (k_interp, single precision only)?
 bool interp3_in_windows(const Geometry &g, bool f64);
+// ... and in double precision cell by cell (k_interp_direct3)?
+bool interp3_direct(const Geometry &g, uint32_t npts);
 // 3D (launch_interp goes here where interp3_in_windows)
 void launch_interp_run3(const PointsDesc &pts, const Geometry &g, const KernelPoly<float> &kp,
                         const void *grid, int64_t gtrans, void *out, int64_t os, int64_t otrans,

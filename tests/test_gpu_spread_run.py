@@ -148,7 +148,7 @@ def test_smallest_grids(single, W, ndim):
 
 
 @pytest.mark.parametrize("W,nover,M", [(8, (36, 48, 20), 4500), (9, (36, 48, 20), 4500),
-                                       (10, (20, 40, 36), 4500), (11, (30, 40, 36), 35000),
+                                       (10, (20, 40, 36), 4500), (11, (30, 40, 36), 45000),
                                        (11, (110, 120, 126), 17000), (12, (126, 120, 128), 17000),
                                        (13, (72, 70, 80), 17000), (14, (72, 70, 80), 17000),
                                        (15, (90, 88, 80), 17000)])
